@@ -131,4 +131,25 @@ static inline void illm_launch(void (*kern)(KArgs...), dim3 grid, dim3 block, si
     cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
+// The same with clusters of `cluster` blocks along x (grid.x a multiple of it).
+template <typename... KArgs, typename... Args>
+static inline int illm_launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, int cluster, size_t smem, cudaStream_t s, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = cluster > 1 ? attr : attr + 1;
+    cfg.numAttrs = (cluster > 1 ? 1 : 0) + (g_illm_pdl ? 1 : 0);
+    g_illm_launches++;
+    cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+    return (int)cudaGetLastError();
+}
+
 static inline int illm_launch_status() { return (int)cudaGetLastError(); }

@@ -5,85 +5,153 @@
 // cache or the batching that rounding would otherwise excuse.
 // The reference calls cublasSgemm here (src/kern/gpu/kernel_gpu.cu:420-435), formula
 // src/kern/naive/naive.cpp:363-379 (weight row-major [out, in], no bias).
-// 64x64 tile of C per block, 16-wide slices of K through shared memory, 4x4 outputs a thread.
+//
+// Tile kernel: a BM x BN tile of C per block, TM x TN outputs a thread, slices of 16 values of k in two shared-memory
+// buffers (k-major, so that the columns of a pair lie side by side), the next slice on its way to registers while
+// this one is used, one barrier per slice.  What bounds it is the float32 FMA rate: two neighbouring columns share
+// one packed fma.rn.f32x2 (each half rounded like a scalar fused multiply-add, so the chain per output and its bits
+// stay what they were), and an 8 x 8 thread tile reads 64 bytes of shared memory per 32 packed instructions, its
+// warp covering 32 x 64 outputs so that each 16-byte read is one conflict-free pass.
 #include "tc_common.cuh"
 
-#define GF_BM 64
-#define GF_BN 64
 #define GF_BK 16
 
-__global__ void __launch_bounds__(256)
+__device__ __forceinline__ unsigned long long gf_pair(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ unsigned long long gf_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+// 16-byte pieces of a ROWS x 16 slice of a row-major matrix: a thread's share of them on their way through registers.
+template <int ROWS, int THREADS>
+struct GfSlice {
+    static constexpr int N = ROWS * (GF_BK / 4) / THREADS;
+    static_assert(N >= 1 && ROWS * (GF_BK / 4) % THREADS == 0, "a slice is whole pieces per thread");
+    float4 v[N];
+    // rows beyond the matrix and values beyond K arrive as zeros, which change no sum
+    __device__ __forceinline__ void load(const float* __restrict__ src, int row0, int rows, int ld, int k0, int K, bool vec) {
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const int piece = threadIdx.x + i * THREADS, row = row0 + (piece >> 2), k = k0 + (piece & 3) * 4;
+            v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (row < rows && k < K) {
+                const float* p = src + (size_t)row * ld + k;
+                if (vec) {                       // K % 4 == 0: a piece that begins inside ends inside
+                    v[i] = *reinterpret_cast<const float4*>(p);
+                } else {
+                    v[i].x = p[0];
+                    if (k + 1 < K) v[i].y = p[1];
+                    if (k + 2 < K) v[i].z = p[2];
+                    if (k + 3 < K) v[i].w = p[3];
+                }
+            }
+        }
+    }
+    __device__ __forceinline__ void store(float (*dst)[ROWS + 4]) const {
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const int piece = threadIdx.x + i * THREADS, row = piece >> 2, k = (piece & 3) * 4;
+            dst[k][row] = v[i].x;
+            dst[k + 1][row] = v[i].y;
+            dst[k + 2][row] = v[i].z;
+            dst[k + 3][row] = v[i].w;
+        }
+    }
+};
+
+// A warp is 4 threads along the rows by 8 along the columns; a thread's rows and columns are pieces of four, a warp's
+// tile apart.  TM, TN: 4 or 8.
+template <int BM, int BN, int TM, int TN>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), BM * BN >= 128 * 128 ? 2 : 4)
 gemm_f32_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
                    int M, int N, int K, int lda, int ldw, int ldc) {
+    constexpr int THREADS = (BM / TM) * (BN / TN), WARPS_N = BN / (8 * TN);
     pdl_grid_sync();
-    __shared__ __align__(16) float As[GF_BK][GF_BM + 4];
-    __shared__ __align__(16) float Ws[GF_BK][GF_BN + 4];
-    const int tid = threadIdx.x;
-    const int m0 = blockIdx.y * GF_BM, n0 = blockIdx.x * GF_BN;
-    const int lr = tid >> 2, lk = (tid & 3) * 4;  // loader: row within the tile, k offset
-    const int ty = tid >> 4, tx = tid & 15;
+    __shared__ __align__(16) float As[2][GF_BK][BM + 4];
+    __shared__ __align__(16) float Ws[2][GF_BK][BN + 4];
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // first row and column of the thread's first piece; the second piece lies 16 rows / 32 columns further on
+    const int tm = (warp / WARPS_N) * 4 * TM + (lane >> 3) * 4, tn = (warp % WARPS_N) * 8 * TN + (lane & 7) * 4;
     const bool vec = ((K & 3) == 0) && ((lda & 3) == 0) && ((ldw & 3) == 0) &&
                      ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
-    float acc[4][4];
+    unsigned long long acc[TM][TN / 2];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < TM; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+        for (int j = 0; j < TN / 2; j++) acc[i][j] = 0ull;
 
-    for (int k0 = 0; k0 < K; k0 += GF_BK) {
-        float a[4] = {0.f, 0.f, 0.f, 0.f}, w[4] = {0.f, 0.f, 0.f, 0.f};
-        const int k = k0 + lk;
-        if (m0 + lr < M) {
-            const float* src = A + (size_t)(m0 + lr) * lda + k;
-            if (vec && k + 3 < K) {
-                float4 v = *reinterpret_cast<const float4*>(src);
-                a[0] = v.x; a[1] = v.y; a[2] = v.z; a[3] = v.w;
-            } else {
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-                    if (k + i < K) a[i] = src[i];
-            }
+    GfSlice<BM, THREADS> a;
+    GfSlice<BN, THREADS> w;
+    a.load(A, m0, M, lda, 0, K, vec);
+    w.load(W, n0, N, ldw, 0, K, vec);
+    a.store(As[0]);
+    w.store(Ws[0]);
+    __syncthreads();
+    int buf = 0;
+    for (int k0 = 0; k0 < K; k0 += GF_BK, buf ^= 1) {
+        const bool more = k0 + GF_BK < K;
+        if (more) {
+            a.load(A, m0, M, lda, k0 + GF_BK, K, vec);
+            w.load(W, n0, N, ldw, k0 + GF_BK, K, vec);
         }
-        if (n0 + lr < N) {
-            const float* src = W + (size_t)(n0 + lr) * ldw + k;
-            if (vec && k + 3 < K) {
-                float4 v = *reinterpret_cast<const float4*>(src);
-                w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-            } else {
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-                    if (k + i < K) w[i] = src[i];
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            As[lk + i][lr] = a[i];
-            Ws[lk + i][lr] = w[i];
-        }
-        __syncthreads();
 #pragma unroll
         for (int kk = 0; kk < GF_BK; kk++) {
-            const float4 av = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
-            const float4 wv = *reinterpret_cast<const float4*>(&Ws[kk][tx * 4]);
-            const float ar[4] = {av.x, av.y, av.z, av.w};
-            const float wr[4] = {wv.x, wv.y, wv.z, wv.w};
+            float av[TM];
+            unsigned long long wv[TN / 2];
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < TM; i += 4) *reinterpret_cast<float4*>(av + i) = *reinterpret_cast<const float4*>(&As[buf][kk][tm + 4 * i]);
 #pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(ar[i], wr[j], acc[i][j]);
+            for (int j = 0; j < TN / 2; j += 2)
+                *reinterpret_cast<ulonglong2*>(wv + j) = *reinterpret_cast<const ulonglong2*>(&Ws[buf][kk][tn + 16 * j]);
+#pragma unroll
+            for (int i = 0; i < TM; i++) {
+                const unsigned long long ai = gf_pair(av[i], av[i]);
+#pragma unroll
+                for (int j = 0; j < TN / 2; j++) acc[i][j] = gf_fma2(ai, wv[j], acc[i][j]);
+            }
         }
+        if (more) {
+            // the other buffer was read in the round before, which every thread has left (the barrier below)
+            a.store(As[buf ^ 1]);
+            w.store(Ws[buf ^ 1]);
+        }
+        __syncthreads();
     }
+    const bool vec_c = (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int m = m0 + ty * 4 + i;
+    for (int i = 0; i < TM; i++) {
+        const int m = m0 + tm + (i >> 2) * 16 + (i & 3);
         if (m >= M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int n = n0 + tx * 4 + j;
-            if (n < N) C[(size_t)m * ldc + n] = acc[i][j];
+        for (int j = 0; j < TN; j += 4) {
+            const int n = n0 + tn + 8 * j;
+            float r[4];
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(r[0]), "=f"(r[1]) : "l"(acc[i][j / 2]));
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(r[2]), "=f"(r[3]) : "l"(acc[i][j / 2 + 1]));
+            float* dst = C + (size_t)m * ldc + n;
+            if (vec_c && n + 4 <= N) {
+                *reinterpret_cast<float4*>(dst) = make_float4(r[0], r[1], r[2], r[3]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    if (n + c < N) dst[c] = r[c];
+            }
         }
     }
+}
+
+template <int BM, int BN, int TM, int TN>
+static int launch_gemm_f32_tile(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
+    const dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN);      // the row tiles of a panel of W next to each other
+    if (grid.y > 65535) return ILLM_ERR_BAD_ARG;
+    illm_launch(gemm_f32_nt_kernel<BM, BN, TM, TN>, grid, dim3((BM / TM) * (BN / TN)), 0, s, A, W, C, M, N, K, lda, ldw, ldc);
+    return illm_launch_status();
 }
 
 // The same product for at most 8 rows (single tokens of a few sequences), where the tile kernel above
@@ -241,8 +309,11 @@ extern "C" int illm_gemm_f32_nt(const float* A, const float* W, float* C, int M,
         if (M <= 4) return launch_gemm_f32_small<4>(A, W, C, M, N, K, lda, ldw, ldc, err, s);
         return launch_gemm_f32_small<8>(A, W, C, M, N, K, lda, ldw, ldc, err, s);
     }
-    dim3 grid((N + GF_BN - 1) / GF_BN, (M + GF_BM - 1) / GF_BM);
-    if (grid.y > 65535) return ILLM_ERR_BAD_ARG;
-    illm_launch(gemm_f32_nt_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, A, W, C, M, N, K, lda, ldw, ldc);
-    return illm_launch_status();
+    // The larger tile needs half the shared-memory traffic per FMA; the smaller ones run where the larger would leave
+    // SMs without a block, or where most of its rows lie beyond M.
+    cudaStream_t s = (cudaStream_t)stream;
+    auto blocks = [&](long long bm, long long bn) { return ((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
+    if (M > 64 && blocks(128, 128) >= 120) return launch_gemm_f32_tile<128, 128, 8, 8>(A, W, C, M, N, K, lda, ldw, ldc, s);
+    if (M > 32 && blocks(64, 64) >= 120) return launch_gemm_f32_tile<64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
+    return launch_gemm_f32_tile<32, 64, 4, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
 }

@@ -165,7 +165,7 @@ int illm_latent_rope_prep(const float* x, int ld, int q_off, int H, int d, int d
 // stream_ops.cu
 int illm_add_bias(void* y, int dtype, const float* b, int T, int H, void* stream);
 int illm_scaled_add_rmsnorm(float* resid, const float* delta, const float* ls, const float* w, void* y, int act_dtype, int T, int H, float eps, void* stream);
-int illm_attention_generic_ex(const void* q, int q_stride, const void* kc, const void* vc, const int* block_table, int max_pages, const int* token_pos, const int* token_seq, void* out, int act_dtype, int T, int nh, int nkv, int d, int page_size, int span, float scale, int dv, const float* sinks, const float* gate, int gate_stride, int gate_wide, float softcap, void* stream);
+int illm_attention_generic_ex(const void* q, int q_stride, const void* kc, const void* vc, const int* block_table, int max_pages, const int* token_pos, const int* token_seq, void* out, int act_dtype, int T, int nh, int nkv, int d, int page_size, int span, float scale, int dv, const float* sinks, const float* gate, int gate_stride, int gate_wide, float softcap, int prompts, void* stream);
 int illm_qk_prep_mix(const void* x, int x_dtype, int ld, int q_off, int k_off, int v_off, int nh, int nkv, int d, int dv, const float* bq, const float* bk, const float* bv, const float* wq, const float* wk, float eps, const float* cos_sin, int rot, int pairs, int n_pos, const int* token_pos, const int* token_seq, const int* block_table, int max_pages, int page_size, void* q_out, void* kc, void* vc, int act_dtype, int T, int* err, float qt_coef, int qt_every, const float* v_first, int v_first_ld, const float* v_lambda, float* v_keep, void* stream);
 int illm_gemm_bf16_tc_gated_ex(const void* X, const void* W, void* out, int M, int N, int K, int act, float act_limit, int* err, void* stream);
 int illm_gemm_bf16_tc2_ex(const void* X, const void* W, void* out, int out_dtype, int epi, float act_limit, int M, int N, int K, int* err, void* stream);

@@ -437,7 +437,7 @@ Mat attention_generic(Device& dev, const Mat& qkv, const KVView& kv, const StepV
                                            code_of(qkv.dtype, "attention_generic"), (int)qkv.rows, g.n_heads, g.n_kv_heads, g.head_dim, kv.page_size,
                                            kv.span(), scale, dv, extras ? extras->sinks : nullptr, extras ? extras->gate : nullptr,
                                            extras ? extras->gate_stride : 0, extras && extras->wide_gate ? 1 : 0, extras ? extras->softcap : 0.f,
-                                           dev.stream()),
+                                           ctx.is_decode ? 0 : 1, dev.stream()),
                  "attention_generic");
     return out;
 }

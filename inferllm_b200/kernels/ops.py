@@ -43,6 +43,7 @@ _KERNEL_SIGNATURES = {
     "illm_residual_add": [P_, P_, I_, LL_, P_],
     "illm_swiglu": [P_, P_, I_, I_, I_, P_],
     "illm_rope_kv_write": [P_, P_, P_, P_, P_, I_, P_, P_, I_, I_, I_, I_, I_, I_, I_, I_, I_, P_, P_],
+    "illm_attention_generic_ex": [P_, I_, P_, P_, P_, I_, P_, P_, P_, I_, I_, I_, I_, I_, I_, I_, F_, I_, P_, P_, I_, I_, F_, I_, P_],
     "illm_attention_generic": [P_, I_, P_, P_, P_, I_, P_, P_, P_, I_, I_, I_, I_, I_, I_, I_, F_, I_, P_, P_, I_, P_],
     "illm_attention_decode": [P_, I_, P_, P_, P_, I_, P_, P_, P_, P_, P_, I_, I_, I_, I_, I_, I_, F_, I_, P_],
     "illm_attention_decode_supported": [I_, I_, I_],
@@ -337,9 +338,10 @@ def rope_kv_write(qkv, cos_sin, rot_dim, token_pos, token_seq, block_table, k_ca
 
 
 def attention_generic(qkv, k_cache, v_cache, block_table, token_pos, token_seq, n_heads,
-                      n_kv_heads, head_dim, page_size, window, scale):
+                      n_kv_heads, head_dim, page_size, window, scale, prompts=False):
     """Attention of each token (query heads in the first n_heads*head_dim columns of `qkv`)
-    over its sequence's cache pages; returns [T, n_heads*head_dim]."""
+    over its sequence's cache pages; returns [T, n_heads*head_dim].  `window` may be negative: chunks of that many
+    positions.  `prompts`: the step holds more than one token of a sequence (another kernel, the same result)."""
     if head_dim % 8 or head_dim > MAX_HEAD_DIM_GENERIC:
         raise KernelError(f"attention: head size {head_dim} is not supported (multiples of 8 up to "
                           f"{MAX_HEAD_DIM_GENERIC})")
@@ -350,11 +352,11 @@ def attention_generic(qkv, k_cache, v_cache, block_table, token_pos, token_seq, 
     _need(v_cache, "v_cache", qkv.dtype, 4)
     T = qkv.shape[0]
     out = _rows(T, n_heads * head_dim, qkv.dtype, qkv.device)
-    _check(load().illm_attention_generic(
+    _check(load().illm_attention_generic_ex(
         _ptr(qkv), qkv.shape[1], _ptr(k_cache), _ptr(v_cache), _ptr(block_table),
         block_table.shape[1], _ptr(token_pos), _ptr(token_seq), _ptr(out), act_code(qkv.dtype), T,
         n_heads, n_kv_heads, head_dim, page_size, int(window or 0), float(scale), head_dim, None, None, 0,
-        _stream()),
+        0, 0.0, 1 if prompts else 0, _stream()),
         "attention_generic")
     return out
 

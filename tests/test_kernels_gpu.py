@@ -161,6 +161,19 @@ def test_gemm_f32_is_true_float32_and_row_invariant():
         assert torch.equal(one[0], full[r])
 
 
+@pytest.mark.parametrize("M,N,K", [(65, 15361, 36), (128, 15360, 16), (300, 5124, 35), (257, 8196, 17), (33, 7700, 20), (64, 7681, 48), (12, 130, 100)])
+def test_gemm_f32_tiles(M, N, K):
+    """Edges of the three tile sizes (128 x 128 from 65 rows and 120 tiles on, 64 x 64, 32 x 64): against float64 (K products and
+    sums, each rounded: K 2^-24 of the sum of magnitudes at most), and rows bit for bit what the row alone gives."""
+    g = torch.Generator().manual_seed(M + N + K)
+    x, w = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g)
+    out = ops.gemm_f32(dev(x), dev(w)).cpu()
+    ref, mag = f64(x) @ f64(w).T, np.abs(f64(x)) @ np.abs(f64(w)).T
+    assert (np.abs(f64(out) - ref) <= K * 2.0 ** -24 * mag).all()
+    for r in sorted({0, 31, 32, 63, M // 2, M - 1} & set(range(M))):
+        assert torch.equal(ops.gemm_f32(dev(x[r:r + 1]), dev(w)).cpu()[0], out[r])
+
+
 @pytest.mark.parametrize("M,N,K", [(5, 96, 64), (2048, 300, 128), (1, 1000, 4096)])
 def test_linear_bf16(M, N, K):
     g = torch.Generator().manual_seed(K)
@@ -657,6 +670,36 @@ def test_attention_decode_says_what_it_takes():
     assert not ops.attention_decode_supported(torch.bfloat16, 4, 4, 24, 64)
     assert not ops.attention_decode_supported(torch.bfloat16, 5, 1, 128, 64)
     assert not ops.attention_decode_supported(torch.bfloat16, 4, 4, 128, 12)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("nh,nkv,d,page,window", [(4, 4, 16, 8, None), (6, 2, 24, 16, -48), (5, 5, 128, 32, None), (40, 8, 72, 64, None), (2, 2, 128, 64, 64)])
+def test_attention_generic_bits_do_not_depend_on_the_kernel(dtype, nh, nkv, d, page, window):
+    """Tokens by eights (prompts), a block per token, and 2, 4 or 8 blocks per token (few tokens) give the same bits, with
+    tiles that hold the ends and beginnings of several sequences, chunks (window < 0) and a jump within a sequence; rows
+    behind a sequence are NaN and must not be touched."""
+    lens = [1, 37, 700, 64]
+    pc = Paged(lens, nkv, d, page, DT[dtype], seed=d + 1)
+    g = torch.Generator().manual_seed(8)
+    rows = [(1, p) for p in range(37)] + [(0, 0), (3, 63)] + [(2, p) for p in range(60, 125)] + [(2, p) for p in range(500, 700)]
+    T = len(rows)
+    qkv = torch.randn(T, (nh + 2 * nkv) * d, generator=g).to(DT[dtype])
+    seq = torch.tensor([r[0] for r in rows], dtype=torch.int32)
+    pos = torch.tensor([r[1] for r in rows], dtype=torch.int32)
+
+    def run(idx, prompts):
+        return ops.attention_generic(dev(qkv[idx]), dev(pc.kc), dev(pc.vc), dev(pc.table), dev(pos[idx]), dev(seq[idx]), nh, nkv, d, page, window,
+                                     1.0 / math.sqrt(d), prompts=prompts).cpu()
+
+    every = list(range(T))
+    out = run(every, False)
+    assert torch.isfinite(out.float()).all()
+    assert torch.equal(run(every, True), out)
+    for n in (1, 9, 36):               # 36 tokens of 40 heads: a block each; fewer: clusters of 2, 4, 8
+        some = every[5:5 + n]
+        assert torch.equal(run(some, False), out[some]) and torch.equal(run(some, True), out[some])
+    for t in (T - 1, 37, 40):
+        assert torch.equal(run([t], False)[0], out[t])
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
