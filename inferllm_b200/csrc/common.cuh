@@ -152,4 +152,15 @@ static inline int illm_launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 bl
     return (int)cudaGetLastError();
 }
 
+// SMs of the current device, asked for once.
+static inline int illm_sm_count() {
+    static const int n = [] {
+        int dev = 0, v = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+        return v > 0 ? v : 1;
+    }();
+    return n;
+}
+
 static inline int illm_launch_status() { return (int)cudaGetLastError(); }

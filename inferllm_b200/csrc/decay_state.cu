@@ -34,6 +34,7 @@
 // times an activation of a gate projection (sigmoid or silu), rounded once to the activation dtype.
 #include <type_traits>
 
+#include "chunk_scan.h"
 #include "common.cuh"
 
 #define DS_THREADS 128
@@ -452,6 +453,30 @@ extern "C" int illm_decay_scan(float* x, int T, int ld, int q_off, int k_off, in
     if (!a.inline_prep && (qk_act || v_act || rot || k_scale != 1.0f)) illm_launch(decay_prep_kernel, dim3(T, nh), dim3(128), 0, s, a);
     decay_launch_for<false>(a, B, s);
     return illm_launch_status();
+}
+
+// The same for prompts, eight tokens at a time (chunk_scan.cu; d <= 128): rec is scratch of illm_decay_chunk_scratch floats, max_q
+// the most tokens of one sequence, segments illm_decay_chunk_segments or any number from 1 on.
+extern "C" int illm_decay_chunk_segments(int B, int nh, int dv, int max_q) { return chunk_scan_segments(CHUNK_LINEAR, B, nh, dv, max_q); }
+extern "C" long long illm_decay_chunk_scratch(int T, int B, int nh, int d, int dv, int segments) {
+    const long long rec = (chunk_scan_scratch(T, B, nh) + 63) / 64 * 64;
+    return rec + (segments > 1 ? (long long)B * segments * nh * d * dv : 0);
+}
+extern "C" int illm_decay_chunk_scan(float* x, int T, int ld, int q_off, int k_off, int v_off, int nh, int d, int dv, int qk_act, int v_act,
+                                     const float* cos_sin, int rot, int n_pos, float k_scale, const float* decay, float* state, const int* slots,
+                                     const int* cu_q, const int* token_pos, float* out, int B, int max_q, int segments, int* err, float* rec, void* stream) {
+    if (B <= 0 || T <= 0) return 0;
+    if (nh <= 0 || !chunk_scan_takes(d) || dv <= 0 || nh > 65535 || rot < 0 || rot > d || (rot & 1) || (rot && !cos_sin) || !x || !state || !out || !rec)
+        return ILLM_ERR_BAD_ARG;
+    cudaStream_t s = (cudaStream_t)stream;
+    if (qk_act || v_act || rot || k_scale != 1.0f) {
+        DecayScanArgs a{x, ld, q_off, k_off, v_off, nh, d, dv, qk_act, v_act, cos_sin, rot, n_pos, k_scale, decay, state, slots, cu_q, token_pos, out, err,
+                        0, 0, 0, 1, nullptr, nullptr, nullptr, 1, (long long)nh * d * dv, nullptr};
+        illm_launch(decay_prep_kernel, dim3(T, nh), dim3(128), 0, s, a);
+    }
+    const ChunkScanArgs c{x + q_off, x + k_off, x + v_off, ld, decay, nullptr, nh, 1, d, dv, state, (long long)nh * d * dv, slots, cu_q, rec, out, segments,
+                          segments > 1 ? rec + (chunk_scan_scratch(T, B, nh) + 63) / 64 * 64 : nullptr};
+    return chunk_scan_launch(c, CHUNK_LINEAR, B, max_q, s);
 }
 
 // The same recurrence with a gate pair per token and head (ga, gb: float32 [T, nh]) in place of the fixed decay, the

@@ -18,14 +18,15 @@
 // products of a token are added over the L lanes by a fixed tree of shuffles, and a token's arithmetic does not
 // depend on where the step's cut falls, so prompts, portions and single tokens give the same bits.
 //
-// delta_chunk_scan_kernel: the same with one decay per head, eight tokens at a time, for steps where that order of the sums is
-// allowed (the bfloat16 mode).  With S the state before the eight, G_j the product of the decays up to token j and D_ji
+// Prompts of the bfloat16 mode, where that order of the sums is allowed, take eight tokens at a time: chunk_scan.cu for heads of up
+// to 128 key channels, and for larger ones with one decay per head delta_chunk_scan_kernel.  With S the state before the eight, G_j the product of the decays up to token j and D_ji
 // the product of those behind i up to j,
 //     u_j = beta_j (v_j - G_j S^T k_j - sum_(i<j) D_ji (k_i . k_j) u_i)
 //     o_j = G_j S^T q_j + sum_(i<=j) D_ji (k_i . q_j) u_i
 //     S  <- G_7 S + sum_i D_7i k_i u_i
 // so the sixteen products with S are independent of one another (one round of shuffles for all), and only the short
 // triangular sums follow in order.  The coefficients, which the columns share, are made by delta_chunk_prep_kernel.  float32.
+#include "chunk_scan.h"
 #include "common.cuh"
 
 #define DL_THREADS 128
@@ -686,7 +687,8 @@ static void launch_scan_as(const DeltaArgs& p, int B, int n_sms, cudaStream_t s)
 
 template <int L, int ROWS>
 static void launch_scan(const DeltaArgs& p, int B, int n_sms, cudaStream_t s, const float* rec) {
-    if constexpr (ROWS <= 16) if (rec) {        // (eight tokens at a time with 32 rows per thread do not fit the registers)
+    // (eight tokens at a time with 32 rows per thread do not fit the registers; up to 128 rows chunk_scan.cu takes them)
+    if constexpr (ROWS <= 16 && ROWS * L > 128) if (rec) {
         constexpr int COLS = DL_THREADS / L;
         size_t smem = (size_t)2 * (DL_TILE * (2 * ROWS * L + COLS) + (DL_TILE / DC) * DC_REC) * sizeof(float);
         const long long blocks = (long long)((p.dv + COLS - 1) / COLS) * p.nh * B, per_sm = (blocks + n_sms - 1) / n_sms;
@@ -729,8 +731,8 @@ static void launch_scan_for(const DeltaArgs& p, int B, cudaStream_t s, const flo
 // x: [T, ld] float32 with q at q_off (nkv * d columns), k at k_off, v at v_off (nh * dv), beta's logits at b_off (nh).
 // state: float32 [slots, state_elems], state_elems >= nh * d * dv + (taps - 1) * (2 nkv d + nh dv).
 // a: the decay projection, rows a_ld apart: nh * d columns, or with head_decay nh.
-// chunks (head_decay only; nullptr: token by token): illm_delta_chunk_scratch floats, the scan then takes eight tokens at a
-// time; max_q the most tokens of one sequence.
+// chunks (nullptr: token by token; without head_decay only for d <= 128): illm_delta_chunk_scratch floats, the scan then takes
+// eight tokens at a time; max_q the most tokens of one sequence.
 // Scratch qkv [T, 2 nkv d + nh dv], g [T, nh d] (head_decay: [T, nh]), beta [T, nh]; out [T, nh dv].
 extern "C" int illm_delta_rule(const float* x, int T, int ld, int q_off, int k_off, int v_off, int b_off, const float* a, int a_ld, int head_decay, int nh, int nkv, int d,
                                int dv, int taps, const float* conv_q, const float* conv_k, const float* conv_v, const float* a_log,
@@ -738,7 +740,7 @@ extern "C" int illm_delta_rule(const float* x, int T, int ld, int q_off, int k_o
                                const int* token_pos, const int* token_seq, const int* seq_lens, float* qkv, float* g, float* beta, float* out,
                                int B, int max_q, float* chunks, void* stream) {
     if (T <= 0 || B <= 0) return 0;
-    if (!illm_delta_rule_supported(d, dv, taps) || nkv <= 0 || nh % nkv || a_ld < (head_decay ? nh : nh * d) || (chunks && (!head_decay || max_q <= 0 || nkv > 65535 || B > 65535))) return ILLM_ERR_BAD_ARG;
+    if (!illm_delta_rule_supported(d, dv, taps) || nkv <= 0 || nh % nkv || a_ld < (head_decay ? nh : nh * d) || (chunks && ((!head_decay && !chunk_scan_takes(d)) || max_q <= 0 || nkv > 65535 || B > 65535))) return ILLM_ERR_BAD_ARG;
     const long long C = 2LL * nkv * d + (long long)nh * dv;
     if (state_elems < (long long)nh * d * dv + (taps - 1) * C) return ILLM_ERR_BAD_ARG;
     cudaStream_t s = (cudaStream_t)stream;
@@ -759,6 +761,11 @@ extern "C" int illm_delta_rule(const float* x, int T, int ld, int q_off, int k_o
     else if (taps == 4) illm_launch(delta_prep_kernel<4>, pgrid, dim3(256), 0, s, p);
     else illm_launch(delta_prep_kernel<0>, pgrid, dim3(256), 0, s, p);
     if (taps > 1) illm_launch(conv_state_kernel, dim3((unsigned)((C + 127) / 128), B), dim3(128), 0, s, p);
+    if (chunks && chunk_scan_takes(d)) {
+        const float* base = qkv;
+        const ChunkScanArgs a{base, base + (long long)nkv * d, base + 2LL * nkv * d, C, g, beta, nh, nh / nkv, d, dv, state, state_elems, slots, cu_q, chunks, out, 1, nullptr};
+        return chunk_scan_launch(a, head_decay ? CHUNK_DELTA_HEAD : CHUNK_DELTA_CHANNEL, B, max_q, s);
+    }
     if (chunks) {
         const size_t smem = (size_t)2 * DC * d * sizeof(float);
         illm_launch(delta_chunk_prep_kernel, dim3((max_q + DC - 1) / DC, nkv, B), dim3(128), smem, s, p, chunks);

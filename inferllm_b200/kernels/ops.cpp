@@ -530,6 +530,15 @@ Mat decay_scan(Device& dev, const Mat& x, const DecayScan& p, const StepView& ct
         throw KernelError("decay_scan: a state of " + std::to_string(p.head_dim) + " x " + std::to_string(p.v_head_dim) +
                           " per head is beyond the kernel (head sizes up to 1024)");
     Mat out = new_mat_exact(dev, x.rows, (long long)p.n_heads * p.v_head_dim, DType::F32);
+    if (!p.in_order && ctx.max_q >= kChunkScanMinTokens && p.head_dim <= kChunkScanMaxHeadDim) {
+        const int pieces = illm_decay_chunk_segments(ctx.B, p.n_heads, p.v_head_dim, ctx.max_q);
+        float* rec = dev.alloc_n<float>((size_t)illm_decay_chunk_scratch((int)x.rows, ctx.B, p.n_heads, p.head_dim, p.v_head_dim, pieces));
+        check_kernel(illm_decay_chunk_scan((float*)x.p, (int)x.rows, (int)x.cols, p.q_off, p.k_off, p.v_off, p.n_heads, p.head_dim, p.v_head_dim, p.qk_act,
+                                           p.v_act, p.rot_dim ? p.cos_sin : nullptr, p.rot_dim, (int)p.n_pos, p.k_scale, p.decay, (float*)st.state, st.slots,
+                                           ctx.cu_q, ctx.token_pos, (float*)out.p, ctx.B, ctx.max_q, pieces, ctx.err, rec, dev.stream()),
+                     "decay_scan");
+        return out;
+    }
     const int segments = (p.in_order || ctx.is_decode) ? 1 : decay_scan_segments(ctx.B, p.n_heads, p.v_head_dim, ctx.max_q, dev.n_sms());
     float* seg_state = segments > 1 ? dev.alloc_n<float>((size_t)ctx.B * segments * p.n_heads * p.head_dim * p.v_head_dim) : nullptr;
     check_kernel(illm_decay_scan((float*)x.p, (int)x.rows, (int)x.cols, p.q_off, p.k_off, p.v_off, p.n_heads, p.head_dim, p.v_head_dim, p.qk_act, p.v_act,
@@ -971,7 +980,7 @@ Mat delta_rule(Device& dev, const Mat& x, const Mat* a, const DeltaRule& p, cons
         throw KernelError("delta_rule: the state entry does not have this layer's size");
     Mat qkv = new_mat_exact(dev, T, C, DType::F32), g = new_mat_exact(dev, T, decays, DType::F32), beta = new_mat_exact(dev, T, p.n_heads, DType::F32);
     Mat out = new_mat_exact(dev, T, (long long)p.n_heads * p.v_head_dim, DType::F32);
-    const bool chunked = p.head_decay && !p.in_order && ctx.max_q >= kDeltaChunkMinTokens;
+    const bool chunked = !p.in_order && ctx.max_q >= kChunkScanMinTokens && (p.head_decay || p.head_dim <= kChunkScanMaxHeadDim);
     float* chunks = chunked ? dev.alloc_n<float>((size_t)illm_delta_chunk_scratch((int)T, ctx.B, p.n_heads)) : nullptr;
     check_kernel(illm_delta_rule((const float*)x.p, (int)T, (int)x.cols, p.q_off, p.k_off, p.v_off, p.b_off,
                                  p.head_decay ? (const float*)x.p + p.a_off : (const float*)a->p, p.head_decay ? (int)x.cols : (int)decays,

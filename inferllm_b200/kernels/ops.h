@@ -373,7 +373,9 @@ struct DeltaRule {
     const float *a_log = nullptr, *dt_bias = nullptr;                        // float32 [heads], [heads * head_dim] or [heads]
     float q_scale = 1.f;
 };
-constexpr int kDeltaChunkMinTokens = 16;      // the most tokens of a sequence in a step from which the scan takes eight at a time
+// the most tokens of a sequence in a step from which the recurrences take eight at a time (bfloat16 mode; below, the state's
+// way in and out and the record of a chunk cost as much as the tokens), and the largest key heads of chunk_scan.cu
+constexpr int kChunkScanMinTokens = 16, kChunkScanMaxHeadDim = 128;
 long long delta_rule_state_elements(int n_heads, int n_kv_heads, int head_dim, int v_head_dim, int taps);
 bool delta_rule_supported(int head_dim, int v_head_dim, int taps);
 Mat delta_rule(Device& dev, const Mat& x_f32, const Mat* a_f32, const DeltaRule& p, const StepView& ctx, const StateView& st);

@@ -1,0 +1,119 @@
+"""The recurrences eight tokens at a time (csrc/chunk_scan.cu) against float64 loops, at the edges of chunks, tiles and column
+blocks, beside the token-by-token kernels on the same inputs."""
+import ctypes
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+P_, I_, F_, L_ = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_longlong
+LENS = [1, 7, 8, 9, 16, 17, 131, 30]
+
+
+def entry(name, restype, *argtypes):
+    from inferllm_b200.kernels import ops
+    f = getattr(ops.load(), name)
+    f.restype, f.argtypes = restype, list(argtypes)
+    return f
+
+
+def p(t):
+    return None if t is None else t.data_ptr()
+
+
+def layout():
+    cu = np.concatenate([[0], np.cumsum(LENS)])
+    ints = lambda a: torch.tensor(np.asarray(a), dtype=torch.int32, device="cuda")  # noqa: E731
+    pos, seq = np.concatenate([np.arange(n) for n in LENS]), np.repeat(np.arange(len(LENS)), LENS)
+    return cu, ints(cu), ints(pos), ints(seq), ints(np.arange(len(LENS))[::-1].copy()), ints(LENS)
+
+
+@pytest.mark.parametrize("d,dv,nh,off", [(128, 128, 3, 0), (128, 64, 2, 4), (20, 130, 2, 0), (9, 7, 1, 1), (100, 65, 2, 0), (64, 200, 1, 0)])
+@pytest.mark.parametrize("segments", [1, 2, 5])
+def test_linear_attention(d, dv, nh, off, segments):
+    g = torch.Generator().manual_seed(d + dv)
+    cu, cu_d, pos, _, slots, _ = layout()
+    T, B, C = int(cu[-1]), len(LENS), nh * (2 * d + dv) + off
+    x = torch.randn(T, C, generator=g)
+    S0 = torch.randn(B, nh, dv, d, generator=g)
+    decay = torch.tensor([0.3, 0.97, 0.9999][:nh])
+    q_off, k_off, v_off = off, off + nh * d, off + 2 * nh * d
+    xd, Sd, out, dd = x.cuda(), S0.cuda(), torch.full((T, nh * dv), float("nan"), device="cuda"), decay.cuda()
+    n = entry("illm_decay_chunk_scratch", L_, I_, I_, I_, I_, I_, I_)(T, B, nh, d, dv, segments)
+    rec, err = torch.full((n,), float("nan"), device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    rc = entry("illm_decay_chunk_scan", I_, P_, I_, I_, I_, I_, I_, I_, I_, I_, I_, I_, P_, I_, I_, F_, P_, P_, P_, P_, P_, P_, I_, I_, I_, P_, P_, P_)(
+        p(xd), T, C, q_off, k_off, v_off, nh, d, dv, 0, 0, None, 0, 0, 1.0, p(dd), p(Sd), p(slots), p(cu_d), p(pos), p(out), B, max(LENS), segments, p(err), p(rec),
+        torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    got, state = out.cpu().double().numpy().reshape(T, nh, dv), Sd.cpu().double().numpy()
+    q, k, v = (x[:, o:o + nh * w].double().numpy().reshape(T, nh, w) for o, w in ((q_off, d), (k_off, d), (v_off, dv)))
+    a = decay.double().numpy()
+    # a term goes through at most d + 2 roundings in sums over rows, 2 per chunk or segment in the state, one per token of a segment in
+    # the powers of the decay (twice: a fold and a read-out), and 20 more
+    bound = 2.0 ** -24 * (d + 2 * (max(LENS) / 8) + 22 + (2 * max(LENS) if segments > 1 else 0))
+    for b in range(B):
+        s = B - 1 - b
+        S, M = S0[s].double().numpy().copy(), S0[s].abs().double().numpy()
+        for t in range(cu[b], cu[b + 1]):
+            S = a[:, None, None] * S + v[t][:, :, None] * k[t][:, None, :]
+            M = a[:, None, None] * M + np.abs(v[t])[:, :, None] * np.abs(k[t])[:, None, :]
+            ref, mag = np.einsum("hvd,hd->hv", S, q[t]), np.einsum("hvd,hd->hv", M, np.abs(q[t]))
+            assert (np.abs(got[t] - ref) <= bound * mag).all(), (b, t - cu[b])
+        assert (np.abs(state[s] - S) <= bound * M).all()
+
+
+@pytest.mark.parametrize("head_decay", [0, 1])
+@pytest.mark.parametrize("d,dv,nh,nkv", [(128, 128, 4, 2), (128, 64, 1, 1), (20, 130, 2, 2), (9, 7, 3, 1), (100, 65, 2, 1)])
+@pytest.mark.parametrize("strong", [False, True])
+def test_delta_rule(head_decay, d, dv, nh, nkv, strong):
+    """The recurrence feeds its own output back, so the reference for its rounding is the token-by-token kernel: no more than twice as
+    far from float64 (both measured as 2-norms over a sequence).  strong: decays down to e^-60."""
+    taps = 2
+    g = torch.Generator().manual_seed(d * dv + head_decay)
+    cu, cu_d, pos, seq, slots, lens = layout()
+    T, B = int(cu[-1]), len(LENS)
+    C = 2 * nkv * d + nh * dv
+    ld = C + nh
+    x = torch.randn(T, ld, generator=g)
+    na = nh if head_decay else nh * d
+    a = torch.randn(T, na, generator=g) * (20.0 if strong else 1.0)
+    conv = [torch.randn(w, taps, generator=g) for w in (nkv * d, nkv * d, nh * dv)]
+    a_log, dt = torch.randn(nh, generator=g) * 0.5, torch.randn(na, generator=g)
+    elems = nh * d * dv + (taps - 1) * C
+    S0 = torch.randn(B, elems, generator=g)
+    f = entry("illm_delta_rule", I_, P_, I_, I_, I_, I_, I_, I_, P_, I_, I_, I_, I_, I_, I_, I_, P_, P_, P_, P_, P_, F_, P_, L_, P_, P_, P_, P_, P_, P_, P_, P_, P_, I_,
+              I_, P_, P_)
+    n = entry("illm_delta_chunk_scratch", L_, I_, I_, I_)(T, B, nh)
+    dev = [t.cuda() for t in (x, a, *conv, a_log, dt)]
+
+    def run(chunks):
+        S = S0.cuda()
+        qkv, gg, beta = torch.empty(T, C, device="cuda"), torch.empty(T, na, device="cuda"), torch.empty(T, nh, device="cuda")
+        out = torch.full((T, nh * dv), float("nan"), device="cuda")
+        rec = torch.full((n,), float("nan"), device="cuda") if chunks else None
+        rc = f(p(dev[0]), T, ld, 0, nkv * d, 2 * nkv * d, C, p(dev[1]), na, head_decay, nh, nkv, d, dv, taps, p(dev[2]), p(dev[3]), p(dev[4]), p(dev[5]),
+               p(dev[6]), d ** -0.5, p(S), elems, p(slots), p(cu_d), p(pos), p(seq), p(lens), p(qkv), p(gg), p(beta), p(out), B, max(LENS), p(rec),
+               torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        return [t.cpu().double().numpy() for t in (out, S, qkv, gg, beta)]
+
+    chunked, (out, S, qkv, gg, beta) = run(True), run(False)
+    share = nh // nkv
+    for b in range(B):
+        s = B - 1 - b
+        refs = []
+        St = S0[s, :nh * d * dv].double().numpy().reshape(nh, dv, d).copy()
+        for t in range(cu[b], cu[b + 1]):
+            q, k, v = qkv[t, :nkv * d].reshape(nkv, d).repeat(share, 0), qkv[t, nkv * d:2 * nkv * d].reshape(nkv, d).repeat(share, 0), qkv[t, 2 * nkv * d:].reshape(nh, dv)
+            St = St * (gg[t].reshape(nh, 1, 1) if head_decay else gg[t].reshape(nh, 1, d))
+            u = beta[t][:, None] * (v - np.einsum("hvd,hd->hv", St, k))
+            St = St + u[:, :, None] * k[:, None, :]
+            refs.append(np.einsum("hvd,hd->hv", St, q).reshape(-1))
+        refs, rows = np.array(refs), slice(cu[b], cu[b + 1])
+        for mine, token, ref in ((chunked[0][rows], out[rows], refs), (chunked[1][s, :nh * d * dv], S[s, :nh * d * dv], St.reshape(-1))):
+            assert np.isfinite(mine).all()
+            floor = 2.0 ** -24 * np.linalg.norm(ref)
+            assert np.linalg.norm(mine - ref) <= 2 * np.linalg.norm(token - ref) + 4 * floor
+        assert np.array_equal(chunked[1][s, nh * d * dv:], S[s, nh * d * dv:])       # the convolution's rows
