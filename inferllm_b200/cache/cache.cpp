@@ -320,10 +320,16 @@ int SequenceCache::alloc_slot() {
     seq_len[slot] = 0;
     if (device_)
         for (StateGroup& g : states) {
-            const size_t row = (size_t)g.request.elements() * dtype_size(g.request.dtype);
-            for (size_t e = 0; e < g.entries.size(); e++)
-                check_cuda(cudaMemsetAsync((char*)g.state + e * g.entry_bytes + (size_t)slot * row, 0, row, device_->stream()),
-                           "zeroing a sequence's state");
+            // the slot's rows of all the group's entries in one call where the pitch allows (a call per layer and sequence was a
+            // tenth of a prompt step of 32 sequences)
+            const size_t row = (size_t)g.request.elements() * dtype_size(g.request.dtype), n = g.entries.size();
+            char* first = (char*)g.state + (size_t)slot * row;
+            if (n > 1 && g.entry_bytes <= (size_t)0x7fffffff) {
+                check_cuda(cudaMemset2DAsync(first, g.entry_bytes, 0, row, n, device_->stream()), "zeroing a sequence's state");
+            } else {
+                for (size_t e = 0; e < n; e++)
+                    check_cuda(cudaMemsetAsync(first + e * g.entry_bytes, 0, row, device_->stream()), "zeroing a sequence's state");
+            }
         }
     return slot;
 }
