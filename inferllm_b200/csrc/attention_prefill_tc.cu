@@ -216,18 +216,21 @@ static FtCap ft_make_cap(float softcap, float scale) {
 // gate[row * gate_stride + head], or with gate_wide gate[row * gate_stride + head * D + channel]): the output is multiplied by
 // its sigmoid.  Either may be nullptr.  CAP: the scaled scores s become cap * tanh(s / cap) before the mask (FtCap); the kernel
 // then works on capped scores in units of log2 and its scale is 1.
-template <int D, bool WIDE_P, bool CAP>
+// DK: score channels, D but for the differential form (DIFF): there head h has two score maps of DK channels over the same
+// values, its query row holds [q_1, q_2] and a key row [k_1, k_2]; a block takes one (head, map), reads the map's columns of
+// both, and leaves the map's output in float32, rows of nh x 2 x D, for attention_diff_combine_kernel.
+template <int D, int DK, bool WIDE_P, bool CAP, bool DIFF>
 __global__ void __launch_bounds__(FT_THREADS, 2)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const int* __restrict__ block_table,
                             int max_pages, const int* __restrict__ cu_q, const int* __restrict__ seq_lens,
-                            bf16* __restrict__ out, int nh, int nkv, int page_size, int span,
+                            void* __restrict__ out, int nh, int nkv, int page_size, int span,
                             float scale_log2e, int* __restrict__ err, const float* __restrict__ sinks,
                             const float* __restrict__ gate, int gate_stride, int gate_wide, const FtCap cap) {
     constexpr int FT_MMA_WARP = 4, FT_TMA_WARP = 5;
-    constexpr int NA = D / 64;                            // 64-channel atoms of the head
-    constexpr unsigned Q_TILE = FT_BM * D * 2;            // the query tile: [NA][128 rows][128 B]
-    constexpr unsigned KV_BYTES = FT_BN * D * 2;          // K: [NA][64 keys][128 B]; V: the same shape
+    constexpr int NA = DK / 64, NV = D / 64;              // 64-channel atoms of the keys and of the values
+    constexpr unsigned Q_TILE = FT_BM * DK * 2;           // the query tile: [NA][128 rows][128 B]
+    constexpr unsigned K_BYTES = FT_BN * DK * 2, V_BYTES = FT_BN * D * 2;      // K: [NA][64 keys][128 B]; V: [NV] of the same
     constexpr unsigned Q_ATOM = 128 * 128, KV_ATOM = FT_BN * 128;
     constexpr unsigned TMEM_COLS = 256, S_COLS = FT_BN, O_COL = 2 * FT_BN;
     constexpr unsigned IDESC_S = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(FT_BN >> 3) << 17) | ((unsigned)(FT_BM >> 4) << 24);
@@ -237,8 +240,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     // swizzle's period) and two blocks fit an SM.  Barriers sit behind the tiles.
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const unsigned base = s_u32(smem_raw);
-    const unsigned q_s = base, k_s = q_s + Q_TILE, v_s = k_s + FT_KSTAGES * KV_BYTES;
-    const unsigned bars0 = v_s + FT_VSTAGES * KV_BYTES;
+    const unsigned q_s = base, k_s = q_s + Q_TILE, v_s = k_s + FT_KSTAGES * K_BYTES;
+    const unsigned bars0 = v_s + FT_VSTAGES * V_BYTES;
     const unsigned q_full = bars0, k_full0 = bars0 + 8, k_empty0 = k_full0 + 8 * FT_KSTAGES;
     const unsigned v_full0 = k_empty0 + 8 * FT_KSTAGES, v_empty0 = v_full0 + 8 * FT_VSTAGES;
     const unsigned s_full0 = v_empty0 + 8 * FT_VSTAGES, p_full0 = s_full0 + 16, pv_done = p_full0 + 16;
@@ -287,7 +290,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     // end and the x-th from the start, which gives all blocks equal work, was slower at every prompt
     // length: 52.5 against 50.2 us at 2,048 tokens of 32 heads, 138 against 101 us at 3,072.)  With chunks the work of a
     // tile grows with its place inside its chunk, and the tiles of all chunks are taken in the order of that place.
-    const int b = blockIdx.z, h = blockIdx.x;
+    const int b = blockIdx.z, h = DIFF ? blockIdx.x >> 1 : blockIdx.x, map = DIFF ? blockIdx.x & 1 : 0;
     const int q0 = cu_q[b], qlen = cu_q[b + 1] - q0;
     const int n_tiles = (qlen + FT_BM - 1) / FT_BM;
     int tile = n_tiles - 1 - (int)blockIdx.y;                 // < 0: this sequence is shorter than the longest
@@ -317,7 +320,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         // block i-2 has; the loop asks in the order in which those come true.
         if (lane == 0 && has_rows) {
             bar_expect_tx(q_full, Q_TILE);
-            for (int a = 0; a < NA; a++) tma_2d(q_s + a * Q_ATOM, &map_q, h * D + 64 * a, q0 + row0, q_full);
+            for (int a = 0; a < NA; a++) tma_2d(q_s + a * Q_ATOM, &map_q, (int)blockIdx.x * DK + 64 * a, q0 + row0, q_full);
             auto kv_row = [&](int i) {
                 const int key0 = (jb0 + i) * FT_BN;
                 return (bt[key0 / page_size] * nkv + hk) * page_size + (key0 % page_size);
@@ -327,16 +330,16 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 const int st = i % FT_KSTAGES;
                 if (i >= FT_KSTAGES && !bar_wait(k_empty0 + 8 * st, ((i / FT_KSTAGES) - 1) & 1, err)) return false;
                 const int row = kv_row(i);
-                bar_expect_tx(k_full0 + 8 * st, KV_BYTES);
-                for (int a = 0; a < NA; a++) tma_2d(k_s + st * KV_BYTES + a * KV_ATOM, &map_k, 64 * a, row, k_full0 + 8 * st);
+                bar_expect_tx(k_full0 + 8 * st, K_BYTES);
+                for (int a = 0; a < NA; a++) tma_2d(k_s + st * K_BYTES + a * KV_ATOM, &map_k, map * DK + 64 * a, row, k_full0 + 8 * st);
                 return true;
             };
             auto load_v = [&](int i) {
                 const int st = i % FT_VSTAGES;
                 if (i >= FT_VSTAGES && !bar_wait(v_empty0 + 8 * st, ((i / FT_VSTAGES) - 1) & 1, err)) return false;
                 const int row = kv_row(i);
-                bar_expect_tx(v_full0 + 8 * st, KV_BYTES);
-                for (int a = 0; a < NA; a++) tma_2d(v_s + st * KV_BYTES + a * KV_ATOM, &map_v, 64 * a, row, v_full0 + 8 * st);
+                bar_expect_tx(v_full0 + 8 * st, V_BYTES);
+                for (int a = 0; a < NV; a++) tma_2d(v_s + st * V_BYTES + a * KV_ATOM, &map_v, 64 * a, row, v_full0 + 8 * st);
                 return true;
             };
             for (int i = 0; i < FT_KSTAGES && i < n_blocks && alive; i++) alive = load_k(i);
@@ -355,9 +358,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 if (!bar_wait(k_full0 + 8 * st, (i / FT_KSTAGES) & 1, err)) return false;
                 fence_after();
 #pragma unroll
-                for (int kk = 0; kk < D / 16; kk++) {
+                for (int kk = 0; kk < DK / 16; kk++) {
                     const unsigned qo = (kk >> 2) * Q_ATOM + (kk & 3) * 32;
-                    const unsigned ko = st * KV_BYTES + (kk >> 2) * KV_ATOM + (kk & 3) * 32;
+                    const unsigned ko = st * K_BYTES + (kk >> 2) * KV_ATOM + (kk & 3) * 32;
                     mma_bf16_ss(tmem + (i & 1) * S_COLS, desc_kmajor(q_s + qo), desc_kmajor(k_s + ko), IDESC_S, kk > 0);
                 }
                 mma_commit(s_full0 + 8 * (i & 1));     // the scores are there
@@ -379,12 +382,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 #pragma unroll
                 for (int ks = 0; ks < FT_BN / 16; ks++)
                     mma_bf16_ts(tmem + O_COL, tmem + (i & 1) * S_COLS + ks * 8,
-                                desc_mnmajor(v_s + st * KV_BYTES + ks * 16 * 128, KV_ATOM), IDESC_O, (i > 0 || ks > 0) ? 1u : 0u);
+                                desc_mnmajor(v_s + st * V_BYTES + ks * 16 * 128, KV_ATOM), IDESC_O, (i > 0 || ks > 0) ? 1u : 0u);
                 if (WIDE_P) {
 #pragma unroll
                     for (int ks = 0; ks < FT_BN / 16; ks++)
                         mma_bf16_ts(tmem + O_COL, tmem + (i & 1) * S_COLS + FT_BN / 2 + ks * 8,
-                                    desc_mnmajor(v_s + st * KV_BYTES + ks * 16 * 128, KV_ATOM), IDESC_O, 1u);
+                                    desc_mnmajor(v_s + st * V_BYTES + ks * 16 * 128, KV_ATOM), IDESC_O, 1u);
                 }
                 mma_commit(v_empty0 + 8 * st);
                 mma_commit(pv_done);
@@ -520,8 +523,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 alive = __all_sync(0xffffffffu, bar_wait(v_full0 + 8 * st, (i / FT_VSTAGES) & 1, err));
                 if (r < FT_BN && key0 + r > last_pos) {
 #pragma unroll
-                    for (int a = 0; a < NA; a++) {
-                        const unsigned row_addr = v_s + st * KV_BYTES + a * KV_ATOM + r * 128;
+                    for (int a = 0; a < NV; a++) {
+                        const unsigned row_addr = v_s + st * V_BYTES + a * KV_ATOM + r * 128;
 #pragma unroll
                         for (int q8 = 0; q8 < 8; q8++)
                             asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(row_addr + q8 * 16), "r"(0u) : "memory");
@@ -553,13 +556,14 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 inv = 1.0f / l_run;
             }
             if (gate && !gate_wide && r < rows) inv *= 1.0f / (1.0f + expf(-gate[(size_t)(q0 + row0 + r) * gate_stride + h]));
-            bf16* dst = out + ((size_t)(q0 + row0 + r) * nh + h) * D;
+            bf16* dst = (bf16*)out + ((size_t)(q0 + row0 + r) * nh + h) * D;
+            float* dst_map = (float*)out + ((size_t)(q0 + row0 + r) * 2 * nh + blockIdx.x) * D;      // DIFF
             // a gate per channel: a warp brings its 32 rows, whole rows at a time, into the shared memory that the tiles of
             // Q and K no longer need (every product has been done), from where a thread reads its own row
             constexpr int G_ROW = D * 4 + 16;
             const unsigned g_s = base + warp * 32 * G_ROW;
-            static_assert(4 * 32 * G_ROW <= (int)(Q_TILE + FT_KSTAGES * KV_BYTES), "the gate rows must fit the tiles of Q and K");
-            if (WIDE_P && gate && gate_wide == 2) {
+            static_assert(DIFF || 4 * 32 * G_ROW <= (int)(Q_TILE + FT_KSTAGES * K_BYTES), "the gate rows must fit the tiles of Q and K");
+            if (WIDE_P && !DIFF && gate && gate_wide == 2) {
 #pragma unroll 8
                 for (int rr = 0; rr < 32; rr++) {
                     const int row = warp * 32 + rr;
@@ -581,7 +585,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                         float f[8];
 #pragma unroll
                         for (int e = 0; e < 8; e++) f[e] = __uint_as_float(orr[c + e]) * inv;
-                        if (WIDE_P && gate && gate_wide) {
+                        if (WIDE_P && !DIFF && gate && gate_wide) {
                             const float* gr = gate + (size_t)(q0 + row0 + r) * gate_stride + (size_t)h * D + c0 + c;
                             float g8[8];
                             if (gate_wide == 2) {          // rows of whole 16-byte pieces
@@ -595,7 +599,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 #pragma unroll
                             for (int e = 0; e < 8; e++) f[e] = __fdividef(f[e], 1.0f + __expf(-g8[e]));
                         }
-                        store8(dst + c0 + c, f);
+                        if (DIFF) {
+                            *reinterpret_cast<float4*>(dst_map + c0 + c) = make_float4(f[0], f[1], f[2], f[3]);
+                            *reinterpret_cast<float4*>(dst_map + c0 + c + 4) = make_float4(f[4], f[5], f[6], f[7]);
+                        } else {
+                            store8(dst + c0 + c, f);
+                        }
                     }
                 }
             }
@@ -641,25 +650,25 @@ static int ft_make_map(CUtensorMap* map, const void* ptr, long long rows, long l
     return r == CUDA_SUCCESS ? 0 : ILLM_ERR_BAD_ARG;
 }
 
-template <int D, bool WIDE_P, bool CAP>
+template <int D, bool WIDE_P, bool CAP, int DK = D, bool DIFF = false>
 static int ft_launch(const void* q, int q_stride, int T, const void* kc, const void* vc, long long n_pages,
                      const int* block_table, int max_pages, const int* cu_q, const int* seq_lens, void* out, int B,
                      int max_q, int nh, int nkv, int page_size, int span, float scale, int* err, const float* sinks,
                      const float* gate, int gate_stride, int gate_wide, float softcap, cudaStream_t s) {
     CUtensorMap mq, mk, mv;
     int rc;
-    if ((rc = ft_make_map(&mq, q, T, (long long)nh * D, q_stride, FT_BM)) != 0) return rc;
+    if ((rc = ft_make_map(&mq, q, T, (long long)nh * (DIFF ? 2 : 1) * DK, q_stride, FT_BM)) != 0) return rc;
     const long long kv_rows = n_pages * nkv * page_size;
-    if ((rc = ft_make_map(&mk, kc, kv_rows, D, D, FT_BN)) != 0) return rc;
+    if ((rc = ft_make_map(&mk, kc, kv_rows, DIFF ? 2 * DK : DK, DIFF ? 2 * DK : DK, FT_BN)) != 0) return rc;
     if ((rc = ft_make_map(&mv, vc, kv_rows, D, D, FT_BN)) != 0) return rc;
-    const size_t smem = (size_t)FT_BM * D * 2 + (size_t)(FT_KSTAGES + FT_VSTAGES) * FT_BN * D * 2 +
+    const size_t smem = (size_t)FT_BM * DK * 2 + (size_t)(FT_KSTAGES * DK + FT_VSTAGES * D) * FT_BN * 2 +
                         256;   // + barriers and the tensor-memory address
-    auto kern = attention_prefill_tc_kernel<D, WIDE_P, CAP>;
+    auto kern = attention_prefill_tc_kernel<D, DK, WIDE_P, CAP, DIFF>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    dim3 grid(nh, (max_q + FT_BM - 1) / FT_BM, B);
+    dim3 grid(DIFF ? 2 * nh : nh, (max_q + FT_BM - 1) / FT_BM, B);
     illm_launch(kern, grid, dim3(FT_THREADS), smem, s, mq, mk, mv, block_table, max_pages, cu_q, seq_lens,
-                (bf16*)out, nh, nkv, page_size, span, CAP ? 1.0f : scale * 1.4426950408889634f, err, sinks, gate, gate_stride, gate_wide,
+                out, nh, nkv, page_size, span, CAP ? 1.0f : scale * 1.4426950408889634f, err, sinks, gate, gate_stride, gate_wide,
                 CAP ? ft_make_cap(softcap, scale) : FtCap{});
     return illm_launch_status();
 }
@@ -698,4 +707,47 @@ extern "C" int illm_attention_prefill_tc(const void* q, int q_stride, int T, con
                                          void* stream) {
     return illm_attention_prefill_tc_ex(q, q_stride, T, kc, vc, n_pages, block_table, max_pages, cu_q, seq_lens, out, B, max_q, nh, nkv, d,
                                         page_size, window, scale, err, 0, nullptr, nullptr, 0, 0, 0.f, stream);
+}
+
+// o = a_1 - lambda a_2 of every (token, head), the head's unit norm over its D values and the factor: a warp per head, a lane per
+// four channels.  maps: float32 [T, nh, 2, D].
+template <int D>
+__global__ void __launch_bounds__(256) attention_diff_combine_kernel(const float* __restrict__ maps, bf16* __restrict__ out, long long heads, float lambda,
+                                                                     float eps, float out_scale) {
+    pdl_grid_sync();
+    const long long i = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int c = (threadIdx.x & 31) * 4;
+    if (i >= heads) return;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 a = c < D ? *reinterpret_cast<const float4*>(maps + i * 2 * D + c) : zero, b = c < D ? *reinterpret_cast<const float4*>(maps + (i * 2 + 1) * D + c) : zero;
+    const float4 o = make_float4(fmaf(-lambda, b.x, a.x), fmaf(-lambda, b.y, a.y), fmaf(-lambda, b.z, a.z), fmaf(-lambda, b.w, a.w));
+    const float ss = warp_sum(fmaf(o.x, o.x, fmaf(o.y, o.y, fmaf(o.z, o.z, o.w * o.w))));
+    const float f = out_scale / sqrtf(ss / (float)D + eps);
+    if (c >= D) return;
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(o.x * f, o.y * f), hi = __floats2bfloat162_rn(o.z * f, o.w * f);
+    *reinterpret_cast<uint2*>(out + i * D + c) = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
+}
+
+// Differential attention of prompts (two score maps of 64 channels over values of 128): q [T, q_stride] with head h's
+// [q_1, q_2] at column h * 128, pages of key rows [k_1, k_2] and value rows; maps: scratch, float32 [T, nh, 2, dv]; window: see
+// first_visible.  A map is one pass of the kernel above over its own columns, so the two maps run side by side on
+// tensor memory; the warp-level MMA kernel of attention_maps.cu, which holds both maps' outputs in registers, took 622 us for
+// 1,777 tokens of 32 heads.
+extern "C" int illm_attention_diff_tc_supported(int nh, int nkv, int d, int dv, int page_size) {
+    return d == 64 && dv == 128 && page_size > 0 && page_size % 64 == 0 && nkv > 0 && nh % nkv == 0 && nh <= 32767;
+}
+extern "C" int illm_attention_diff_tc(const void* q, int q_stride, int T, const void* kc, const void* vc, long long n_pages, const int* block_table,
+                                      int max_pages, const int* cu_q, const int* seq_lens, float* maps, void* out, int B, int max_q, int nh, int nkv, int d,
+                                      int dv, int page_size, int window, float scale, float lambda, float eps, float out_scale, int* err, void* stream) {
+    if (B <= 0 || max_q <= 0 || T <= 0) return 0;
+    if (!illm_attention_diff_tc_supported(nh, nkv, d, dv, page_size) || max_q > 65535 * FT_BM || B > 65535 || (q_stride & 7) || !maps || ((uintptr_t)q & 15) ||
+        ((uintptr_t)kc & 15) || ((uintptr_t)vc & 15) || ((uintptr_t)maps & 15) || ((uintptr_t)out & 15))
+        return ILLM_ERR_BAD_ARG;
+    cudaStream_t s = (cudaStream_t)stream;
+    const int rc = ft_launch<128, true, false, 64, true>(q, q_stride, T, kc, vc, n_pages, block_table, max_pages, cu_q, seq_lens, maps, B, max_q, nh, nkv,
+                                                         page_size, window, scale, err, nullptr, nullptr, 0, 0, 0.f, s);
+    if (rc) return rc;
+    const long long heads = (long long)T * nh;
+    illm_launch(attention_diff_combine_kernel<128>, dim3((unsigned)((heads + 7) / 8)), dim3(256), 0, s, maps, (bf16*)out, heads, lambda, eps, out_scale);
+    return illm_launch_status();
 }

@@ -831,6 +831,14 @@ Mat attention_diff(Device& dev, const Mat& q, const KVView& kv, const StepView& 
     if (!kv.k || !kv.v || kv.dtype != q.dtype || kv.n_kv_heads != g.n_kv_heads || kv.head_dim != 2 * g.head_dim || q.cols < (long long)g.n_heads * 2 * g.head_dim)
         throw KernelError("attention_diff: the cache entry must hold key rows of two maps (2 x " + std::to_string(g.head_dim) + " channels) in the queries' dtype");
     Mat out = new_mat(dev, q.rows, (long long)g.n_heads * dv, q.dtype);
+    if (q.dtype == DType::BF16 && !ctx.is_decode && q.cols % 8 == 0 && illm_attention_diff_tc_supported(g.n_heads, g.n_kv_heads, g.head_dim, dv, kv.page_size)) {
+        float* maps = dev.alloc_n<float>((size_t)q.rows * g.n_heads * 2 * dv);
+        check_kernel(illm_attention_diff_tc(q.p, (int)q.cols, (int)q.rows, kv.k, kv.v, kv.num_pages, kv.block_table, kv.width, ctx.cu_q, ctx.seq_lens, maps, out.p,
+                                            ctx.B, ctx.max_q, g.n_heads, g.n_kv_heads, g.head_dim, dv, kv.page_size, kv.window, scale, p.lambda, p.eps, p.out_scale,
+                                            dev.tc_error_word(), dev.stream()),
+                     "attention_diff_tc");
+        return out;
+    }
     if (q.dtype == DType::BF16 && !ctx.is_decode && illm_attention_diff_mma_supported(g.head_dim, dv) && q.cols % 8 == 0) {
         check_kernel(illm_attention_diff_mma(q.p, (int)q.cols, kv.k, kv.v, kv.block_table, kv.width, ctx.cu_q, ctx.seq_lens, out.p, ctx.B, ctx.max_q, g.n_heads,
                                              g.n_kv_heads, g.head_dim, dv, kv.page_size, kv.window, scale, p.lambda, p.eps, p.out_scale, dev.stream()),

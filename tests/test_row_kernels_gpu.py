@@ -1,0 +1,177 @@
+"""The kernels that keep a token's row in registers (norms, the preparation of q, k and v) and differential attention on tensor
+memory, at the edges of their pieces, against float64 and against the kernels they stand in for."""
+import math
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from test_chunk_scan_gpu import F_, I_, L_, P_, entry, p   # noqa: E402
+
+WIDTHS = [4, 36, 128, 516, 2048, 4096, 4100, 8192, 8196, 16384, 16388, 30, 4097]     # the last three: not whole pieces, or too wide
+
+
+def stream():
+    return torch.cuda.current_stream().cuda_stream
+
+
+def close(got, ref, roundings, mag=None):
+    """At most so many float32 roundings of the magnitude, plus the output's own rounding."""
+    tol = roundings * 2.0 ** -24 + (2.0 ** -8 if got.dtype == torch.bfloat16 else 0.0)
+    mag = np.abs(ref) if mag is None else mag
+    assert (np.abs(got.cpu().double().numpy() - ref) <= tol * mag + 1e-30).all()
+
+
+@pytest.mark.parametrize("H", WIDTHS)
+@pytest.mark.parametrize("splits", [0, 3, 9])
+def test_scale_add_rmsnorm(H, splits):
+    g = torch.Generator().manual_seed(H + splits)
+    n, alpha, eps = 3, 1.5, 1e-5
+    x, w = torch.randn(n, H, generator=g), torch.randn(H, generator=g)
+    add = torch.randn(max(1, splits), n, H, generator=g)
+    xd, wd, ad = x.cuda(), w.cuda(), add.cuda()
+    y = torch.empty(n, H, dtype=torch.bfloat16, device="cuda")
+    rc = entry("illm_scale_add_rmsnorm", I_, P_, P_, I_, P_, P_, I_, I_, I_, F_, F_, P_, I_, L_, P_)(
+        p(xd), None if splits else p(ad), 0, p(wd), p(y), 1, n, H, alpha, eps, p(ad) if splits else None, splits, n * H, stream())
+    assert rc == 0
+    v = alpha * x.double().numpy() + add.double().numpy().sum(0)
+    mag = alpha * x.abs().double().numpy() + add.abs().double().numpy().sum(0)
+    inv = 1.0 / np.sqrt((v * v).mean(-1, keepdims=True) + eps)
+    ref, m = v * inv * w.double().numpy(), mag * inv * w.abs().double().numpy()
+    for got in (xd, y):
+        close(got, ref, 2 * math.sqrt(H) + 16, m)
+
+
+@pytest.mark.parametrize("H", WIDTHS)
+@pytest.mark.parametrize("center", [0, 1])
+@pytest.mark.parametrize("with_y,with_rows", [(True, False), (False, True), (True, True)])
+def test_norm_sandwich(H, center, with_y, with_rows):
+    g = torch.Generator().manual_seed(H + center)
+    n, eps, post = 4, 1e-5, 1.0 if center else 0.5
+    x, y, wb, w = torch.randn(n, H, generator=g), torch.randn(n, H, generator=g), torch.randn(H, generator=g), torch.randn(H, generator=g)
+    rows = torch.tensor([3, 1], dtype=torch.int32) if with_rows else None
+    xd, yd, wbd, wd, rd = x.cuda(), y.cuda(), wb.cuda(), w.cuda(), rows.cuda() if with_rows else None
+    n_out = 2 if with_rows else n
+    out = torch.empty(n_out, H, dtype=torch.bfloat16, device="cuda")
+    rc = entry("illm_norm_sandwich", I_, P_, P_, P_, P_, P_, I_, P_, I_, I_, F_, I_, I_, F_, P_)(
+        p(xd), p(yd) if with_y else None, p(wbd) if with_y else None, p(wd), p(out), 1, p(rd), n_out, H, eps, 0 if with_rows else 1, center, post, stream())
+    assert rc == 0
+
+    def norm(v, weight):
+        v = v - v.mean(-1, keepdims=True) if center else v
+        return v / np.sqrt((v * v).mean(-1, keepdims=True) + eps) * weight.double().numpy()
+
+    v = x.double().numpy() + (post * norm(y.double().numpy(), wb) if with_y else 0.0)
+    if not with_rows:
+        close(xd, v, 2 * math.sqrt(H) + 16, np.abs(v) + np.abs(x.double().numpy()) + 4)
+    ref = norm(v, w)[[3, 1]] if with_rows else norm(v, w)
+    close(out, ref, 4 * math.sqrt(H) + 32, np.abs(ref) + 4 * w.abs().double().numpy())
+
+
+@pytest.mark.parametrize("width,group", [(2048, 2048), (1032, 516), (8192, 8192), (1024, 128), (12, 4), (8196, 8196), (30, 15)])
+@pytest.mark.parametrize("act", [1, 2])
+def test_group_norm_gate(width, group, act):
+    g = torch.Generator().manual_seed(width + act)
+    T, eps = 3, 1e-5
+    o, gate, w = torch.randn(T, width, generator=g), torch.randn(T, width + 4, generator=g), torch.randn(group, generator=g)
+    y, od, gd, wd = torch.empty(T, width, device="cuda"), o.cuda(), gate.cuda(), w.cuda()
+    rc = entry("illm_group_norm_gate_ex", I_, P_, I_, I_, I_, P_, I_, F_, P_, I_, I_, I_, P_, I_, P_, P_, I_, P_, I_, P_)(
+        p(od), T, width, group, p(wd), group, eps, p(gd), width + 4, act, 0, None, 0, None, None, 0, p(y), 0, stream())
+    assert rc == 0
+    v, z = o.double().numpy().reshape(T, -1, group), gate.double().numpy()[:, :width]
+    sig = 1.0 / (1.0 + np.exp(-z))
+    ref = (v / np.sqrt((v * v).mean(-1, keepdims=True) + eps) * w.double().numpy()).reshape(T, width) * (z * sig if act == 1 else sig)
+    close(y, ref, 2 * math.sqrt(group) + 24)
+
+
+@pytest.mark.parametrize("nh,nkv,d,dv,rot,pairs,norm,qt,mix,own", [
+    (8, 2, 128, 128, 64, 1, "whole", 0, False, True), (8, 2, 128, 128, 64, 1, "head", 0, False, True), (4, 4, 64, 96, 30, 0, "none", 4, False, True),
+    (5, 1, 36, 20, 36, 1, "none", 0, True, True), (6, 2, 16, 16, 6, 0, "head", 0, False, True), (16, 4, 128, 128, 128, 0, "whole", 0, False, False),
+    (32, 8, 128, 128, 0, 1, "none", 16, False, True), (3, 3, 4, 4, 4, 1, "whole", 0, True, True), (40, 40, 128, 128, 64, 1, "none", 0, False, True)])
+def test_qk_prep_by_pieces(nh, nkv, d, dv, rot, pairs, norm, qt, mix, own):
+    """Rows that begin on 16-byte boundaries (four channels per thread) and the same rows one float further on (the channel by channel
+    kernel) give the same values up to the order of a norm's sum."""
+    g = torch.Generator().manual_seed(nh * d + rot)
+    T, page, n_pos = 5, 8, 64
+    nq, nk, nv = nh * d, nkv * d, nkv * dv
+    cols = nq + (nk + nv if own else 0)
+    rnd = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    x, bq, bk, bv = rnd(T, cols), rnd(nq), rnd(nk), rnd(nv)
+    wq, wk = (rnd(nq), rnd(nk)) if norm == "whole" else (rnd(d), rnd(d))
+    cs, first, lam = rnd(n_pos, max(1, rot // 2), 2), rnd(T, nv), torch.tensor([0.3])
+    pos, seq = torch.tensor([0, 7, 8, 30, 63], dtype=torch.int32), torch.tensor([0, 0, 0, 1, 1], dtype=torch.int32)
+    table = torch.arange(16, dtype=torch.int32).view(2, 8).flip(0).contiguous()
+    f = entry("illm_qk_prep_heads", I_, P_, I_, I_, I_, I_, I_, I_, I_, I_, I_, P_, P_, P_, P_, P_, F_, P_, I_, I_, I_, P_, P_, P_, I_, I_, P_, P_, P_, I_, I_, P_, F_,
+              I_, P_, I_, P_, P_, I_, P_)
+    keep = [t.cuda() for t in (bq, bk, bv, wq, wk, cs, first, lam, pos, seq, table)]
+
+    def run(shift):
+        xd = torch.zeros(T, cols + 4, device="cuda")
+        xd[:, shift:shift + cols] = x.cuda()
+        q = torch.full((T, nq), float("nan"), device="cuda")
+        kc, vc = torch.zeros(16, nkv, page, d, device="cuda"), torch.zeros(16, nkv, page, dv, device="cuda")
+        kept, err = torch.zeros(T, nv, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        bqd, bkd, bvd, wqd, wkd, csd, fd, ld, pd, sd, td = keep
+        rc = f(p(xd), 0, cols + 4, shift, shift + nq if own else -1, shift + nq + nk if own else -1, nh, nkv, d, dv, p(bqd), p(bkd) if own else None,
+               p(bvd) if own else None, None if norm == "none" else p(wqd), None if norm == "none" or not own else p(wkd), 1e-5, p(csd), rot, pairs, n_pos, p(pd),
+               p(sd), p(td), 8, page, p(q), p(kc) if own else None, p(vc) if own else None, 0, T, p(err), 0.25, qt, p(fd) if mix else None, nv,
+               p(ld) if mix else None, p(kept) if mix else None, 1 if norm == "head" else 0, stream())
+        assert rc == 0 and int(err) == 0
+        return [t.cpu() for t in (q, kc, vc, kept)]
+
+    for a, b in zip(run(0), run(1)):
+        assert torch.isfinite(a).all()
+        assert (a - b).abs().max() <= (2 * math.sqrt(nq) + 8) * 2.0 ** -24 * max(1.0, float(b.abs().max()))
+    assert not own or float(run(0)[1].abs().sum()) > 0
+
+
+@pytest.mark.parametrize("nh,nkv,window,lens", [(4, 2, 0, [1, 63, 64, 65, 300]), (8, 1, 0, [129]), (3, 3, 70, [200, 5]), (2, 1, 1, [70])])
+def test_differential_attention_on_tensor_memory(nh, nkv, window, lens):
+    """Beside the warp-level MMA kernel, both against float64: no farther from it than that one by more than a half, and within two
+    bfloat16 roundings of the output."""
+    d, dv, page = 64, 128, 64
+    g = torch.Generator().manual_seed(nh + window)
+    T, B = sum(lens), len(lens)
+    width = max(-(-n // page) for n in lens) + 1
+    n_pages = B * width
+    table = torch.randperm(n_pages, generator=g).to(torch.int32).view(B, width)
+    q = (torch.randn(T, nh * 2 * d, generator=g)).bfloat16()
+    ks, vs = [torch.randn(n, nkv, 2 * d, generator=g).bfloat16() for n in lens], [torch.randn(n, nkv, dv, generator=g).bfloat16() for n in lens]
+    kc, vc = (torch.full((n_pages, nkv, page, w), float("nan"), dtype=torch.bfloat16) for w in (2 * d, dv))
+    for b, n in enumerate(lens):
+        for t in range(n):
+            kc[table[b, t // page], :, t % page], vc[table[b, t // page], :, t % page] = ks[b][t], vs[b][t]
+    cu = torch.tensor([0] + list(np.cumsum(lens)), dtype=torch.int32)
+    dev = [t.cuda() for t in (q, kc, vc, table.contiguous(), cu, torch.tensor(lens, dtype=torch.int32))]
+    scale, lam, eps, factor = d ** -0.5, 0.45, 1e-6, 0.6
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    maps = torch.empty(T, nh, 2, dv, device="cuda")
+    outs = [torch.full((T, nh * dv), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    rc = entry("illm_attention_diff_tc", I_, P_, I_, I_, P_, P_, L_, P_, I_, P_, P_, P_, P_, I_, I_, I_, I_, I_, I_, I_, I_, F_, F_, F_, F_, P_, P_)(
+        p(dev[0]), nh * 2 * d, T, p(dev[1]), p(dev[2]), n_pages, p(dev[3]), width, p(dev[4]), p(dev[5]), p(maps), p(outs[0]), B, max(lens), nh, nkv, d, dv, page,
+        window, scale, lam, eps, factor, p(err), stream())
+    assert rc == 0
+    rc = entry("illm_attention_diff_mma", I_, P_, I_, P_, P_, P_, I_, P_, P_, P_, I_, I_, I_, I_, I_, I_, I_, I_, F_, F_, F_, F_, P_)(
+        p(dev[0]), nh * 2 * d, p(dev[1]), p(dev[2]), p(dev[3]), width, p(dev[4]), p(dev[5]), p(outs[1]), B, max(lens), nh, nkv, d, dv, page, window, scale, lam, eps,
+        factor, stream())
+    assert rc == 0 and int(err) == 0
+    got, other = (o.cpu().double().numpy().reshape(T, nh, dv) for o in outs)
+    for b, n in enumerate(lens):
+        qq = q[cu[b]:cu[b + 1]].double().numpy().reshape(n, nh, 2, d)
+        i, j = np.arange(n)[:, None], np.arange(n)[None]
+        hide = (j > i) | ((i - j >= window) if window else False)
+        ref = np.zeros((n, nh, dv))
+        for h in range(nh):
+            k, v = ks[b][:, h // (nh // nkv)].double().numpy().reshape(n, 2, d), vs[b][:, h // (nh // nkv)].double().numpy()
+            a = []
+            for m in range(2):
+                s = np.where(hide, -np.inf, qq[:, h, m] @ k[:, m].T * scale)
+                e = np.exp(s - s.max(-1, keepdims=True))
+                a.append(e / e.sum(-1, keepdims=True) @ v)
+            o = a[0] - lam * a[1]
+            ref[:, h] = o / np.sqrt((o * o).mean(-1, keepdims=True) + eps) * factor
+        mine, theirs = (np.abs(x[cu[b]:cu[b + 1]] - ref) for x in (got, other))
+        assert (mine <= 2.0 ** -7 * np.abs(ref) + 2.0 ** -9).all()
+        assert np.linalg.norm(mine) <= 1.5 * np.linalg.norm(theirs) + 1e-6
