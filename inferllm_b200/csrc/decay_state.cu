@@ -592,6 +592,49 @@ __global__ void __launch_bounds__(256) group_norm_gate_vec_kernel(GroupNormGateA
     }
 }
 
+// The same for larger groups (a norm over all heads together): a block per (token, group), IT pieces of four neighbouring columns per
+// thread, everything on its way before the sum (one row of 2,048 took 18 us channel by channel, each pass waiting for
+// its own loads).
+template <typename TA, int IT>
+__global__ void __launch_bounds__(1024) group_norm_gate_row_kernel(GroupNormGateArgs a, TA* __restrict__ y) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    __shared__ float scratch[32];
+    const int t = blockIdx.x, g0 = blockIdx.y * a.group;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v[IT], gv[IT], wv[IT];
+#pragma unroll
+    for (int i = 0; i < IT; i++) {
+        const int c = 4 * (threadIdx.x + i * (int)blockDim.x);
+        wv[i] = a.w && c < a.group ? *reinterpret_cast<const float4*>(a.w + (g0 + c) % a.w_len) : make_float4(1.f, 1.f, 1.f, 1.f);
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < IT; i++) {
+        const int c = 4 * (threadIdx.x + i * (int)blockDim.x);
+        v[i] = c < a.group ? *reinterpret_cast<const float4*>(a.o + (size_t)t * a.width + g0 + c) : zero;
+        gv[i] = a.gate && c < a.group ? *reinterpret_cast<const float4*>(a.gate + (size_t)t * a.gate_ld + g0 + c) : zero;
+    }
+#pragma unroll
+    for (int i = 0; i < IT; i++) ss = fmaf(v[i].x, v[i].x, ss), ss = fmaf(v[i].y, v[i].y, ss), ss = fmaf(v[i].z, v[i].z, ss), ss = fmaf(v[i].w, v[i].w, ss);
+    ss = block_sum(ss, scratch);
+    const float inv = 1.0f / sqrtf(ss / (float)a.group + a.eps);
+#pragma unroll
+    for (int i = 0; i < IT; i++) {
+        const int c = 4 * (threadIdx.x + i * (int)blockDim.x);
+        if (c >= a.group) continue;
+        float r[4] = {(v[i].x * inv) * wv[i].x, (v[i].y * inv) * wv[i].y, (v[i].z * inv) * wv[i].z, (v[i].w * inv) * wv[i].w};
+        if (a.gate) r[0] *= act_of(gv[i].x, a.gate_act), r[1] *= act_of(gv[i].y, a.gate_act), r[2] *= act_of(gv[i].z, a.gate_act), r[3] *= act_of(gv[i].w, a.gate_act);
+        TA* out = y + (size_t)t * a.width + g0 + c;
+        if (sizeof(TA) == 4) {
+            *reinterpret_cast<float4*>(out) = make_float4(r[0], r[1], r[2], r[3]);
+        } else {
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(r[0], r[1]), hi = __floats2bfloat162_rn(r[2], r[3]);
+            *reinterpret_cast<uint2*>(out) = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
+        }
+    }
+}
+
 // w_len: the weight's length, the whole width or a divisor of it (a weight of one group's size is shared by the groups);
 // head: columns per entry of row_scale and skip_w (0 when neither is given)
 extern "C" int illm_group_norm_gate_ex(const float* o, int T, int width, int group, const float* w, int w_len, float eps, const float* gate,
@@ -619,6 +662,19 @@ extern "C" int illm_group_norm_gate_ex(const float* o, int T, int width, int gro
         else if (group <= 256) ILLM_GNG(2);
         else ILLM_GNG(4);
 #undef ILLM_GNG
+        return illm_launch_status();
+    }
+    if (!row_scale && !skip_w && !(gate && gate_first) && group % 4 == 0 && group <= 8192 && (!w || (w_len % 4 == 0 && !((uintptr_t)w & 15))) && !((uintptr_t)o & 15) &&
+        !((uintptr_t)y & 15) && (!gate || (gate_ld % 4 == 0 && !((uintptr_t)gate & 15))) && (act_dtype == ILLM_BF16 || act_dtype == ILLM_F32)) {
+        const int pieces = group / 4, threads = pieces < 1024 ? (pieces + 31) / 32 * 32 : 1024;
+#define ILLM_GNR(IT)                                                                                                          \
+    do {                                                                                                                      \
+        if (act_dtype == ILLM_BF16) illm_launch((group_norm_gate_row_kernel<bf16, IT>), grid, dim3(threads), 0, s, a, (bf16*)y);   \
+        else illm_launch((group_norm_gate_row_kernel<float, IT>), grid, dim3(threads), 0, s, a, (float*)y);                        \
+    } while (0)
+        if (pieces <= 1024) ILLM_GNR(1);
+        else ILLM_GNR(2);
+#undef ILLM_GNR
         return illm_launch_status();
     }
     if (act_dtype == ILLM_BF16) illm_launch(group_norm_gate_kernel<bf16>, grid, dim3(128), 0, s, a, (bf16*)y);

@@ -61,6 +61,16 @@ __global__ void embedding_scaled_kernel(const int* __restrict__ ids, const int* 
         return;
     }
     const TW* row = table + (size_t)id * H;
+    if (!inv_freq && (H & 7) == 0) {        // whole 16-byte pieces of a row that comes from memory: a thread's loads together
+        for (int c = threadIdx.x * 8; c < H; c += blockDim.x * 8) {
+            float v[8];
+            load8(row + c, v);
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] *= scale;
+            store8(o + c, v);
+        }
+        return;
+    }
     const float p = (float)token_pos[t];
     for (int c = threadIdx.x; c < H; c += blockDim.x) {
         float v = to_f32(row[c]) * scale;

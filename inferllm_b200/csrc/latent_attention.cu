@@ -116,15 +116,17 @@ latent_rope_prep_kernel(const float* __restrict__ x, int ld, int q_off, int H, i
     }
     const float* cs = rot ? cos_sin + (size_t)p * rot : nullptr;      // rot / 2 pairs of (cos, sin)
     auto turned = [&](const float* v, int e) { return latent_turned(v, e, rot, pairs, cs); };       // channel e of the dr-vector v
-    for (int i = threadIdx.x; i < H * d; i += blockDim.x) {
+    // the queries' channels are dealt to the blocks of the token (one in a step of many tokens), the cache row is the first block's
+    const int part = blockIdx.y * blockDim.x + threadIdx.x, step = gridDim.y * blockDim.x;
+    for (int i = part; i < H * d; i += step) {
         const int h = i / d, c = i - h * d;
         q_nope[(size_t)t * H * d + i] = from_f32<TQ>(row[q_off + h * (d + dr) + c]);
     }
-    for (int i = threadIdx.x; i < H * dr; i += blockDim.x) {
+    for (int i = part; i < H * dr; i += step) {
         const int h = i / dr, e = i - h * dr;
         qa[((size_t)t * H + h) * (R + dr) + R + e] = from_f32<TA>(turned(row + q_off + h * (d + dr) + d, e));
     }
-    if (!kc) return;
+    if (!kc || blockIdx.y) return;
     float sk = 0.f;
     for (int c = threadIdx.x; c < R; c += blockDim.x) sk = fmaf(row[c_off + c], row[c_off + c], sk);
     sk = block_sum(sk, scratch);
@@ -149,7 +151,7 @@ extern "C" int illm_latent_rope_prep(const float* x, int ld, int q_off, int H, i
     if (H <= 0 || d <= 0 || dr < 0 || R <= 0 || rot < 0 || rot > dr || (rot & 1) || (rot && !cos_sin) || !x || !q_nope || !qa || !wkv) return ILLM_ERR_BAD_ARG;
     cudaStream_t s = (cudaStream_t)stream;
 #define ILLM_LRP(TQ, TA)                                                                                                                 \
-    illm_launch(latent_rope_prep_kernel<TQ, TA>, dim3(T), dim3(256), 0, s, x, ld, q_off, H, d, dr, c_off, R, wkv, eps, cos_sin, rot, pairs, n_pos, \
+    illm_launch(latent_rope_prep_kernel<TQ, TA>, dim3(T, T <= 32 ? 8 : 1), dim3(256), 0, s, x, ld, q_off, H, d, dr, c_off, R, wkv, eps, cos_sin, rot, pairs, n_pos, \
                 token_pos, token_seq, block_table, max_pages, page_size, (TQ*)q_nope, (TA*)qa, (TA*)kc, err)
     if (act_dtype == ILLM_BF16 && q_f32) ILLM_LRP(float, bf16);
     else if (act_dtype == ILLM_BF16) ILLM_LRP(bf16, bf16);

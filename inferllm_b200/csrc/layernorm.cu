@@ -6,8 +6,7 @@
 //   n(v) = (v - mean(v)) / sqrt(mean((v - mean(v))^2) + eps)      CENTER (layer norm; a = 1)
 //   n(v) = v / sqrt(mean(v^2) + eps)                              otherwise (RMS norm)
 //
-// in one kernel, because the second norm reads the row the first one has just made.  One block per row, the row in
-// shared memory, every statistic of the layer norm in two passes (mean, then the mean squared deviation), the RMS norm's
+// in one kernel, because the second norm reads the row the first one has just made.  One block per row, every statistic of the layer norm in two passes (mean, then the mean squared deviation), the RMS norm's
 // in one, with a fixed order of the sums, all float32.  `rows` (int32) gathers: only those rows are made, and x is then left as it is (the model's
 // last norm, for the rows whose logits are wanted).
 #include "common.cuh"
@@ -19,11 +18,9 @@ __device__ __forceinline__ void ln_store4(bf16* o, float a, float b, float c, fl
     *reinterpret_cast<uint2*>(o) = make_uint2(lo, hi);
 }
 
-// V = 4: a thread takes four neighbouring channels at a time (the width a multiple of four); V = 1: any width.  A
-// thread's part of a sum is taken in the order of its channels in both; which of the two runs follows from the
-// width alone.
-template <typename TO, int V, bool CENTER>
-__global__ void __launch_bounds__(1024)
+// Any width, the row in shared memory, a channel per thread at a time.
+template <typename TO, bool CENTER>
+__global__ void __launch_bounds__(256)
 ln_sandwich_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ wb, const float* __restrict__ w,
                    TO* __restrict__ out, const int* __restrict__ rows, int H, float eps, float post_scale, int write_x) {
     pdl_grid_sync();
@@ -31,109 +28,125 @@ ln_sandwich_kernel(float* __restrict__ x, const float* __restrict__ y, const flo
     __shared__ float scratch[32];
     const int r = rows ? rows[blockIdx.x] : blockIdx.x;
     float* xr = x + (size_t)r * H;
-    const int first = threadIdx.x * V, step = blockDim.x * V;
-    if (y) {
-        const float* yr = y + (size_t)r * H;
-        float s = 0.f;
-        for (int c = first; c < H; c += step) {
-            if (V == 4) {
-                const float4 v = *reinterpret_cast<const float4*>(yr + c);
-                *reinterpret_cast<float4*>(row + c) = v;
-                if (CENTER) s += v.x, s += v.y, s += v.z, s += v.w;
-                else s = fmaf(v.x, v.x, s), s = fmaf(v.y, v.y, s), s = fmaf(v.z, v.z, s), s = fmaf(v.w, v.w, s);
-            } else {
-                const float v = yr[c];
-                row[c] = v;
-                s = CENTER ? s + v : fmaf(v, v, s);
-            }
-        }
-        float mean = 0.f, q = s;
+    // the mean (CENTER) and 1 / sqrt(the mean square of the deviation + eps) of what lies in `row`
+    auto statistics = [&](float& mean) {
+        mean = 0.f;
         if (CENTER) {
+            float s = 0.f;
+            for (int c = threadIdx.x; c < H; c += blockDim.x) s += row[c];
             mean = block_sum(s, scratch) / (float)H;
-            q = 0.f;
-            for (int c = first; c < H; c += step) {
-#pragma unroll
-                for (int i = 0; i < V; i++) {
-                    const float dlt = row[c + i] - mean;
-                    q = fmaf(dlt, dlt, q);
-                }
-            }
         }
-        const float inv = 1.0f / sqrtf(block_sum(q, scratch) / (float)H + eps);
-        for (int c = first; c < H; c += step) {
-            if (V == 4) {
-                const float4 xv = *reinterpret_cast<const float4*>(xr + c), wv = *reinterpret_cast<const float4*>(wb + c);
-                float4 v;
-                if (CENTER) {
-                    v.x = xv.x + ((row[c] - mean) * inv) * wv.x;
-                    v.y = xv.y + ((row[c + 1] - mean) * inv) * wv.y;
-                    v.z = xv.z + ((row[c + 2] - mean) * inv) * wv.z;
-                    v.w = xv.w + ((row[c + 3] - mean) * inv) * wv.w;
-                } else {
-                    v.x = fmaf(post_scale, (row[c] * inv) * wv.x, xv.x);
-                    v.y = fmaf(post_scale, (row[c + 1] * inv) * wv.y, xv.y);
-                    v.z = fmaf(post_scale, (row[c + 2] * inv) * wv.z, xv.z);
-                    v.w = fmaf(post_scale, (row[c + 3] * inv) * wv.w, xv.w);
-                }
-                *reinterpret_cast<float4*>(row + c) = v;
-                if (write_x) *reinterpret_cast<float4*>(xr + c) = v;
-            } else {
-                const float v = CENTER ? xr[c] + ((row[c] - mean) * inv) * wb[c] : fmaf(post_scale, (row[c] * inv) * wb[c], xr[c]);
-                row[c] = v;
-                if (write_x) xr[c] = v;
-            }
+        float q = 0.f;
+        for (int c = threadIdx.x; c < H; c += blockDim.x) {
+            const float dlt = row[c] - mean;
+            q = fmaf(dlt, dlt, q);
+        }
+        return 1.0f / sqrtf(block_sum(q, scratch) / (float)H + eps);
+    };
+    float mean;
+    if (y) {
+        for (int c = threadIdx.x; c < H; c += blockDim.x) row[c] = y[(size_t)r * H + c];
+        const float inv = statistics(mean);
+        for (int c = threadIdx.x; c < H; c += blockDim.x) {
+            const float v = fmaf(post_scale, ((row[c] - mean) * inv) * wb[c], xr[c]);
+            row[c] = v;
+            if (write_x) xr[c] = v;
         }
     } else {
-        for (int c = first; c < H; c += step) {
-            if (V == 4) *reinterpret_cast<float4*>(row + c) = *reinterpret_cast<const float4*>(xr + c);
-            else row[c] = xr[c];
+        for (int c = threadIdx.x; c < H; c += blockDim.x) row[c] = xr[c];
+    }
+    if (!out) return;
+    const float inv = statistics(mean);
+    TO* o = out + (size_t)blockIdx.x * H;
+    for (int c = threadIdx.x; c < H; c += blockDim.x) o[c] = from_f32<TO>(((row[c] - mean) * inv) * w[c]);
+}
+
+// Rows of whole 16-byte pieces up to 16,384 wide: IT pieces per thread in registers.  Both rows and both weights are on
+// their way before the first sum (the weights while the kernel before drains), so that a single token's block, which
+// is bound by latency alone, waits for memory once (a row of 4,096 took 6.3 us with the row going through shared
+// memory and the stream and the weights asked for behind the first sum).
+template <typename TO, int IT, bool CENTER>
+__global__ void __launch_bounds__(1024)
+ln_sandwich_vec_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ wb, const float* __restrict__ w,
+                       TO* __restrict__ out, const int* __restrict__ rows, int H, float eps, float post_scale, int write_x) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    __shared__ float scratch[32];
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v[IT], yv[IT], wv[IT], wbv[IT];
+#pragma unroll
+    for (int i = 0; i < IT; i++) {
+        const int c = 4 * (threadIdx.x + i * (int)blockDim.x);
+        wbv[i] = y && c < H ? *reinterpret_cast<const float4*>(wb + c) : zero;
+        wv[i] = out && c < H ? *reinterpret_cast<const float4*>(w + c) : zero;
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int r = rows ? rows[blockIdx.x] : blockIdx.x;
+    float* xr = x + (size_t)r * H;
+#pragma unroll
+    for (int i = 0; i < IT; i++) {
+        const int c = 4 * (threadIdx.x + i * (int)blockDim.x);
+        v[i] = c < H ? *reinterpret_cast<const float4*>(xr + c) : zero;
+        yv[i] = y && c < H ? *reinterpret_cast<const float4*>(y + (size_t)r * H + c) : zero;
+    }
+    // the mean (CENTER) and 1 / sqrt(the mean square of the deviation + eps) of a row; pieces beyond it count for nothing
+    auto statistics = [&](const float4 (&a)[IT], float& mean) {
+        mean = 0.f;
+        float s = 0.f;
+        if (CENTER) {
+#pragma unroll
+            for (int i = 0; i < IT; i++) s += a[i].x, s += a[i].y, s += a[i].z, s += a[i].w;
+            mean = block_sum(s, scratch) / (float)H;
+            s = 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < IT; i++) {
+            if (CENTER && 4 * (threadIdx.x + i * (int)blockDim.x) >= (unsigned)H) continue;
+            const float dx = a[i].x - mean, dy = a[i].y - mean, dz = a[i].z - mean, dw = a[i].w - mean;
+            s = fmaf(dx, dx, s), s = fmaf(dy, dy, s), s = fmaf(dz, dz, s), s = fmaf(dw, dw, s);
+        }
+        return 1.0f / sqrtf(block_sum(s, scratch) / (float)H + eps);
+    };
+    float mean;
+    if (y) {
+        const float inv = statistics(yv, mean);
+#pragma unroll
+        for (int i = 0; i < IT; i++) {
+            const int c = 4 * (threadIdx.x + i * (int)blockDim.x);
+            if (c >= H) continue;
+            v[i].x = fmaf(post_scale, ((yv[i].x - mean) * inv) * wbv[i].x, v[i].x);
+            v[i].y = fmaf(post_scale, ((yv[i].y - mean) * inv) * wbv[i].y, v[i].y);
+            v[i].z = fmaf(post_scale, ((yv[i].z - mean) * inv) * wbv[i].z, v[i].z);
+            v[i].w = fmaf(post_scale, ((yv[i].w - mean) * inv) * wbv[i].w, v[i].w);
+            if (write_x) *reinterpret_cast<float4*>(xr + c) = v[i];
         }
     }
     if (!out) return;
-    float mean = 0.f;
-    if (CENTER) {
-        float s = 0.f;
-        for (int c = first; c < H; c += step) {
-#pragma unroll
-            for (int i = 0; i < V; i++) s += row[c + i];
-        }
-        mean = block_sum(s, scratch) / (float)H;
-    }
-    float q = 0.f;
-    for (int c = first; c < H; c += step) {
-#pragma unroll
-        for (int i = 0; i < V; i++) {
-            const float dlt = row[c + i] - mean;
-            q = fmaf(dlt, dlt, q);
-        }
-    }
-    const float inv = 1.0f / sqrtf(block_sum(q, scratch) / (float)H + eps);
+    const float inv = statistics(v, mean);
     TO* o = out + (size_t)blockIdx.x * H;
-    for (int c = first; c < H; c += step) {
-        if (V == 4) {
-            const float4 wv = *reinterpret_cast<const float4*>(w + c);
-            ln_store4(o + c, ((row[c] - mean) * inv) * wv.x, ((row[c + 1] - mean) * inv) * wv.y, ((row[c + 2] - mean) * inv) * wv.z,
-                      ((row[c + 3] - mean) * inv) * wv.w);
-        } else {
-            o[c] = from_f32<TO>(((row[c] - mean) * inv) * w[c]);
-        }
+#pragma unroll
+    for (int i = 0; i < IT; i++) {
+        const int c = 4 * (threadIdx.x + i * (int)blockDim.x);
+        if (c < H)
+            ln_store4(o + c, ((v[i].x - mean) * inv) * wv[i].x, ((v[i].y - mean) * inv) * wv[i].y, ((v[i].z - mean) * inv) * wv[i].z,
+                      ((v[i].w - mean) * inv) * wv[i].w);
     }
 }
 
 template <typename TO, bool CENTER>
 static void ln_launch(float* x, const float* y, const float* wb, const float* w, TO* out, const int* rows, int n_rows, int H, float eps,
                       float post_scale, int write_x, cudaStream_t s) {
-    const size_t smem = (size_t)H * sizeof(float);
-    // a thread per four channels up to 512 threads: a step of few rows is a few blocks, each bound by the latency of its
-    // passes.  The block's size follows from the width alone, so a row's sums have one order in every step.
-    if (H % 4 == 0) {
-        const int threads = H >= 2048 ? 512 : H >= 1024 ? 256 : 128;
-        if (smem > 48 * 1024) cudaFuncSetAttribute(ln_sandwich_kernel<TO, 4, CENTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        illm_launch((ln_sandwich_kernel<TO, 4, CENTER>), dim3(n_rows), dim3(threads), smem, s, x, y, wb, w, out, rows, H, eps, post_scale, write_x);
-    } else {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(ln_sandwich_kernel<TO, 1, CENTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        illm_launch((ln_sandwich_kernel<TO, 1, CENTER>), dim3(n_rows), dim3(256), smem, s, x, y, wb, w, out, rows, H, eps, post_scale, write_x);
+    // which kernel runs and its threads follow from the width and the layout alone, so a row's sums have one order in every step
+    auto aligned = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
+    if (H % 4 == 0 && H <= 16384 && aligned(x) && aligned(y) && aligned(wb) && aligned(w) && aligned(out)) {
+        const int pieces = H / 4, threads = pieces < 1024 ? (pieces + 31) / 32 * 32 : 1024;
+        if (pieces <= 1024) illm_launch((ln_sandwich_vec_kernel<TO, 1, CENTER>), dim3(n_rows), dim3(threads), 0, s, x, y, wb, w, out, rows, H, eps, post_scale, write_x);
+        else if (pieces <= 2048) illm_launch((ln_sandwich_vec_kernel<TO, 2, CENTER>), dim3(n_rows), dim3(threads), 0, s, x, y, wb, w, out, rows, H, eps, post_scale, write_x);
+        else illm_launch((ln_sandwich_vec_kernel<TO, 4, CENTER>), dim3(n_rows), dim3(threads), 0, s, x, y, wb, w, out, rows, H, eps, post_scale, write_x);
+        return;
     }
+    const size_t smem = (size_t)H * sizeof(float);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(ln_sandwich_kernel<TO, CENTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    illm_launch((ln_sandwich_kernel<TO, CENTER>), dim3(n_rows), dim3(256), smem, s, x, y, wb, w, out, rows, H, eps, post_scale, write_x);
 }
 
 // y, wb: nullptr for no addition; w, out: nullptr for the addition alone; rows: nullptr for rows 0 .. n_rows - 1;

@@ -142,6 +142,173 @@ __global__ void __launch_bounds__(256) qk_prep_kernel(QkPrepArgs a) {
     }
 }
 
+// The same for rows of whole 16-byte pieces (sizes, offsets and strides of four channels): a thread holds IT pieces of four
+// neighbouring channels of q, k and v in registers.  All its loads, the weights, biases, the value to mix in and the page's
+// number among them, are on their way before the first sum, because a single token's block is bound by nothing but the
+// latency of its dependent loads: the kernel above, which walks the channels one by one in five passes over shared memory,
+// took 13 to 17 us for one token of 32 + 2 x 8 heads of 128.  A head's norm is added within the d / 4 lanes that hold the head (d / 4 a power
+// of two up to 32).  Only the rotate-half layout, whose channels pair up across threads, goes through shared memory.
+// The block size follows from the sizes alone, so that a row's sums have one order in every step.
+template <typename TI> __device__ __forceinline__ float4 qk_load4(const TI* p);
+template <> __device__ __forceinline__ float4 qk_load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
+template <> __device__ __forceinline__ float4 qk_load4<bf16>(const bf16* p) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void qk_store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void qk_store4(bf16* p, float4 v) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
+}
+
+template <typename TI, typename TA, int IT>
+__global__ void __launch_bounds__(1024) qk_prep_vec_kernel(const QkPrepArgs a) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    extern __shared__ __align__(16) float buf[];      // the rotate-half layout: [nh d] q, then [nkv d] k
+    __shared__ float scratch[32];
+    const int t = blockIdx.x, threads = blockDim.x, d4 = a.d >> 2;
+    const int nq4 = a.nh * d4, nk4 = a.k_off >= 0 ? a.nkv * d4 : 0, nv4 = nk4 && a.v_off >= 0 && a.kc ? a.nkv * (a.dv >> 2) : 0;
+    const bool whole = a.wq && !a.head_norm, halves = a.rot && !a.pairs;
+    // weights, biases and the indices of the step are no result of the kernel before
+    const int pos = a.token_pos[t];
+    float4 w[IT], bias[IT];
+#pragma unroll
+    for (int i = 0; i < IT; i++) {
+        const int at = threadIdx.x + i * threads;
+        const bool is_q = at < nq4, is_k = !is_q && at < nq4 + nk4;
+        const int c = is_q ? at : is_k ? at - nq4 : at - nq4 - nk4;
+        const float* wp = is_q ? a.wq : is_k ? a.wk : nullptr;
+        const float* bp = is_q ? a.bq : is_k ? a.bk : a.bv;
+        const bool in = at < nq4 + nk4 + nv4;
+        w[i] = in && wp ? *reinterpret_cast<const float4*>(wp + 4 * (a.head_norm ? c % d4 : c)) : make_float4(1.f, 1.f, 1.f, 1.f);
+        bias[i] = in && bp ? *reinterpret_cast<const float4*>(bp + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const int page = nk4 && a.kc ? a.block_table[(size_t)a.token_seq[t] * a.max_pages + pos / a.page_size] : -1;
+    int p = pos;
+    if (a.rot && (p < 0 || p >= a.n_pos)) {
+        if (threadIdx.x == 0) atomicExch(a.err, 3);
+        p = 0;
+    }
+    const float* cs = a.rot ? a.cos_sin + (size_t)p * a.rot : nullptr;      // rot / 2 pairs of (cos, sin)
+    const float q_temp = a.qt_every > 0 ? 1.0f + a.qt_coef * logf((float)((pos + 1) / a.qt_every + 1)) : 1.0f;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const TI* x = (const TI*)a.x + (size_t)t * a.ld;
+    const float lambda = a.v_first ? *a.v_lambda : 0.f;
+    float4 v[IT], first[IT];
+#pragma unroll
+    for (int i = 0; i < IT; i++) {
+        const int at = threadIdx.x + i * threads;
+        const bool is_q = at < nq4, is_k = !is_q && at < nq4 + nk4, is_v = !is_q && !is_k && at < nq4 + nk4 + nv4;
+        const int c = is_q ? at : is_k ? at - nq4 : at - nq4 - nk4, off = is_q ? a.q_off : is_k ? a.k_off : a.v_off;
+        v[i] = is_q || is_k || is_v ? qk_load4(x + off + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        first[i] = is_v && a.v_first ? *reinterpret_cast<const float4*>(a.v_first + (size_t)t * a.v_first_ld + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float ssq = 0.f, ssk = 0.f;
+#pragma unroll
+    for (int i = 0; i < IT; i++) {
+        const int at = threadIdx.x + i * threads;
+        v[i].x += bias[i].x, v[i].y += bias[i].y, v[i].z += bias[i].z, v[i].w += bias[i].w;
+        if (at < nq4 && a.qt_every > 0) v[i].x *= q_temp, v[i].y *= q_temp, v[i].z *= q_temp, v[i].w *= q_temp;
+        float s = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, v[i].w * v[i].w)));
+        if (a.head_norm) {          // every head by itself; the lanes beyond k add among themselves what nobody uses
+            for (int o = 1; o < d4; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (at < nq4 + nk4) {
+                const float inv = 1.0f / sqrtf(s / (float)a.d + a.eps);
+                v[i].x = (v[i].x * inv) * w[i].x, v[i].y = (v[i].y * inv) * w[i].y, v[i].z = (v[i].z * inv) * w[i].z, v[i].w = (v[i].w * inv) * w[i].w;
+            }
+        }
+        if (at < nq4) ssq += s;
+        else if (at < nq4 + nk4) ssk += s;
+    }
+    if (whole) {
+        ssq = block_sum(ssq, scratch);
+        if (nk4 && a.wk) ssk = block_sum(ssk, scratch);
+        const float inv_q = 1.0f / sqrtf(ssq / (float)(4 * nq4) + a.eps), inv_k = nk4 ? 1.0f / sqrtf(ssk / (float)(4 * nk4) + a.eps) : 0.f;
+#pragma unroll
+        for (int i = 0; i < IT; i++) {
+            const int at = threadIdx.x + i * threads;
+            if (at >= nq4 && (at >= nq4 + nk4 || !a.wk)) continue;
+            const float inv = at < nq4 ? inv_q : inv_k;
+            v[i].x = (v[i].x * inv) * w[i].x, v[i].y = (v[i].y * inv) * w[i].y, v[i].z = (v[i].z * inv) * w[i].z, v[i].w = (v[i].w * inv) * w[i].w;
+        }
+    }
+    if (halves) {
+#pragma unroll
+        for (int i = 0; i < IT; i++) {
+            const int at = threadIdx.x + i * threads;
+            if (at < nq4 + nk4) *reinterpret_cast<float4*>(buf + 4 * at) = v[i];
+        }
+        __syncthreads();
+    }
+    if (page < 0 && nk4 && a.kc && threadIdx.x == 0) atomicExch(a.err, 2);
+    const int slot = pos % a.page_size;
+#pragma unroll
+    for (int i = 0; i < IT; i++) {
+        const int at = threadIdx.x + i * threads;
+        if (at >= nq4 + nk4 + nv4) continue;
+        if (at < nq4 + nk4) {
+            const int c = at < nq4 ? at : at - nq4, hd = c / d4, e = (c - hd * d4) * 4;
+            if (e < a.rot) {
+                if (a.pairs) {
+                    const float4 f = *reinterpret_cast<const float4*>(cs + e);      // cos, sin of the two pairs
+                    v[i] = make_float4(v[i].x * f.x - v[i].y * f.y, v[i].y * f.x + v[i].x * f.y, v[i].z * f.z - v[i].w * f.w, v[i].w * f.z + v[i].z * f.w);
+                } else {
+                    const float* head = buf + 4 * (at - (c - hd * d4));
+                    v[i].x = rotated(head, e, a.rot, 0, cs);
+                    if (e + 1 < a.rot) v[i].y = rotated(head, e + 1, a.rot, 0, cs);
+                    if (e + 2 < a.rot) v[i].z = rotated(head, e + 2, a.rot, 0, cs);
+                    if (e + 3 < a.rot) v[i].w = rotated(head, e + 3, a.rot, 0, cs);
+                }
+            }
+            if (at < nq4) qk_store4((TA*)a.q_out + (size_t)t * 4 * nq4 + 4 * c, v[i]);
+            else if (a.kc && page >= 0) qk_store4((TA*)a.kc + (((size_t)page * a.nkv + hd) * a.page_size + slot) * a.d + e, v[i]);
+        } else if (page >= 0) {
+            const int c = at - nq4 - nk4, hd = c / (a.dv >> 2), e = (c - hd * (a.dv >> 2)) * 4;
+            if (a.v_keep) *reinterpret_cast<float4*>(a.v_keep + (size_t)t * 4 * nv4 + 4 * c) = v[i];
+            if (a.v_first)
+                v[i] = make_float4((1.0f - lambda) * v[i].x + lambda * first[i].x, (1.0f - lambda) * v[i].y + lambda * first[i].y,
+                                   (1.0f - lambda) * v[i].z + lambda * first[i].z, (1.0f - lambda) * v[i].w + lambda * first[i].w);
+            qk_store4((TA*)a.vc + (((size_t)page * a.nkv + hd) * a.page_size + slot) * a.dv + e, v[i]);
+        }
+    }
+}
+
+// Whether the rows are whole 16-byte pieces throughout, and the norm of a head lies within a warp.
+static bool qk_prep_vec_takes(const QkPrepArgs& a) {
+    auto odd = [](const void* p) { return ((uintptr_t)p & 15) != 0; };
+    if ((a.d | a.dv | a.ld | a.q_off) & 3) return false;
+    if (a.k_off >= 0 && (a.k_off & 3)) return false;
+    if (a.v_off >= 0 && (a.v_off & 3)) return false;
+    if (a.pairs && (a.rot & 3)) return false;
+    if (odd(a.x) || odd(a.q_out) || odd(a.kc) || odd(a.vc) || odd(a.bq) || odd(a.bk) || odd(a.bv) || odd(a.wq) || odd(a.wk) || odd(a.cos_sin) ||
+        odd(a.v_keep) || odd(a.v_first) || (a.v_first && (a.v_first_ld & 3)))
+        return false;
+    if (a.wk && !a.wq) return false;
+    if (a.head_norm && (a.d / 4 > 32 || (a.d / 4 & (a.d / 4 - 1)))) return false;
+    return true;
+}
+
+template <typename TI, typename TA>
+static int qk_prep_vec_launch(const QkPrepArgs& a, int T, cudaStream_t s) {
+    const int pieces = (a.nh * a.d + (a.k_off >= 0 ? a.nkv * (a.d + (a.v_off >= 0 ? a.dv : 0)) : 0)) / 4;
+    const int iters = pieces <= 1024 ? 1 : pieces <= 2048 ? 2 : pieces <= 4096 ? 4 : 0;
+    if (!iters) return -1;
+    const int threads = ((pieces + iters - 1) / iters + 31) / 32 * 32;
+    const size_t smem = a.rot && !a.pairs ? (size_t)(a.nh + (a.k_off >= 0 ? a.nkv : 0)) * a.d * sizeof(float) : 0;
+    if (smem > 200 * 1024) return -1;
+#define ILLM_QKV(IT)                                                                                                                          \
+    do {                                                                                                                                      \
+        if (smem > 48 * 1024) cudaFuncSetAttribute(qk_prep_vec_kernel<TI, TA, IT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
+        illm_launch(qk_prep_vec_kernel<TI, TA, IT>, dim3(T), dim3(threads), smem, s, a);                                                       \
+    } while (0)
+    if (iters == 1) ILLM_QKV(1);
+    else if (iters == 2) ILLM_QKV(2);
+    else ILLM_QKV(4);
+#undef ILLM_QKV
+    return illm_launch_status();
+}
+
 // the same with a temperature on the queries that grows with the position (qt_every 0: none), applied behind the bias
 extern "C" int illm_qk_prep_ex(const void* x, int x_dtype, int ld, int q_off, int k_off, int v_off, int nh, int nkv, int d, int dv, const float* bq,
                                const float* bk, const float* bv, const float* wq, const float* wk, float eps, const float* cos_sin, int rot,
@@ -200,6 +367,13 @@ extern "C" int illm_qk_prep_heads(const void* x, int x_dtype, int ld, int q_off,
     const size_t smem = (size_t)(nh * d + (k_off >= 0 ? nkv * d : 0)) * sizeof(float);
     if (smem > 200 * 1024) return ILLM_ERR_BAD_ARG;
     cudaStream_t s = (cudaStream_t)stream;
+    if (qk_prep_vec_takes(a)) {
+        int rc = -1;
+        if (x_dtype == ILLM_F32 && act_dtype == ILLM_BF16) rc = qk_prep_vec_launch<float, bf16>(a, T, s);
+        else if (x_dtype == ILLM_F32 && act_dtype == ILLM_F32) rc = qk_prep_vec_launch<float, float>(a, T, s);
+        else if (x_dtype == ILLM_BF16 && act_dtype == ILLM_BF16) rc = qk_prep_vec_launch<bf16, bf16>(a, T, s);
+        if (rc >= 0) return rc;
+    }
 #define ILLM_QKP(TI, TA)                                                                                                    \
     do {                                                                                                                    \
         if (smem > 48 * 1024) cudaFuncSetAttribute(qk_prep_kernel<TI, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
