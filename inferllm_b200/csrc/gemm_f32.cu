@@ -10,8 +10,8 @@
 // buffers (k-major, so that the columns of a pair lie side by side), the next slice on its way to registers while
 // this one is used, one barrier per slice.  What bounds it is the float32 FMA rate: two neighbouring columns share
 // one packed fma.rn.f32x2 (each half rounded like a scalar fused multiply-add, so the chain per output and its bits
-// stay what they were), and an 8 x 8 thread tile reads 64 bytes of shared memory per 32 packed instructions, its
-// warp covering 32 x 64 outputs so that each 16-byte read is one conflict-free pass.
+// stay what they were), and the large tile's 8 x 16 outputs a thread read 96 bytes of shared memory per 64 packed
+// instructions, the lanes of a warp (4 along the rows by 8 along the columns) each 16-byte read in one pass.
 #include "tc_common.cuh"
 
 #define GF_BK 16
@@ -64,10 +64,10 @@ struct GfSlice {
     }
 };
 
-// A warp is 4 threads along the rows by 8 along the columns; a thread's rows and columns are pieces of four, a warp's
-// tile apart.  TM, TN: 4 or 8.
+// A warp is 4 threads along the rows by 8 along the columns; a thread's rows and columns are pieces of four, 16 rows and 32
+// columns apart.  TM: 4 or 8, TN: 4, 8 or 16.
 template <int BM, int BN, int TM, int TN>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN), BM * BN >= 128 * 128 ? 2 : 4)
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), TM * TN >= 64 ? 2 : 4)
 gemm_f32_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
                    int M, int N, int K, int lda, int ldw, int ldc) {
     constexpr int THREADS = (BM / TM) * (BN / TN), WARPS_N = BN / (8 * TN);
@@ -309,11 +309,16 @@ extern "C" int illm_gemm_f32_nt(const float* A, const float* W, float* C, int M,
         if (M <= 4) return launch_gemm_f32_small<4>(A, W, C, M, N, K, lda, ldw, ldc, err, s);
         return launch_gemm_f32_small<8>(A, W, C, M, N, K, lda, ldw, ldc, err, s);
     }
-    // The larger tile needs half the shared-memory traffic per FMA; the smaller ones run where the larger would leave
-    // SMs without a block, or where most of its rows lie beyond M.
+    // A larger thread tile reads less shared memory per FMA, a smaller block leaves fewer SMs idle in the last round and fewer
+    // rows beyond M: the tile with the least work on the busiest SM, per output 1 : 1.2 : 1.6 (512 rows of 7B size: Q/K/V and
+    // gate/up 49 TF/s with 8 x 16 outputs a thread against 44 with 8 x 8).  Where an SM gets one block of the large tile, 256
+    // threads of 8 x 8 outputs hide more than 128 of 8 x 16 (output and down products 39 TF/s; 64 x 128 tiles 28).
     cudaStream_t s = (cudaStream_t)stream;
-    auto blocks = [&](long long bm, long long bn) { return ((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
-    if (M > 64 && blocks(128, 128) >= 120) return launch_gemm_f32_tile<128, 128, 8, 8>(A, W, C, M, N, K, lda, ldw, ldc, s);
-    if (M > 32 && blocks(64, 64) >= 120) return launch_gemm_f32_tile<64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
+    const int sms = illm_sm_count();
+    auto rounds = [&](long long bm, long long bn) { return (double)(((M + bm - 1) / bm * ((N + bn - 1) / bn) + sms - 1) / sms); };
+    const double r0 = rounds(128, 128), c0 = r0 * 128 * 128, c1 = rounds(64, 64) * 64 * 64 * 1.2, c2 = rounds(32, 64) * 32 * 64 * 1.6;
+    if (c0 <= c1 && c0 <= c2)
+        return r0 < 2 ? launch_gemm_f32_tile<128, 128, 8, 8>(A, W, C, M, N, K, lda, ldw, ldc, s) : launch_gemm_f32_tile<128, 128, 8, 16>(A, W, C, M, N, K, lda, ldw, ldc, s);
+    if (c1 <= c2) return launch_gemm_f32_tile<64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
     return launch_gemm_f32_tile<32, 64, 4, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
 }
