@@ -35,7 +35,7 @@
 #include <type_traits>
 
 #include "chunk_scan.h"
-#include "common.cuh"
+#include "row_ops.cuh"
 
 #define DS_THREADS 128
 #define DS_MAX_TILE 16
@@ -107,6 +107,59 @@ __global__ void __launch_bounds__(128) decay_prep_kernel(DecayScanArgs a) {
     if (a.v_act) {
         float* v = row + a.v_off + h * a.dv;
         for (int c = threadIdx.x; c < a.dv; c += blockDim.x) v[c] = act_of(v[c], a.v_act);
+    }
+}
+
+// The same for rows of whole 16-byte pieces whose heads are rotated whole or not at all: a thread takes four channels of a head's
+// lower half and the four they are rotated with, of q, k and v, all six loads on their way together (channel by
+// channel, each pair waiting for its own loads, the kernel above took 138 us for 16,364 tokens of 8 heads of 128: 400 MB).
+__global__ void __launch_bounds__(256) decay_prep_vec_kernel(DecayScanArgs a, int T) {
+    pdl_grid_sync();
+    const int per = a.d >> 3, half = a.d >> 1;
+    const long long item = (long long)blockIdx.x * 256 + threadIdx.x;
+    const long long th = item / per;
+    const int t = (int)(th / a.nh), h = (int)(th - (long long)t * a.nh), c = (int)(item - th * per) * 4;
+    if (t >= T) return;
+    float* row = a.x + (size_t)t * a.ld;
+    float4* q = reinterpret_cast<float4*>(row + a.q_off + h * a.d + c);
+    float4* k = reinterpret_cast<float4*>(row + a.k_off + h * a.d + c);
+    float4* v = reinterpret_cast<float4*>(row + a.v_off + h * a.dv + c);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 q1 = q[0], q2 = q[half / 4], k1 = k[0], k2 = k[half / 4], v1 = a.v_act ? v[0] : zero, v2 = a.v_act ? v[half / 4] : zero;
+    auto act4 = [](float4& x, int act) { x = make_float4(act_of(x.x, act), act_of(x.y, act), act_of(x.z, act), act_of(x.w, act)); };
+    act4(q1, a.qk_act), act4(q2, a.qk_act), act4(k1, a.qk_act), act4(k2, a.qk_act);
+    if (a.rot) {
+        int p = a.token_pos[t];
+        if (p < 0 || p >= a.n_pos) {
+            atomicExch(a.err, 3);
+            p = 0;
+        }
+        const float4* f = reinterpret_cast<const float4*>(a.cos_sin + ((size_t)p * half + c) * 2);
+        const float4 f0 = f[0], f1 = f[1];              // (cos, sin) of the four pairs
+        auto turn = [&](float4& lo, float4& hi) {
+            const float4 l = lo, u = hi;
+            lo = make_float4(rot_val(l.x, u.x, f0.x, f0.y, true), rot_val(l.y, u.y, f0.z, f0.w, true), rot_val(l.z, u.z, f1.x, f1.y, true), rot_val(l.w, u.w, f1.z, f1.w, true));
+            hi = make_float4(rot_val(u.x, l.x, f0.x, f0.y, false), rot_val(u.y, l.y, f0.z, f0.w, false), rot_val(u.z, l.z, f1.x, f1.y, false),
+                             rot_val(u.w, l.w, f1.z, f1.w, false));
+        };
+        turn(q1, q2), turn(k1, k2);
+    }
+    auto scale4 = [&](float4& x) { x = make_float4(x.x * a.k_scale, x.y * a.k_scale, x.z * a.k_scale, x.w * a.k_scale); };
+    scale4(k1), scale4(k2);
+    q[0] = q1, q[half / 4] = q2, k[0] = k1, k[half / 4] = k2;
+    if (a.v_act) {
+        act4(v1, a.v_act), act4(v2, a.v_act);
+        v[0] = v1, v[half / 4] = v2;
+    }
+}
+
+static void decay_prep_launch(const DecayScanArgs& a, int T, cudaStream_t s) {
+    auto odd = [](const void* p) { return ((uintptr_t)p & 15) != 0; };
+    if (a.d % 8 == 0 && (a.rot == 0 || a.rot == a.d) && (!a.v_act || a.dv == a.d) && !((a.ld | a.q_off | a.k_off | a.v_off) & 3) && !odd(a.x) && !odd(a.cos_sin)) {
+        const long long items = (long long)T * a.nh * (a.d / 8);
+        illm_launch(decay_prep_vec_kernel, dim3((unsigned)((items + 255) / 256)), dim3(256), 0, s, a, T);
+    } else {
+        illm_launch(decay_prep_kernel, dim3(T, a.nh), dim3(128), 0, s, a);
     }
 }
 
@@ -450,7 +503,7 @@ extern "C" int illm_decay_scan(float* x, int T, int ld, int q_off, int k_off, in
     cudaStream_t s = (cudaStream_t)stream;
     // a step of few tokens (single tokens of a batch) is not worth a launch of its own for the preparation
     a.inline_prep = T <= 64 ? 1 : 0;
-    if (!a.inline_prep && (qk_act || v_act || rot || k_scale != 1.0f)) illm_launch(decay_prep_kernel, dim3(T, nh), dim3(128), 0, s, a);
+    if (!a.inline_prep && (qk_act || v_act || rot || k_scale != 1.0f)) decay_prep_launch(a, T, s);
     decay_launch_for<false>(a, B, s);
     return illm_launch_status();
 }
@@ -472,7 +525,7 @@ extern "C" int illm_decay_chunk_scan(float* x, int T, int ld, int q_off, int k_o
     if (qk_act || v_act || rot || k_scale != 1.0f) {
         DecayScanArgs a{x, ld, q_off, k_off, v_off, nh, d, dv, qk_act, v_act, cos_sin, rot, n_pos, k_scale, decay, state, slots, cu_q, token_pos, out, err,
                         0, 0, 0, 1, nullptr, nullptr, nullptr, 1, (long long)nh * d * dv, nullptr};
-        illm_launch(decay_prep_kernel, dim3(T, nh), dim3(128), 0, s, a);
+        decay_prep_launch(a, T, s);
     }
     const ChunkScanArgs c{x + q_off, x + k_off, x + v_off, ld, decay, nullptr, nh, 1, d, dv, state, (long long)nh * d * dv, slots, cu_q, rec, out, segments,
                           segments > 1 ? rec + (chunk_scan_scratch(T, B, nh) + 63) / 64 * 64 : nullptr};
@@ -625,13 +678,7 @@ __global__ void __launch_bounds__(1024) group_norm_gate_row_kernel(GroupNormGate
         if (c >= a.group) continue;
         float r[4] = {(v[i].x * inv) * wv[i].x, (v[i].y * inv) * wv[i].y, (v[i].z * inv) * wv[i].z, (v[i].w * inv) * wv[i].w};
         if (a.gate) r[0] *= act_of(gv[i].x, a.gate_act), r[1] *= act_of(gv[i].y, a.gate_act), r[2] *= act_of(gv[i].z, a.gate_act), r[3] *= act_of(gv[i].w, a.gate_act);
-        TA* out = y + (size_t)t * a.width + g0 + c;
-        if (sizeof(TA) == 4) {
-            *reinterpret_cast<float4*>(out) = make_float4(r[0], r[1], r[2], r[3]);
-        } else {
-            const __nv_bfloat162 lo = __floats2bfloat162_rn(r[0], r[1]), hi = __floats2bfloat162_rn(r[2], r[3]);
-            *reinterpret_cast<uint2*>(out) = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
-        }
+        row_store4(y + (size_t)t * a.width + g0 + c, make_float4(r[0], r[1], r[2], r[3]));
     }
 }
 
@@ -666,13 +713,13 @@ extern "C" int illm_group_norm_gate_ex(const float* o, int T, int width, int gro
     }
     if (!row_scale && !skip_w && !(gate && gate_first) && group % 4 == 0 && group <= 8192 && (!w || (w_len % 4 == 0 && !((uintptr_t)w & 15))) && !((uintptr_t)o & 15) &&
         !((uintptr_t)y & 15) && (!gate || (gate_ld % 4 == 0 && !((uintptr_t)gate & 15))) && (act_dtype == ILLM_BF16 || act_dtype == ILLM_F32)) {
-        const int pieces = group / 4, threads = pieces < 1024 ? (pieces + 31) / 32 * 32 : 1024;
+        const int threads = row_threads(group);
 #define ILLM_GNR(IT)                                                                                                          \
     do {                                                                                                                      \
         if (act_dtype == ILLM_BF16) illm_launch((group_norm_gate_row_kernel<bf16, IT>), grid, dim3(threads), 0, s, a, (bf16*)y);   \
         else illm_launch((group_norm_gate_row_kernel<float, IT>), grid, dim3(threads), 0, s, a, (float*)y);                        \
     } while (0)
-        if (pieces <= 1024) ILLM_GNR(1);
+        if (row_pieces(group) == 1) ILLM_GNR(1);
         else ILLM_GNR(2);
 #undef ILLM_GNR
         return illm_launch_status();

@@ -190,6 +190,117 @@ __global__ void __launch_bounds__(256) delta_prep_kernel(DeltaArgs p) {
     }
 }
 
+// The same for rows of whole 16-byte pieces and heads of 4, 8, .. 128 channels that fill warps evenly (a power of two): a warp takes 128 neighbouring
+// channels (one of d = 128, or several smaller heads) of TOK tokens in turn, four channels per lane.  Its rows are on
+// their way together and every row serves the taps of the tokens behind it from registers, so that the projection is
+// read once; the kernel above reads every row once per tap and channel by channel, and was bound by the instructions
+// that took (391 us for 7,868 tokens of 4,096 convolved and 2,048 decay channels, 390 MB).  The taps of a
+// channel are added in the same order; a head's sum of squares is added within its d / 4 lanes.
+// grid (T / TOK, groups of 128 channels / 8), 8 warps: the groups of q, k, v, the decay channels, then one for the numbers per head.
+struct DeltaPrepGroups { int q, v, g; };
+template <int KT, int TOK>
+__global__ void __launch_bounds__(256) delta_prep_vec_kernel(DeltaArgs p, DeltaPrepGroups n) {
+    pdl_grid_sync();
+    const int lane = threadIdx.x & 31, t0 = blockIdx.x * TOK;
+    int grp = blockIdx.y * 8 + (threadIdx.x >> 5);
+    const int d = p.d, nq = p.nkv * d, nv = p.nh * p.dv, C = 2 * nq + nv;
+    const int tokens = min(TOK, p.T - t0);
+    if (grp < 2 * n.q + n.v) {
+        const bool is_q = grp < n.q, is_k = !is_q && grp < 2 * n.q;
+        const int c = 128 * (is_q ? grp : is_k ? grp - n.q : grp - 2 * n.q) + 4 * lane;
+        const bool live = c < (is_q || is_k ? nq : nv);
+        const int col = (is_q ? p.q_off : is_k ? p.k_off : p.v_off) + c, at = (is_q ? 0 : is_k ? nq : 2 * nq) + c;
+        const float* taps = (is_q ? p.conv_q : is_k ? p.conv_k : p.conv_v) + (size_t)c * KT;
+        float w[4][KT];
+        float4 x[TOK];
+#pragma unroll
+        for (int i = 0; i < TOK; i++) x[i] = live && i < tokens ? *reinterpret_cast<const float4*>(p.x + (size_t)(t0 + i) * p.ld + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+            for (int j = 0; j < KT; j++) w[k][j] = live ? __ldg(taps + k * KT + j) : 0.f;
+#pragma unroll
+        for (int i = 0; i < TOK; i++) {
+            if (i >= tokens) break;
+            const int t = t0 + i, seq = p.token_seq[t], pos = p.token_pos[t], i_step = t - p.cu_q[seq];
+            float y[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int j = KT - 1; j >= 0; j--) {
+                float4 in = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (j <= i_step) {
+                    if (j <= i) in = x[i >= j ? i - j : 0];
+                    else if (live) in = *reinterpret_cast<const float4*>(p.x + (size_t)(t - j) * p.ld + col);
+                } else if (live && pos - j >= 0) {
+                    const float* state = p.state + (size_t)p.slots[seq] * p.state_elems + (size_t)p.nh * d * p.dv;
+                    in = *reinterpret_cast<const float4*>(state + (size_t)(KT - 1 - (j - i_step)) * C + at);
+                }
+                if (pos - j < 0) continue;
+                y[0] = fmaf(w[0][KT - 1 - j], in.x, y[0]);
+                y[1] = fmaf(w[1][KT - 1 - j], in.y, y[1]);
+                y[2] = fmaf(w[2][KT - 1 - j], in.z, y[2]);
+                y[3] = fmaf(w[3][KT - 1 - j], in.w, y[3]);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) y[k] = silu_fast(y[k]);
+            if (is_q || is_k) {
+                float ss = fmaf(y[0], y[0], fmaf(y[1], y[1], fmaf(y[2], y[2], y[3] * y[3])));
+                for (int o = 1; o < d / 4; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                const float f = (1.0f / sqrtf(ss + 1e-6f)) * (is_q ? p.q_scale : 1.0f);
+#pragma unroll
+                for (int k = 0; k < 4; k++) y[k] *= f;
+            }
+            if (live) *reinterpret_cast<float4*>(p.qkv + (size_t)t * C + at) = make_float4(y[0], y[1], y[2], y[3]);
+        }
+        return;
+    }
+    grp -= 2 * n.q + n.v;
+    if (grp < n.g) {            // a decay per channel
+        const int c = 128 * grp + 4 * lane, ng = p.nh * d;
+        if (c >= ng) return;
+        const float rate = expf(p.a_log[c / d]);
+        const float4 dt = *reinterpret_cast<const float4*>(p.dt_bias + c);
+        float4 a[TOK];
+#pragma unroll
+        for (int i = 0; i < TOK; i++) a[i] = i < tokens ? *reinterpret_cast<const float4*>(p.a + (size_t)(t0 + i) * p.a_ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < TOK; i++) {
+            if (i >= tokens) break;
+            float z[4] = {a[i].x + dt.x, a[i].y + dt.y, a[i].z + dt.z, a[i].w + dt.w};
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const float sp = z[k] > 20.f ? z[k] : log1pf(expf(z[k]));
+                z[k] = expf(-rate * sp);
+            }
+            *reinterpret_cast<float4*>(p.g + (size_t)(t0 + i) * ng + c) = make_float4(z[0], z[1], z[2], z[3]);
+        }
+    } else if (grp == n.g) {    // the write strengths, and with head_decay the decays
+        for (int e = lane; e < tokens * p.nh; e += 32) {
+            const int t = t0 + e / p.nh, h = e % p.nh;
+            p.beta[(size_t)t * p.nh + h] = 1.0f / (1.0f + expf(-p.x[(size_t)t * p.ld + p.b_off + h]));
+            if (p.head_decay) {
+                const float z = p.a[(size_t)t * p.a_ld + h] + p.dt_bias[h];
+                const float sp = z > 20.f ? z : log1pf(expf(z));
+                p.g[(size_t)t * p.nh + h] = expf(-expf(p.a_log[h]) * sp);
+            }
+        }
+    }
+}
+
+template <int KT>
+static void delta_prep_vec_launch(const DeltaArgs& p, cudaStream_t s) {
+    const int q = (p.nkv * p.d + 127) / 128, v = (p.nh * p.dv + 127) / 128, g = p.head_decay ? 0 : (p.nh * p.d + 127) / 128;
+    const DeltaPrepGroups n{q, v, g};
+    const unsigned blocks = (unsigned)((2 * q + v + g + 1 + 7) / 8);
+    if (p.T >= 512) illm_launch((delta_prep_vec_kernel<KT, 8>), dim3((p.T + 7) / 8, blocks), dim3(256), 0, s, p, n);
+    else illm_launch((delta_prep_vec_kernel<KT, 1>), dim3(p.T, blocks), dim3(256), 0, s, p, n);
+}
+static bool delta_prep_vec_takes(const DeltaArgs& p) {
+    auto odd = [](const void* a) { return ((uintptr_t)a & 15) != 0; };
+    return p.d >= 4 && p.d <= 128 && (p.d & (p.d - 1)) == 0 && p.taps >= 2 && p.taps <= 4 && !((p.ld | p.q_off | p.k_off | p.v_off) & 3) && !((p.nh * p.dv) & 3) &&
+           !(p.state_elems & 3) && (p.head_decay || !(p.a_ld & 3)) && !odd(p.x) && !odd(p.state) && !odd(p.qkv) &&
+           (p.head_decay || (!odd(p.a) && !odd(p.dt_bias) && !odd(p.g)));
+}
+
 // The convolution's rows after the step: the raw projections of the sequence's last taps - 1 positions (zeros for
 // positions before its start).  A thread owns a channel and goes through the rows in ascending order, so that a
 // row kept from before the step is read before it is overwritten.
@@ -753,13 +864,19 @@ extern "C" int illm_delta_rule(const float* x, int T, int ld, int q_off, int k_o
     const int hpb = d > 256 ? 1 : 256 / ((d + 31) / 32 * 32);
     const long long units = (2LL * nkv + hpb - 1) / hpb + ((long long)nh * dv + 1023) / 1024 + ((long long)nh * (head_decay ? 1 : d) + 1023) / 1024 + 1;
     if (units > 65535) return ILLM_ERR_BAD_ARG;
-    p.prep_tokens = T >= 512 ? DL_PREP_TOKENS : 1;
-    const dim3 pgrid((T + p.prep_tokens - 1) / p.prep_tokens, (unsigned)units);
-    if (taps == 1) illm_launch(delta_prep_kernel<1>, pgrid, dim3(256), 0, s, p);
-    else if (taps == 2) illm_launch(delta_prep_kernel<2>, pgrid, dim3(256), 0, s, p);
-    else if (taps == 3) illm_launch(delta_prep_kernel<3>, pgrid, dim3(256), 0, s, p);
-    else if (taps == 4) illm_launch(delta_prep_kernel<4>, pgrid, dim3(256), 0, s, p);
-    else illm_launch(delta_prep_kernel<0>, pgrid, dim3(256), 0, s, p);
+    if (delta_prep_vec_takes(p)) {
+        if (taps == 2) delta_prep_vec_launch<2>(p, s);
+        else if (taps == 3) delta_prep_vec_launch<3>(p, s);
+        else delta_prep_vec_launch<4>(p, s);
+    } else {
+        p.prep_tokens = T >= 512 ? DL_PREP_TOKENS : 1;
+        const dim3 pgrid((T + p.prep_tokens - 1) / p.prep_tokens, (unsigned)units);
+        if (taps == 1) illm_launch(delta_prep_kernel<1>, pgrid, dim3(256), 0, s, p);
+        else if (taps == 2) illm_launch(delta_prep_kernel<2>, pgrid, dim3(256), 0, s, p);
+        else if (taps == 3) illm_launch(delta_prep_kernel<3>, pgrid, dim3(256), 0, s, p);
+        else if (taps == 4) illm_launch(delta_prep_kernel<4>, pgrid, dim3(256), 0, s, p);
+        else illm_launch(delta_prep_kernel<0>, pgrid, dim3(256), 0, s, p);
+    }
     if (taps > 1) illm_launch(conv_state_kernel, dim3((unsigned)((C + 127) / 128), B), dim3(128), 0, s, p);
     if (chunks && chunk_scan_takes(d)) {
         const float* base = qkv;

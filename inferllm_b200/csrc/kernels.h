@@ -91,6 +91,8 @@ int illm_moe_gemm_tc(const void* xs, const void* w, void* y, int P, int E, int N
 // stream_ops.cu
 int illm_gated_act(const void* gu, void* out, int act_dtype, int T, int I, int act, void* stream);
 int illm_take_columns(const float* x, int ld, int off, int n_cols, void* y, int act_dtype, int T, void* stream);
+int illm_add2_rmsnorm_slices(float* resid, const float* d1, int n1, long long stride1, const float* d2, int n2, long long stride2, const float* w, void* y, int act_dtype, int T, int H, float eps, void* stream);
+int illm_scaled_add_rmsnorm_slices(float* resid, const float* delta, int splits, long long split_stride, const float* ls, const float* w, void* y, int act_dtype, int T, int H, float eps, void* stream);
 int illm_add2_rmsnorm(float* resid, const float* d1, const float* d2, const float* w, void* y, int act_dtype, int T, int H, float eps, void* stream);
 int illm_join_rows(const float* a, const float* b, int H, void* y, int act_dtype, int T, void* stream);
 
@@ -176,6 +178,7 @@ int illm_gemm_bf16_tc_gated_ex(const void* X, const void* W, void* out, int M, i
 int illm_gemm_bf16_tc2_ex(const void* X, const void* W, void* out, int out_dtype, int epi, float act_limit, int M, int N, int K, int* err, void* stream);
 int illm_gated_act_ex(const void* gu, void* out, int act_dtype, int T, int I, int act, float limit, void* stream);
 int illm_soft_cap(float* x, long long n, float cap, void* stream);
+int illm_norm_sandwich_slices(float* x, const float* y, int splits, long long split_stride, const float* wb, const float* w, void* out, int out_dtype, const int* rows, int n_rows, int H, float eps, int write_x, int center, float post_scale, void* stream);
 int illm_norm_sandwich(float* x, const float* y, const float* wb, const float* w, void* out, int out_dtype, const int* rows, int n_rows, int H, float eps, int write_x, int center, float post_scale, void* stream);
 
 // outnorm.cu

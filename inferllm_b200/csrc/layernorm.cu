@@ -9,14 +9,7 @@
 // in one kernel, because the second norm reads the row the first one has just made.  One block per row, every statistic of the layer norm in two passes (mean, then the mean squared deviation), the RMS norm's
 // in one, with a fixed order of the sums, all float32.  `rows` (int32) gathers: only those rows are made, and x is then left as it is (the model's
 // last norm, for the rows whose logits are wanted).
-#include "common.cuh"
-
-__device__ __forceinline__ void ln_store4(float* o, float a, float b, float c, float d) { *reinterpret_cast<float4*>(o) = make_float4(a, b, c, d); }
-__device__ __forceinline__ void ln_store4(bf16* o, float a, float b, float c, float d) {
-    const unsigned lo = (unsigned)__bfloat16_as_ushort(__float2bfloat16_rn(a)) | ((unsigned)__bfloat16_as_ushort(__float2bfloat16_rn(b)) << 16);
-    const unsigned hi = (unsigned)__bfloat16_as_ushort(__float2bfloat16_rn(c)) | ((unsigned)__bfloat16_as_ushort(__float2bfloat16_rn(d)) << 16);
-    *reinterpret_cast<uint2*>(o) = make_uint2(lo, hi);
-}
+#include "row_ops.cuh"
 
 // Any width, the row in shared memory, a channel per thread at a time.
 template <typename TO, bool CENTER>
@@ -64,11 +57,13 @@ ln_sandwich_kernel(float* __restrict__ x, const float* __restrict__ y, const flo
 // Rows of whole 16-byte pieces up to 16,384 wide: IT pieces per thread in registers.  Both rows and both weights are on
 // their way before the first sum (the weights while the kernel before drains), so that a single token's block, which
 // is bound by latency alone, waits for memory once (a row of 4,096 took 6.3 us with the row going through shared
-// memory and the stream and the weights asked for behind the first sum).
+// memory and the stream and the weights asked for behind the first sum).  y may come as the unreduced K slices of its
+// product, which are added here.
 template <typename TO, int IT, bool CENTER>
 __global__ void __launch_bounds__(1024)
 ln_sandwich_vec_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ wb, const float* __restrict__ w,
-                       TO* __restrict__ out, const int* __restrict__ rows, int H, float eps, float post_scale, int write_x) {
+                       TO* __restrict__ out, const int* __restrict__ rows, int H, float eps, float post_scale, int write_x, int splits,
+                       long long split_stride) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __shared__ float scratch[32];
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -86,7 +81,7 @@ ln_sandwich_vec_kernel(float* __restrict__ x, const float* __restrict__ y, const
     for (int i = 0; i < IT; i++) {
         const int c = 4 * (threadIdx.x + i * (int)blockDim.x);
         v[i] = c < H ? *reinterpret_cast<const float4*>(xr + c) : zero;
-        yv[i] = y && c < H ? *reinterpret_cast<const float4*>(y + (size_t)r * H + c) : zero;
+        yv[i] = y && c < H ? row_sum_slices(y + (size_t)r * H + c, splits, split_stride) : zero;
     }
     // the mean (CENTER) and 1 / sqrt(the mean square of the deviation + eps) of a row; pieces beyond it count for nothing
     auto statistics = [&](const float4 (&a)[IT], float& mean) {
@@ -127,44 +122,51 @@ ln_sandwich_vec_kernel(float* __restrict__ x, const float* __restrict__ y, const
     for (int i = 0; i < IT; i++) {
         const int c = 4 * (threadIdx.x + i * (int)blockDim.x);
         if (c < H)
-            ln_store4(o + c, ((v[i].x - mean) * inv) * wv[i].x, ((v[i].y - mean) * inv) * wv[i].y, ((v[i].z - mean) * inv) * wv[i].z,
-                      ((v[i].w - mean) * inv) * wv[i].w);
+            row_store4(o + c, make_float4(((v[i].x - mean) * inv) * wv[i].x, ((v[i].y - mean) * inv) * wv[i].y, ((v[i].z - mean) * inv) * wv[i].z,
+                                          ((v[i].w - mean) * inv) * wv[i].w));
     }
 }
 
 template <typename TO, bool CENTER>
-static void ln_launch(float* x, const float* y, const float* wb, const float* w, TO* out, const int* rows, int n_rows, int H, float eps,
-                      float post_scale, int write_x, cudaStream_t s) {
+static int ln_launch(float* x, const float* y, const float* wb, const float* w, TO* out, const int* rows, int n_rows, int H, float eps,
+                     float post_scale, int write_x, int splits, long long split_stride, cudaStream_t s) {
     // which kernel runs and its threads follow from the width and the layout alone, so a row's sums have one order in every step
-    auto aligned = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
-    if (H % 4 == 0 && H <= 16384 && aligned(x) && aligned(y) && aligned(wb) && aligned(w) && aligned(out)) {
-        const int pieces = H / 4, threads = pieces < 1024 ? (pieces + 31) / 32 * 32 : 1024;
-        if (pieces <= 1024) illm_launch((ln_sandwich_vec_kernel<TO, 1, CENTER>), dim3(n_rows), dim3(threads), 0, s, x, y, wb, w, out, rows, H, eps, post_scale, write_x);
-        else if (pieces <= 2048) illm_launch((ln_sandwich_vec_kernel<TO, 2, CENTER>), dim3(n_rows), dim3(threads), 0, s, x, y, wb, w, out, rows, H, eps, post_scale, write_x);
-        else illm_launch((ln_sandwich_vec_kernel<TO, 4, CENTER>), dim3(n_rows), dim3(threads), 0, s, x, y, wb, w, out, rows, H, eps, post_scale, write_x);
-        return;
+    if (H % 4 == 0 && row_pieces(H) && split_stride % 4 == 0 && !row_odd(x) && !row_odd(y) && !row_odd(wb) && !row_odd(w) && !row_odd(out)) {
+        const dim3 grid(n_rows), block(row_threads(H));
+#define ILLM_LNV(IT) \
+    illm_launch((ln_sandwich_vec_kernel<TO, IT, CENTER>), grid, block, 0, s, x, y, wb, w, out, rows, H, eps, post_scale, write_x, splits, split_stride)
+        if (row_pieces(H) == 1) ILLM_LNV(1);
+        else if (row_pieces(H) == 2) ILLM_LNV(2);
+        else ILLM_LNV(4);
+#undef ILLM_LNV
+        return illm_launch_status();
     }
+    if (splits > 1) return ILLM_ERR_BAD_ARG;
     const size_t smem = (size_t)H * sizeof(float);
     if (smem > 48 * 1024) cudaFuncSetAttribute(ln_sandwich_kernel<TO, CENTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     illm_launch((ln_sandwich_kernel<TO, CENTER>), dim3(n_rows), dim3(256), smem, s, x, y, wb, w, out, rows, H, eps, post_scale, write_x);
+    return illm_launch_status();
 }
 
 // y, wb: nullptr for no addition; w, out: nullptr for the addition alone; rows: nullptr for rows 0 .. n_rows - 1;
 // center: layer norm (post_scale is then 1), else RMS norm
+// splits > 1: y is that many float32 slices, split_stride floats apart, to be added up (rows of whole 16-byte pieces up to 16,384)
+extern "C" int illm_norm_sandwich_slices(float* x, const float* y, int splits, long long split_stride, const float* wb, const float* w, void* out,
+                                         int out_dtype, const int* rows, int n_rows, int H, float eps, int write_x, int center, float post_scale,
+                                         void* stream) {
+    if (n_rows <= 0) return 0;
+    if (H <= 0 || !x || (y && !wb) || ((out != nullptr) != (w != nullptr)) || splits < 1) return ILLM_ERR_BAD_ARG;
+    if ((size_t)H * sizeof(float) > 200 * 1024 || (center && post_scale != 1.f)) return ILLM_ERR_BAD_ARG;
+    cudaStream_t s = (cudaStream_t)stream;
+    if (out_dtype == ILLM_BF16 && center) return ln_launch<bf16, true>(x, y, wb, w, (bf16*)out, rows, n_rows, H, eps, 1.f, write_x, splits, split_stride, s);
+    if (out_dtype == ILLM_BF16) return ln_launch<bf16, false>(x, y, wb, w, (bf16*)out, rows, n_rows, H, eps, post_scale, write_x, splits, split_stride, s);
+    if (out_dtype == ILLM_F32 && center) return ln_launch<float, true>(x, y, wb, w, (float*)out, rows, n_rows, H, eps, 1.f, write_x, splits, split_stride, s);
+    if (out_dtype == ILLM_F32) return ln_launch<float, false>(x, y, wb, w, (float*)out, rows, n_rows, H, eps, post_scale, write_x, splits, split_stride, s);
+    return ILLM_ERR_BAD_ARG;
+}
 extern "C" int illm_norm_sandwich(float* x, const float* y, const float* wb, const float* w, void* out, int out_dtype, const int* rows,
                                   int n_rows, int H, float eps, int write_x, int center, float post_scale, void* stream) {
-    if (n_rows <= 0) return 0;
-    if (H <= 0 || !x || (y && !wb) || ((out != nullptr) != (w != nullptr))) return ILLM_ERR_BAD_ARG;
-    const size_t smem = (size_t)H * sizeof(float);
-    if (smem > 200 * 1024) return ILLM_ERR_BAD_ARG;
-    cudaStream_t s = (cudaStream_t)stream;
-    if (center && post_scale != 1.f) return ILLM_ERR_BAD_ARG;
-    if (out_dtype == ILLM_BF16 && center) ln_launch<bf16, true>(x, y, wb, w, (bf16*)out, rows, n_rows, H, eps, 1.f, write_x, s);
-    else if (out_dtype == ILLM_BF16) ln_launch<bf16, false>(x, y, wb, w, (bf16*)out, rows, n_rows, H, eps, post_scale, write_x, s);
-    else if (out_dtype == ILLM_F32 && center) ln_launch<float, true>(x, y, wb, w, (float*)out, rows, n_rows, H, eps, 1.f, write_x, s);
-    else if (out_dtype == ILLM_F32) ln_launch<float, false>(x, y, wb, w, (float*)out, rows, n_rows, H, eps, post_scale, write_x, s);
-    else return ILLM_ERR_BAD_ARG;
-    return illm_launch_status();
+    return illm_norm_sandwich_slices(x, y, 1, 0, wb, w, out, out_dtype, rows, n_rows, H, eps, write_x, center, post_scale, stream);
 }
 
 extern "C" int illm_layernorm_sandwich(float* x, const float* y, const float* wb, const float* w, void* out, int out_dtype, const int* rows,

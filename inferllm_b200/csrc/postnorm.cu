@@ -9,7 +9,7 @@
 // The addend may also come as the unreduced K slices of a split matrix product (float32
 // [splits, rows, H]); they are added in ascending order, as the stand-alone reduction would.
 // One block per row and a fixed order of the sums, so a row's bits do not depend on the launch.
-#include "common.cuh"
+#include "row_ops.cuh"
 
 template <typename TD, typename TY>
 __global__ void __launch_bounds__(1024)
@@ -56,19 +56,6 @@ scale_add_rmsnorm_kernel(float* __restrict__ resid, const TD* __restrict__ delta
 // before drains, and the row's pieces of the stream, the addend and up to eight of its slices are on their way together: a
 // single token's block is bound by the latency of its loads (one row of 2,048 with eight slices took 7 us channel by
 // channel with the sum going out to the stream and back).
-__device__ __forceinline__ float4 pn_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 pn_load4(const bf16* p) {
-    const uint2 u = *reinterpret_cast<const uint2*>(p);
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
-    return make_float4(a.x, a.y, b.x, b.y);
-}
-__device__ __forceinline__ void pn_store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-__device__ __forceinline__ void pn_store4(bf16* p, float4 v) {
-    const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
-}
-__device__ __forceinline__ void pn_add(float4& a, const float4 b) { a.x += b.x, a.y += b.y, a.z += b.z, a.w += b.w; }
-
 template <typename TD, typename TY, int IT>
 __global__ void __launch_bounds__(1024)
 scale_add_rmsnorm_vec_kernel(float* __restrict__ resid, const TD* __restrict__ delta, const float* __restrict__ w, TY* __restrict__ y, int H,
@@ -79,7 +66,7 @@ scale_add_rmsnorm_vec_kernel(float* __restrict__ resid, const TD* __restrict__ d
 #pragma unroll
     for (int i = 0; i < IT; i++) {
         const int c = 4 * (threadIdx.x + i * (int)blockDim.x);
-        wv[i] = c < H ? pn_load4(w + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        wv[i] = c < H ? row_load4(w + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const size_t base = (size_t)blockIdx.x * H;
@@ -89,19 +76,10 @@ scale_add_rmsnorm_vec_kernel(float* __restrict__ resid, const TD* __restrict__ d
         const int c = 4 * (threadIdx.x + i * (int)blockDim.x);
         v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (c >= H) continue;
-        const float4 x = pn_load4(resid + base + c);
+        const float4 x = row_load4(resid + base + c);
         float4 add = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (delta) add = pn_load4(delta + base + c);
-        if (partials) {             // slices in ascending order, eight loads in flight
-            const float* ps = partials + base + c;
-            for (int z = 0; z < splits; z += 8) {
-                float4 t[8];
-#pragma unroll
-                for (int u = 0; u < 8; u++) t[u] = z + u < splits ? pn_load4(ps + (size_t)(z + u) * split_stride) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                for (int u = 0; u < 8; u++) pn_add(add, t[u]);
-            }
-        }
+        if (delta) add = row_load4(delta + base + c);
+        else if (partials) add = row_sum_slices(partials + base + c, splits, split_stride);
         v[i] = make_float4(fmaf(alpha, x.x, add.x), fmaf(alpha, x.y, add.y), fmaf(alpha, x.z, add.z), fmaf(alpha, x.w, add.w));
         ss = fmaf(v[i].x, v[i].x, ss), ss = fmaf(v[i].y, v[i].y, ss), ss = fmaf(v[i].z, v[i].z, ss), ss = fmaf(v[i].w, v[i].w, ss);
     }
@@ -112,8 +90,8 @@ scale_add_rmsnorm_vec_kernel(float* __restrict__ resid, const TD* __restrict__ d
         const int c = 4 * (threadIdx.x + i * (int)blockDim.x);
         if (c >= H) continue;
         const float4 r = make_float4((v[i].x * inv) * wv[i].x, (v[i].y * inv) * wv[i].y, (v[i].z * inv) * wv[i].z, (v[i].w * inv) * wv[i].w);
-        pn_store4(resid + base + c, r);
-        if (y) pn_store4(y + base + c, r);
+        row_store4(resid + base + c, r);
+        if (y) row_store4(y + base + c, r);
     }
 }
 
@@ -123,17 +101,16 @@ extern "C" int illm_scale_add_rmsnorm(float* resid, const void* delta, int delta
     if (n_rows <= 0) return 0;
     if (H <= 0 || !resid || !w) return ILLM_ERR_BAD_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    auto aligned = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
     // which kernel runs and its threads follow from the width and the layout alone, so a row's sums have the same order in every launch
-    if (H % 4 == 0 && H <= 16384 && split_stride % 4 == 0 && aligned(resid) && aligned(delta) && aligned(w) && aligned(y) && aligned(partials)) {
-        const int pieces = H / 4, vthreads = pieces < 1024 ? (pieces + 31) / 32 * 32 : 1024;
+    if (H % 4 == 0 && row_pieces(H) && split_stride % 4 == 0 && !row_odd(resid) && !row_odd(delta) && !row_odd(w) && !row_odd(y) && !row_odd(partials)) {
+        const int pieces = row_pieces(H), vthreads = row_threads(H);
 #define ILLM_PNV(TD, TY, IT)                                                                                                          \
     illm_launch(scale_add_rmsnorm_vec_kernel<TD, TY, IT>, dim3(n_rows), dim3(vthreads), 0, s, resid, (const TD*)delta, w, (TY*)y, H, alpha, eps, \
                 partials, splits, split_stride)
 #define ILLM_PNV_FOR(TD, TY)                            \
     do {                                                \
-        if (pieces <= 1024) ILLM_PNV(TD, TY, 1);        \
-        else if (pieces <= 2048) ILLM_PNV(TD, TY, 2);   \
+        if (pieces == 1) ILLM_PNV(TD, TY, 1);           \
+        else if (pieces == 2) ILLM_PNV(TD, TY, 2);      \
         else ILLM_PNV(TD, TY, 4);                       \
     } while (0)
         if (delta_dtype == ILLM_F32 && y_dtype == ILLM_F32) ILLM_PNV_FOR(float, float);

@@ -17,7 +17,7 @@
 // A layer that attends to another layer's keys and values passes k_off < 0: only q is made.  A layer whose keys are
 // also its values passes v_off < 0: k alone is stored.
 // Everything is float32 until the stores.  One block per token; the sums have a fixed order.
-#include "common.cuh"
+#include "row_ops.cuh"
 
 struct QkPrepArgs {
     const void* x;
@@ -149,19 +149,6 @@ __global__ void __launch_bounds__(256) qk_prep_kernel(QkPrepArgs a) {
 // took 13 to 17 us for one token of 32 + 2 x 8 heads of 128.  A head's norm is added within the d / 4 lanes that hold the head (d / 4 a power
 // of two up to 32).  Only the rotate-half layout, whose channels pair up across threads, goes through shared memory.
 // The block size follows from the sizes alone, so that a row's sums have one order in every step.
-template <typename TI> __device__ __forceinline__ float4 qk_load4(const TI* p);
-template <> __device__ __forceinline__ float4 qk_load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
-template <> __device__ __forceinline__ float4 qk_load4<bf16>(const bf16* p) {
-    const uint2 u = *reinterpret_cast<const uint2*>(p);
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
-    return make_float4(a.x, a.y, b.x, b.y);
-}
-__device__ __forceinline__ void qk_store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-__device__ __forceinline__ void qk_store4(bf16* p, float4 v) {
-    const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
-}
-
 template <typename TI, typename TA, int IT>
 __global__ void __launch_bounds__(1024) qk_prep_vec_kernel(const QkPrepArgs a) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -201,7 +188,7 @@ __global__ void __launch_bounds__(1024) qk_prep_vec_kernel(const QkPrepArgs a) {
         const int at = threadIdx.x + i * threads;
         const bool is_q = at < nq4, is_k = !is_q && at < nq4 + nk4, is_v = !is_q && !is_k && at < nq4 + nk4 + nv4;
         const int c = is_q ? at : is_k ? at - nq4 : at - nq4 - nk4, off = is_q ? a.q_off : is_k ? a.k_off : a.v_off;
-        v[i] = is_q || is_k || is_v ? qk_load4(x + off + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[i] = is_q || is_k || is_v ? row_load4(x + off + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
         first[i] = is_v && a.v_first ? *reinterpret_cast<const float4*>(a.v_first + (size_t)t * a.v_first_ld + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     float ssq = 0.f, ssk = 0.f;
@@ -261,28 +248,27 @@ __global__ void __launch_bounds__(1024) qk_prep_vec_kernel(const QkPrepArgs a) {
                     if (e + 3 < a.rot) v[i].w = rotated(head, e + 3, a.rot, 0, cs);
                 }
             }
-            if (at < nq4) qk_store4((TA*)a.q_out + (size_t)t * 4 * nq4 + 4 * c, v[i]);
-            else if (a.kc && page >= 0) qk_store4((TA*)a.kc + (((size_t)page * a.nkv + hd) * a.page_size + slot) * a.d + e, v[i]);
+            if (at < nq4) row_store4((TA*)a.q_out + (size_t)t * 4 * nq4 + 4 * c, v[i]);
+            else if (a.kc && page >= 0) row_store4((TA*)a.kc + (((size_t)page * a.nkv + hd) * a.page_size + slot) * a.d + e, v[i]);
         } else if (page >= 0) {
             const int c = at - nq4 - nk4, hd = c / (a.dv >> 2), e = (c - hd * (a.dv >> 2)) * 4;
             if (a.v_keep) *reinterpret_cast<float4*>(a.v_keep + (size_t)t * 4 * nv4 + 4 * c) = v[i];
             if (a.v_first)
                 v[i] = make_float4((1.0f - lambda) * v[i].x + lambda * first[i].x, (1.0f - lambda) * v[i].y + lambda * first[i].y,
                                    (1.0f - lambda) * v[i].z + lambda * first[i].z, (1.0f - lambda) * v[i].w + lambda * first[i].w);
-            qk_store4((TA*)a.vc + (((size_t)page * a.nkv + hd) * a.page_size + slot) * a.dv + e, v[i]);
+            row_store4((TA*)a.vc + (((size_t)page * a.nkv + hd) * a.page_size + slot) * a.dv + e, v[i]);
         }
     }
 }
 
 // Whether the rows are whole 16-byte pieces throughout, and the norm of a head lies within a warp.
 static bool qk_prep_vec_takes(const QkPrepArgs& a) {
-    auto odd = [](const void* p) { return ((uintptr_t)p & 15) != 0; };
     if ((a.d | a.dv | a.ld | a.q_off) & 3) return false;
     if (a.k_off >= 0 && (a.k_off & 3)) return false;
     if (a.v_off >= 0 && (a.v_off & 3)) return false;
     if (a.pairs && (a.rot & 3)) return false;
-    if (odd(a.x) || odd(a.q_out) || odd(a.kc) || odd(a.vc) || odd(a.bq) || odd(a.bk) || odd(a.bv) || odd(a.wq) || odd(a.wk) || odd(a.cos_sin) ||
-        odd(a.v_keep) || odd(a.v_first) || (a.v_first && (a.v_first_ld & 3)))
+    if (row_odd(a.x) || row_odd(a.q_out) || row_odd(a.kc) || row_odd(a.vc) || row_odd(a.bq) || row_odd(a.bk) || row_odd(a.bv) || row_odd(a.wq) || row_odd(a.wk) || row_odd(a.cos_sin) ||
+        row_odd(a.v_keep) || row_odd(a.v_first) || (a.v_first && (a.v_first_ld & 3)))
         return false;
     if (a.wk && !a.wq) return false;
     if (a.head_norm && (a.d / 4 > 32 || (a.d / 4 & (a.d / 4 - 1)))) return false;

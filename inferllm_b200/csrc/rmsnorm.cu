@@ -195,23 +195,41 @@ extern "C" int illm_add_rmsnorm_partials(float* resid, const float* partials, in
     return ILLM_ERR_BAD_ARG;
 }
 
-// resid[r] += delta[r] without a norm (flushes a pending addition of the residual stream).
-template <typename TA>
+// resid[r] += delta[r] without a norm (flushes a pending addition of the residual stream).  VEC: four neighbouring elements per
+// thread (7,868 rows of 2,048 in float32: 67 us one by one, 193 MB).
+template <typename TA, bool VEC>
 __global__ void residual_add_kernel(float* __restrict__ resid, const TA* __restrict__ delta, size_t n) {
     pdl_grid_sync();
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) resid[i] += to_f32(delta[i]);
+    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * (VEC ? 4 : 1);
+    if (i >= n) return;
+    if (VEC) {
+        float4 r = *reinterpret_cast<const float4*>(resid + i);
+        float d[4];
+        if (sizeof(TA) == 4) {
+            const float4 v = *reinterpret_cast<const float4*>(delta + i);
+            d[0] = v.x, d[1] = v.y, d[2] = v.z, d[3] = v.w;
+        } else {
+            const uint2 u = *reinterpret_cast<const uint2*>(delta + i);
+            const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+            d[0] = lo.x, d[1] = lo.y, d[2] = hi.x, d[3] = hi.y;
+        }
+        r.x += d[0], r.y += d[1], r.z += d[2], r.w += d[3];
+        *reinterpret_cast<float4*>(resid + i) = r;
+    } else {
+        resid[i] += to_f32(delta[i]);
+    }
 }
 
 extern "C" int illm_residual_add(float* resid, const void* delta, int act_dtype, long long n,
                                  void* stream) {
     if (n <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
-    unsigned blocks = (unsigned)((n + 255) / 256);
-    if (act_dtype == ILLM_BF16)
-        illm_launch(residual_add_kernel<bf16>, dim3(blocks), dim3(256), 0, s, resid, (const bf16*)delta, (size_t)n);
-    else if (act_dtype == ILLM_F32)
-        illm_launch(residual_add_kernel<float>, dim3(blocks), dim3(256), 0, s, resid, (const float*)delta, (size_t)n);
+    const bool vec = n % 4 == 0 && !((uintptr_t)resid & 15) && !((uintptr_t)delta & 15);
+    const unsigned blocks = (unsigned)(((vec ? n / 4 : n) + 255) / 256);
+    if (act_dtype == ILLM_BF16 && vec) illm_launch((residual_add_kernel<bf16, true>), dim3(blocks), dim3(256), 0, s, resid, (const bf16*)delta, (size_t)n);
+    else if (act_dtype == ILLM_BF16) illm_launch((residual_add_kernel<bf16, false>), dim3(blocks), dim3(256), 0, s, resid, (const bf16*)delta, (size_t)n);
+    else if (act_dtype == ILLM_F32 && vec) illm_launch((residual_add_kernel<float, true>), dim3(blocks), dim3(256), 0, s, resid, (const float*)delta, (size_t)n);
+    else if (act_dtype == ILLM_F32) illm_launch((residual_add_kernel<float, false>), dim3(blocks), dim3(256), 0, s, resid, (const float*)delta, (size_t)n);
     else
         return ILLM_ERR_BAD_ARG;
     return illm_launch_status();

@@ -141,20 +141,33 @@ Mat embedding_scaled(Device& dev, const StepView& ctx, const Mat& table, float s
     return out;
 }
 
-Mat norm_sandwich(Device& dev, const Mat& resid, const Mat* delta, const Mat* post_w, const Mat* w, float eps, DType out_dtype, const int* rows,
+// A float32 addend as the row kernels take it: its slices where the rows are whole 16-byte pieces, finished otherwise.
+static MatOrPartials row_addend(Device& dev, const MatOrPartials& d, const Mat& resid, const char* what) {
+    MatOrPartials r = d;
+    if (d.is_partials() && (resid.cols % 4 || resid.cols > 16384)) {
+        r.m = materialize(dev, d.part, DType::F32);
+        r.part = Partials();
+    }
+    if (!r.is_partials()) need(r.m, what, true, DType::F32);
+    if (r.rows() != resid.rows || r.cols() != resid.cols) throw KernelError(std::string(what) + " must have the stream's shape");
+    return r;
+}
+
+Mat norm_sandwich(Device& dev, const Mat& resid, const MatOrPartials* delta, const Mat* post_w, const Mat* w, float eps, DType out_dtype, const int* rows,
                   long long n_rows, bool center, float post_scale) {
     need(resid, "the residual stream", true, DType::F32);
     const long long H = resid.cols, n = rows ? n_rows : resid.rows;
+    MatOrPartials d;
     if (delta) {
-        need(*delta, "the sublayer's output", true, DType::F32);
-        if (!post_w || post_w->dtype != DType::F32 || post_w->rows * post_w->cols != H || delta->rows != resid.rows || delta->cols != H)
+        d = row_addend(dev, *delta, resid, "the sublayer's output");
+        if (!post_w || post_w->dtype != DType::F32 || post_w->rows * post_w->cols != H)
             throw KernelError("layernorm: the sublayer's output and its norm weight must be float32 of the stream's shape and width");
     }
     if (w && (w->dtype != DType::F32 || w->rows * w->cols != H)) throw KernelError("layernorm: the weight must be float32 of the stream's width");
     if (H > kMaxNormWidth) throw KernelError("layernorm: rows of " + std::to_string(H) + " elements are beyond the kernel");
     Mat y;
     if (w) y = new_mat(dev, n, H, out_dtype);
-    check_kernel(illm_norm_sandwich((float*)resid.p, delta ? (const float*)delta->p : nullptr, delta ? (const float*)post_w->p : nullptr,
+    check_kernel(illm_norm_sandwich_slices((float*)resid.p, delta ? d.first() : nullptr, delta ? d.slices() : 1, d.stride(), delta ? (const float*)post_w->p : nullptr,
                                          w ? (const float*)w->p : nullptr, w ? y.p : nullptr, w ? code_of(out_dtype, "layernorm") : 0, rows, (int)n,
                                          (int)H, eps, rows == nullptr ? 1 : 0, center ? 1 : 0, post_scale, dev.stream()),
                  "norm_sandwich");
@@ -224,7 +237,7 @@ Mat add_rmsnorm(Device& dev, const Mat& resid, const MatOrPartials* delta, const
 }
 
 void residual_add(Device& dev, const Mat& resid, const MatOrPartials& delta) {
-    Mat d = delta.is_partials() ? materialize(dev, delta.part, DType::BF16) : delta.m;
+    Mat d = delta.is_partials() ? materialize(dev, delta.part, delta.part.dtype) : delta.m;
     need(resid, "resid", true, DType::F32);
     need(d, "delta");
     if (d.rows != resid.rows || d.cols != resid.cols) throw KernelError("residual_add: shapes differ");
@@ -306,6 +319,7 @@ MatOrPartials gemm_bf16_tc(Device& dev, const Mat& x, const Mat& w, DType out_dt
         r.part.splits = splits;
         r.part.rows = M;
         r.part.cols = N;
+        r.part.dtype = out_dtype;
     }
     return r;
 }
@@ -902,32 +916,30 @@ int gate_act_from_name(const std::string& name) {
     return -1;
 }
 
-Mat add2_rmsnorm(Device& dev, const Mat& resid, const Mat& d1, const Mat* d2, const Mat& w, float eps, DType out_dtype) {
+Mat add2_rmsnorm(Device& dev, const Mat& resid, const MatOrPartials& d1, const MatOrPartials* d2, const Mat& w, float eps, DType out_dtype) {
     need(resid, "resid", true, DType::F32);
-    need(d1, "delta", true, DType::F32);
     need(w, "norm weight", true, DType::F32);
-    if (d2) need(*d2, "second delta", true, DType::F32);
-    if (d1.rows != resid.rows || d1.cols != resid.cols || (d2 && (d2->rows != resid.rows || d2->cols != resid.cols)) || w.rows * w.cols != resid.cols)
-        throw KernelError("add2_rmsnorm: the additions and the weight must have the stream's shape");
+    const MatOrPartials a = row_addend(dev, d1, resid, "delta"), b = d2 ? row_addend(dev, *d2, resid, "second delta") : MatOrPartials();
+    if (w.rows * w.cols != resid.cols) throw KernelError("add2_rmsnorm: the weight must have the stream's width");
     if (resid.cols > kMaxNormWidth) throw KernelError("add2_rmsnorm: width " + std::to_string(resid.cols) + " exceeds what one block's shared memory holds");
     Mat y = new_mat(dev, resid.rows, resid.cols, out_dtype);
-    check_kernel(illm_add2_rmsnorm((float*)resid.p, (const float*)d1.p, d2 ? (const float*)d2->p : nullptr, (const float*)w.p, y.p,
+    check_kernel(illm_add2_rmsnorm_slices((float*)resid.p, a.first(), a.slices(), a.stride(), d2 ? b.first() : nullptr, d2 ? b.slices() : 1, b.stride(), (const float*)w.p, y.p,
                                    code_of(out_dtype, "add2_rmsnorm"), (int)resid.rows, (int)resid.cols, eps, dev.stream()),
                  "add2_rmsnorm");
     return y;
 }
 
-Mat scaled_add_rmsnorm(Device& dev, const Mat& resid, const Mat& delta, const float* ls, const Mat* w, float eps, DType out_dtype) {
+Mat scaled_add_rmsnorm(Device& dev, const Mat& resid, const MatOrPartials& delta_in, const float* ls, const Mat* w, float eps, DType out_dtype) {
     need(resid, "resid", true, DType::F32);
-    need(delta, "delta", true, DType::F32);
+    const MatOrPartials delta = row_addend(dev, delta_in, resid, "delta");
     if (w) need(*w, "norm weight", true, DType::F32);
     if (!ls) throw KernelError("scaled_add_rmsnorm: no layer scale");
-    if (delta.rows != resid.rows || delta.cols != resid.cols || (w && w->rows * w->cols != resid.cols))
+    if (w && w->rows * w->cols != resid.cols)
         throw KernelError("scaled_add_rmsnorm: the addition and the weight must have the stream's shape");
     if (resid.cols > kMaxNormWidth) throw KernelError("scaled_add_rmsnorm: width " + std::to_string(resid.cols) + " exceeds what one block's shared memory holds");
     Mat y;
     if (w) y = new_mat(dev, resid.rows, resid.cols, out_dtype);
-    check_kernel(illm_scaled_add_rmsnorm((float*)resid.p, (const float*)delta.p, ls, w ? (const float*)w->p : nullptr, y.p,
+    check_kernel(illm_scaled_add_rmsnorm_slices((float*)resid.p, delta.first(), delta.slices(), delta.stride(), ls, w ? (const float*)w->p : nullptr, y.p,
                                          code_of(out_dtype, "scaled_add_rmsnorm"), (int)resid.rows, (int)resid.cols, eps, dev.stream()),
                  "scaled_add_rmsnorm");
     return y;
@@ -1052,6 +1064,7 @@ MatOrPartials group_linear(Device& dev, GemmBackend backend, const Mat& x, long 
             r.part.splits = splits;
             r.part.rows = M;
             r.part.cols = N;
+        r.part.dtype = DType::F32;
         }
         return r;
     }

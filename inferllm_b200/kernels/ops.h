@@ -36,6 +36,7 @@ struct Partials {
     float* ws = nullptr;
     int splits = 0;
     long long rows = 0, cols = 0;
+    DType dtype = DType::BF16;        // what the finished matrix would be
 };
 
 // Either a finished matrix or unreduced slices.
@@ -45,6 +46,11 @@ struct MatOrPartials {
     bool is_partials() const { return part.ws != nullptr; }
     long long rows() const { return is_partials() ? part.rows : m.rows; }
     long long cols() const { return is_partials() ? part.cols : m.cols; }
+    DType dtype() const { return is_partials() ? part.dtype : m.dtype; }
+    // as the kernels that take slices see it: the first slice, how many, and how far apart
+    const float* first() const { return is_partials() ? part.ws : (const float*)m.p; }
+    int slices() const { return is_partials() ? part.splits : 1; }
+    long long stride() const { return is_partials() ? part.rows * part.cols : 0; }
 };
 
 // What every part sees of a step, on the device: int32 arrays in one buffer.
@@ -127,7 +133,7 @@ Mat embedding_scaled(Device& dev, const StepView& ctx, const Mat& table, float s
 // n(delta) * post_w (delta, post_w nullptr: nothing is added; post_scale other than 1 for the RMS norm only), then
 // n(resid) * w in `out_dtype` (w nullptr: the addition alone, an empty matrix comes back).  rows
 // (int32, device) gathers: only those rows are made and resid is left as it is.
-Mat norm_sandwich(Device& dev, const Mat& resid, const Mat* delta_f32, const Mat* post_w_f32, const Mat* w_f32, float eps, DType out_dtype,
+Mat norm_sandwich(Device& dev, const Mat& resid, const MatOrPartials* delta_f32, const Mat* post_w_f32, const Mat* w_f32, float eps, DType out_dtype,
                   const int* rows, long long n_rows, bool center = true, float post_scale = 1.f);
 // y = act(conv(x) + bias) (+ x): a causal convolution over time per channel of columns [x_off, x_off + C) of the
 // float32 rows x, `taps` taps w [C, taps] (float32, the last the token's own), the rows before the step from the
@@ -340,11 +346,11 @@ Mat group_norm_gate(Device& dev, const Mat& o_f32, int group, const float* w, fl
 enum GateAct { kActSilu = 1, kActRelu = 2, kActGeluTanh = 3, kActSwishClamped = 4, kActReluSquared = 5 };
 int gate_act_from_name(const std::string& name);        // ConfigError-free: -1 for an unknown name
 // resid += d1 (+ d2), all float32 [T, H], and the RMS norm of the new rows times w (float32 [H]) in `out_dtype`: one kernel
-Mat add2_rmsnorm(Device& dev, const Mat& resid, const Mat& d1, const Mat* d2, const Mat& weight_f32, float eps, DType out_dtype);
+Mat add2_rmsnorm(Device& dev, const Mat& resid, const MatOrPartials& d1, const MatOrPartials* d2, const Mat& weight_f32, float eps, DType out_dtype);
 // resid += delta * ls, all float32 (ls float32 [H] on the device), and, with a weight,
 // the RMS norm of the new rows times w (float32 [H]) in `out_dtype`: a sublayer's output through a per-channel layer scale,
 // folded into the next norm.  Without a weight an empty matrix comes back.
-Mat scaled_add_rmsnorm(Device& dev, const Mat& resid, const Mat& delta_f32, const float* ls, const Mat* weight_f32, float eps,
+Mat scaled_add_rmsnorm(Device& dev, const Mat& resid, const MatOrPartials& delta_f32, const float* ls, const Mat* weight_f32, float eps,
                        DType out_dtype);
 // y[t, :] += bias (float32 [cols] on the device), in place
 void add_bias(Device& dev, const Mat& y, const float* bias);

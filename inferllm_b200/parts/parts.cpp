@@ -244,7 +244,8 @@ struct RMSNorm : Norm {
         return ops::scale_add_rmsnorm(*rt->dev, stream.x, d, weight.m, residual_scale, eps, rt->dtype);
     }
     void add_normed_pending(ResidualStream& stream) override {
-        Mat y = stream.pending.is_partials() ? ops::materialize(*rt->dev, stream.pending.part, DType::F32) : ops::cast(*rt->dev, stream.pending.m, DType::F32);
+        MatOrPartials y = stream.pending;
+        if (!y.is_partials()) y.m = ops::cast(*rt->dev, y.m, DType::F32);
         ops::norm_sandwich(*rt->dev, stream.x, &y, &weight.m, nullptr, eps, DType::F32, nullptr, 0, false, post_scale);
         stream.has_pending = false;
     }
@@ -260,13 +261,8 @@ struct RMSNorm : Norm {
     Mat forward(ResidualStream& stream, const int* rows, long long n_rows) override {
         // an addition that passes an RMS norm of its own on its way into the stream: both norms in one kernel
         if (RMSNorm* post = stream.has_pending && !stream.has_pending2 ? dynamic_cast<RMSNorm*>(stream.pending_post) : nullptr) {
-            if (stream.pending.is_partials() && rows != nullptr) {
-                stream.pending.m = ops::materialize(*rt->dev, stream.pending.part, DType::F32);
-                stream.pending.part = Partials();
-            }
-            if (!stream.pending.is_partials() && stream.pending.m.dtype == DType::F32 && post->eps == eps && post->weight.m.dtype == DType::F32 &&
-                weight.m.dtype == DType::F32) {
-                Mat y = ops::norm_sandwich(*rt->dev, stream.x, &stream.pending.m, &post->weight.m, &weight.m, eps, rt->dtype, rows, n_rows, false,
+            if (stream.pending.dtype() == DType::F32 && post->eps == eps && post->weight.m.dtype == DType::F32 && weight.m.dtype == DType::F32) {
+                Mat y = ops::norm_sandwich(*rt->dev, stream.x, &stream.pending, &post->weight.m, &weight.m, eps, rt->dtype, rows, n_rows, false,
                                            post->post_scale);
                 if (rows == nullptr) {
                     stream.has_pending = false;
@@ -278,21 +274,20 @@ struct RMSNorm : Norm {
         // an addition that passes a layer scale on its way into the stream: x + factors * pending and the norm in one kernel
         if (stream.has_pending && stream.pending_post) {
             const Mat* ls = stream.pending_post->channel_scale();
-            if (ls && rows == nullptr && !stream.has_pending2 && !stream.pending.is_partials() && stream.pending.m.dtype == DType::F32 &&
-                weight.m.dtype == DType::F32) {
-                Mat y = ops::scaled_add_rmsnorm(*rt->dev, stream.x, stream.pending.m, (const float*)ls->p, &weight.m, eps, rt->dtype);
+            if (ls && rows == nullptr && !stream.has_pending2 && stream.pending.dtype() == DType::F32 && weight.m.dtype == DType::F32) {
+                Mat y = ops::scaled_add_rmsnorm(*rt->dev, stream.x, stream.pending, (const float*)ls->p, &weight.m, eps, rt->dtype);
                 stream.has_pending = false;
                 stream.pending_post = nullptr;
                 return y;
             }
             stream.flush();
         }
-        // float32 additions (one or two finished matrices) fold into one kernel with the norm; what that kernel does not
+        // float32 additions (one or two, finished or as slices) fold into one kernel with the norm; what that kernel does not
         // take (a second addition otherwise, a float32 addition beside a 16-bit output, gathered rows) is added first
-        const bool f32_pending = stream.has_pending && !stream.pending.is_partials() && stream.pending.m.dtype == DType::F32;
+        const bool f32_pending = stream.has_pending && stream.pending.dtype() == DType::F32;
         if (f32_pending && rows == nullptr && weight.m.dtype == DType::F32 &&
-            (!stream.has_pending2 || (!stream.pending2.is_partials() && stream.pending2.m.dtype == DType::F32))) {
-            Mat y = ops::add2_rmsnorm(*rt->dev, stream.x, stream.pending.m, stream.has_pending2 ? &stream.pending2.m : nullptr, weight.m, eps, rt->dtype);
+            (!stream.has_pending2 || stream.pending2.dtype() == DType::F32)) {
+            Mat y = ops::add2_rmsnorm(*rt->dev, stream.x, stream.pending, stream.has_pending2 ? &stream.pending2 : nullptr, weight.m, eps, rt->dtype);
             stream.has_pending = stream.has_pending2 = false;
             return y;
         }
@@ -319,7 +314,8 @@ struct LayerScale : Norm {
     const Mat* channel_scale() const override { return &factors.m; }
     Mat forward(ResidualStream&, const int*, long long) override { throw EngineError("layer_scale: stands behind a sublayer, not in front of one"); }
     void add_normed_pending(ResidualStream& stream) override {
-        Mat y = stream.pending.is_partials() ? ops::materialize(*rt->dev, stream.pending.part, DType::F32) : ops::cast(*rt->dev, stream.pending.m, DType::F32);
+        MatOrPartials y = stream.pending;
+        if (!y.is_partials()) y.m = ops::cast(*rt->dev, y.m, DType::F32);
         ops::scaled_add_rmsnorm(*rt->dev, stream.x, y, (const float*)factors.m.p, nullptr, 0.f, DType::F32);
         stream.has_pending = false;
     }
@@ -1012,10 +1008,10 @@ struct PreNormBlock : Block {
 struct PreNormScaledBlock : Block {
     void forward(ResidualStream& stream, const StepContext& ctx, const CacheView& cache, bool writes) override {
         Mat h = norms.at("norm1")->forward(stream, nullptr, 0);
-        stream.add_normed(mixer->forward(h, ctx, cache, writes, false), norms.at("ls1"));
+        stream.add_normed(mixer->forward(h, ctx, cache, writes, true), norms.at("ls1"));
         if (!ffn) return;
         h = norms.at("norm2")->forward(stream, nullptr, 0);
-        stream.add_normed(ffn->forward(h, ctx, false), norms.at("ls2"));
+        stream.add_normed(ffn->forward(h, ctx, true), norms.at("ls2"));
     }
 };
 
@@ -1080,8 +1076,8 @@ struct OutNormBlock : Block {
 struct ParallelBlock : Block {
     void forward(ResidualStream& stream, const StepContext& ctx, const CacheView& cache, bool writes) override {
         Mat h = norms.at("norm1")->forward(stream, nullptr, 0);       // folds in what the layer before left pending
-        stream.add(mixer->forward(h, ctx, cache, writes, false));
-        if (ffn) stream.add_second(ffn->forward(h, ctx, false));
+        stream.add(mixer->forward(h, ctx, cache, writes, true));
+        if (ffn) stream.add_second(ffn->forward(h, ctx, true));
     }
 };
 

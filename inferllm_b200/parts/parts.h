@@ -160,15 +160,15 @@ struct ResidualStream {
         pending = delta;
         has_pending = true;
     }
-    // x + post(delta): delta a finished float32 matrix
+    // x + post(delta)
     void add_normed(const MatOrPartials& delta, Norm* post) {
         add(delta);
         pending_post = post;
     }
-    // A second addition behind a pending one, both finished matrices: x + pending + delta, added in that order by flush()
+    // A second addition behind a pending one: x + pending + delta, added in that order by flush()
     // or by a norm that folds both in.  Anything else is added like add().
     void add_second(const MatOrPartials& delta) {
-        if (has_pending && !has_pending2 && !pending.is_partials() && !delta.is_partials()) {
+        if (has_pending && !has_pending2) {
             pending2 = delta;
             has_pending2 = true;
         } else {

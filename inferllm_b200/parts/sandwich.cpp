@@ -38,8 +38,8 @@ struct LayerNorm : Norm {
         // a sublayer's output that still has to pass a layer norm of its own on its way into the stream is normed,
         // added and normed again here; anything else that is pending is added first
         LayerNorm* post = stream.has_pending && !stream.has_pending2 ? dynamic_cast<LayerNorm*>(stream.pending_post) : nullptr;
-        if (post && !stream.pending.is_partials() && stream.pending.m.dtype == DType::F32 && post->eps == eps) {
-            Mat y = ops::norm_sandwich(*rt->dev, stream.x, &stream.pending.m, &post->weight.m, &weight.m, eps, out_dtype(), rows, n_rows);
+        if (post && stream.pending.dtype() == DType::F32 && post->eps == eps) {
+            Mat y = ops::norm_sandwich(*rt->dev, stream.x, &stream.pending, &post->weight.m, &weight.m, eps, out_dtype(), rows, n_rows);
             if (rows == nullptr) {
                 stream.has_pending = false;
                 stream.pending_post = nullptr;
@@ -50,7 +50,8 @@ struct LayerNorm : Norm {
         return ops::norm_sandwich(*rt->dev, stream.x, nullptr, nullptr, &weight.m, eps, out_dtype(), rows, n_rows);
     }
     void add_normed_pending(ResidualStream& stream) override {
-        Mat y = stream.pending.is_partials() ? ops::materialize(*rt->dev, stream.pending.part, DType::F32) : ops::cast(*rt->dev, stream.pending.m, DType::F32);
+        MatOrPartials y = stream.pending;
+        if (!y.is_partials()) y.m = ops::cast(*rt->dev, y.m, DType::F32);
         ops::norm_sandwich(*rt->dev, stream.x, &y, &weight.m, nullptr, eps, DType::F32, nullptr, 0);
         stream.has_pending = false;
     }
@@ -59,10 +60,10 @@ struct LayerNorm : Norm {
 struct SandwichBlock : Block {
     void forward(ResidualStream& stream, const StepContext& ctx, const CacheView& cache, bool writes) override {
         Mat h = norms.at("norm1")->forward(stream, nullptr, 0);
-        stream.add_normed(mixer->forward(h, ctx, cache, writes, false), norms.at("norm1b"));
+        stream.add_normed(mixer->forward(h, ctx, cache, writes, true), norms.at("norm1b"));
         if (!ffn) return;
         h = norms.at("norm2")->forward(stream, nullptr, 0);
-        stream.add_normed(ffn->forward(h, ctx, false), norms.at("norm2b"));
+        stream.add_normed(ffn->forward(h, ctx, true), norms.at("norm2b"));
     }
 };
 

@@ -101,6 +101,21 @@ def test_delta_rule(head_decay, d, dv, nh, nkv, strong):
 
     chunked, (out, S, qkv, gg, beta) = run(True), run(False)
     share = nh // nkv
+    # what the preparation makes of the projection (fast exponentials in silu: 1e-5)
+    sig = lambda z: 1.0 / (1.0 + np.exp(-z))  # noqa: E731
+    raw = x[:, :C].double().numpy()
+    taps_all = np.concatenate([c.double().numpy() for c in conv])
+    y = raw * taps_all[:, 1]
+    y[1:] += raw[:-1] * taps_all[:, 0] * (pos.cpu().numpy()[1:, None] > 0)
+    y = y * sig(y)
+    for lo in range(0, 2 * nkv * d, d):
+        head = y[:, lo:lo + d]
+        y[:, lo:lo + d] = head / np.sqrt((head * head).sum(-1, keepdims=True) + 1e-6) * (d ** -0.5 if lo < nkv * d else 1.0)
+    assert np.abs(qkv - y).max() <= 3e-5 * max(1.0, np.abs(y).max())
+    z = a.double().numpy() + dt.double().numpy()
+    rate = np.exp(a_log.double().numpy())
+    want = np.exp(-(rate if head_decay else np.repeat(rate, d)) * np.logaddexp(0.0, z))
+    assert np.abs(gg - want).max() <= 2e-5 and np.abs(beta - sig(x[:, C:].double().numpy())).max() <= 1e-6
     for b in range(B):
         s = B - 1 - b
         refs = []

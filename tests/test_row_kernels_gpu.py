@@ -175,3 +175,41 @@ def test_differential_attention_on_tensor_memory(nh, nkv, window, lens):
         mine, theirs = (np.abs(x[cu[b]:cu[b + 1]] - ref) for x in (got, other))
         assert (mine <= 2.0 ** -7 * np.abs(ref) + 2.0 ** -9).all()
         assert np.linalg.norm(mine) <= 1.5 * np.linalg.norm(theirs) + 1e-6
+
+
+@pytest.mark.parametrize("H", [4, 516, 4096, 4100, 16384])
+@pytest.mark.parametrize("n1,n2", [(1, 1), (3, 1), (9, 2), (17, 0)])
+def test_addends_as_slices(H, n1, n2):
+    """What the norms make of one or two addends that come as K slices, against float64: add2_rmsnorm, scaled_add_rmsnorm and
+    norm_sandwich (whose first norm reads the sum)."""
+    g = torch.Generator().manual_seed(H + n1)
+    T, eps = 3, 1e-5
+    x, w, ls = torch.randn(T, H, generator=g), torch.randn(H, generator=g), torch.randn(H, generator=g)
+    a, b = torch.randn(n1, T, H, generator=g), torch.randn(max(1, n2), T, H, generator=g)
+    xs, s1, s2 = x.double().numpy(), a.double().numpy().sum(0), b.double().numpy().sum(0) if n2 else 0.0
+    dev = [t.cuda() for t in (a, b, w, ls)]
+    y = torch.empty(T, H, device="cuda")
+    tol = 4 * math.sqrt(H) + 40 + n1
+
+    def norm(v, weight):
+        return v / np.sqrt((v * v).mean(-1, keepdims=True) + eps) * weight.double().numpy()
+
+    big = 4.0 * (n1 + n2 + 2) * w.abs().double().numpy() + 1e-3
+    xd = x.cuda()
+    rc = entry("illm_add2_rmsnorm_slices", I_, P_, P_, I_, L_, P_, I_, L_, P_, P_, I_, I_, I_, F_, P_)(
+        p(xd), p(dev[0]), n1, T * H, p(dev[1]) if n2 else None, max(1, n2), T * H, p(dev[2]), p(y), 0, T, H, eps, stream())
+    assert rc == 0
+    close(xd, xs + s1 + s2, n1 + n2 + 4, np.abs(xs) + 4.0 * (n1 + n2))
+    close(y, norm(xs + s1 + s2, w), tol, big)
+    xd = x.cuda()
+    rc = entry("illm_scaled_add_rmsnorm_slices", I_, P_, P_, I_, L_, P_, P_, P_, I_, I_, I_, F_, P_)(
+        p(xd), p(dev[0]), n1, T * H, p(dev[3]), p(dev[2]), p(y), 0, T, H, eps, stream())
+    assert rc == 0
+    v = xs + s1 * ls.double().numpy()
+    close(y, norm(v, w), tol, big * (1 + ls.abs().double().numpy()) + np.abs(norm(v, w)))
+    xd = x.cuda()
+    rc = entry("illm_norm_sandwich_slices", I_, P_, P_, I_, L_, P_, P_, P_, I_, P_, I_, I_, F_, I_, I_, F_, P_)(
+        p(xd), p(dev[0]), n1, T * H, p(dev[3]), p(dev[2]), p(y), 0, None, T, H, eps, 1, 0, 0.5, stream())
+    assert rc == 0
+    v = xs + 0.5 * norm(s1, ls)
+    close(y, norm(v, w), tol, big * (1 + ls.abs().double().numpy()) + np.abs(norm(v, w)))
