@@ -156,6 +156,12 @@ struct RdExtras {
     int gate_stride;
     int gate_wide;
     float softcap, softcap_x;
+    // alias > 1: every KV head of the cache is walked by so many blocks side by side, each for its own share of the head's query
+    // heads (a group beyond the 16 rows of a block's products; the rows come from L2 from the second on).  0 counts as 1.
+    int alias;
+    // diff: differential attention.  A query row holds [q_1, q_2], a key row [k_1, k_2]; row 2 h + m of a block's products is map m
+    // of query head h, the other half of its channels zero, so that one walk over the keys serves both maps.  nh counts maps.
+    int diff;
 };
 
 // num / den of a head with the sink's term added (m and the sink in units of log2) and the gate applied
@@ -289,7 +295,7 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
                 }
                 const int key0 = (tile_lo + split + i * n_splits) * RD_BN;
                 const int page = bt[key0 / page_size];
-                const int row = (page * nkv + hk) * page_size + key0 % page_size;
+                const int row = (page * nkv + (!FUSE && ex.alias > 1 ? hk / ex.alias : hk)) * page_size + key0 % page_size;
                 const unsigned kdst = base + (unsigned)s * 2 * TILE_BYTES, vdst = kdst + TILE_BYTES;
                 mbar_expect_tx(full0 + 8 * s, 2 * TILE_BYTES);
 #pragma unroll
@@ -312,7 +318,11 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
             store8(Qs + rd_qswz<D>(r, c), f);
         } else {
             uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (r < G) v = *reinterpret_cast<const uint4*>(q + (size_t)t * q_stride + (size_t)(hk * G + r) * D + c * 8);
+            if (!FUSE && ex.diff) {
+                if (r < G && (c >= CH / 2) == ((r & 1) != 0)) v = *reinterpret_cast<const uint4*>(q + (size_t)t * q_stride + (size_t)(hk * (G / 2) + (r >> 1)) * D + c * 8);
+            } else if (r < G) {
+                v = *reinterpret_cast<const uint4*>(q + (size_t)t * q_stride + (size_t)(hk * G + r) * D + c * 8);
+            }
             *reinterpret_cast<uint4*>(Qs + rd_qswz<D>(r, c)) = v;
         }
     }
@@ -480,7 +490,7 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
             den += mrg[((size_t)w * 16 + r) * ROW + D + 1] * wgt;
         }
         const size_t head = (size_t)t * nh + hk * G + r;
-        if (n_splits == 1) {
+        if (n_splits == 1 && out) {
             out[head * D + c] = __float2bfloat16_rn(rd_finish(num, den, M, ex, t, hk * G + r, D, c));
         } else {
             const size_t oidx = head * n_splits + split;
@@ -564,17 +574,18 @@ static int rd_launch(const void* q, int q_stride, const void* kc, const void* vc
     RdExtras ex = {};
     if (extras) ex = *extras;
     if (rope && (wide || extras)) return ILLM_ERR_BAD_ARG;      // the fused form is the plain attention's
+    const int groups = nkv * (ex.alias > 1 ? ex.alias : 1);
     auto launch = [&](auto kern) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
-        illm_launch(kern, dim3(n_splits, nkv, T), dim3(rope ? RD_THREADS + 32 : RD_THREADS), smem, s, mk, mv, (const bf16*)q, q_stride,
+        illm_launch(kern, dim3(n_splits, groups, T), dim3(rope ? RD_THREADS + 32 : RD_THREADS), smem, s, mk, mv, (const bf16*)q, q_stride,
                     block_table, max_pages, token_pos, token_seq, part_acc, part_ml, (bf16*)out, n_splits, nh, nkv,
-                    nh / nkv, page_size, window, scale * 1.4426950408889634f, err, rp, ex);
+                    nh / groups, page_size, window, scale * 1.4426950408889634f, err, rp, ex);
         return illm_launch_status();
     };
     rc = rope ? launch(attention_decode_ring_kernel<D, true, false>)
               : wide ? launch(attention_decode_ring_kernel<D, false, true>) : launch(attention_decode_ring_kernel<D, false, false>);
-    if (rc != 0 || n_splits == 1) return rc;
+    if (rc != 0 || n_splits == 1 || !out) return rc;        // no out: the shares are the caller's to put together
     illm_launch(attention_decode_ring_merge_kernel<D>, dim3(nh, T), dim3(D), 0, s, (const float*)part_acc,
                 (const float*)part_ml, (bf16*)out, n_splits, nh, ex);
     return illm_launch_status();
@@ -585,9 +596,10 @@ static int rd_run(const void* q, int q_stride, const void* kc, const void* vc, l
                   float* part_ml, void* out, int T, int nh, int nkv, int d, int page_size, int window, float scale,
                   int n_splits, int* err, void* stream, const RdRope* rope, const RdExtras* extras = nullptr, bool wide = false) {
     if (T <= 0) return 0;
-    if (nkv <= 0 || nh % nkv || nh / nkv > 16 || T > 65535 || nkv > 65535 || (q_stride & 7) || page_size % RD_BN ||
+    const int alias = extras && extras->alias > 1 ? extras->alias : 1;
+    if (nkv <= 0 || nh % (nkv * alias) || nh / (nkv * alias) > 16 || T > 65535 || nkv * alias > 65535 || (q_stride & 7) || page_size % RD_BN ||
         n_splits < 1 || n_splits > RD_MAX_SPLITS || ((uintptr_t)kc & 15) || ((uintptr_t)vc & 15) ||
-        n_pages * nkv * page_size > 0x7fffffffLL || (n_splits > 1 && (part_acc == nullptr || part_ml == nullptr)))
+        n_pages * nkv * page_size > 0x7fffffffLL || ((n_splits > 1 || !out) && (part_acc == nullptr || part_ml == nullptr)))
         return ILLM_ERR_BAD_ARG;
     if (!(rope && rope->partials) && (q == nullptr || ((uintptr_t)q & 15))) return ILLM_ERR_BAD_ARG;
     cudaStream_t s = (cudaStream_t)stream;
@@ -612,6 +624,11 @@ extern "C" int illm_attention_decode_ring(const void* q, int q_stride, const voi
                   nh, nkv, d, page_size, window, scale, n_splits, err, stream, nullptr);
 }
 
+extern "C" int illm_attention_decode_ring_shared(const void* q, int q_stride, const void* kc, const void* vc, long long n_pages, const int* block_table,
+                                                 int max_pages, const int* token_pos, const int* token_seq, float* part_acc, float* part_ml, void* out, int T,
+                                                 int nh, int nkv, int d, int page_size, int window, float scale, int n_splits, int* err, int wide_p,
+                                                 const float* sinks, const float* gate, int gate_stride, int gate_wide, float softcap, int alias, void* stream);
+
 // The same with sinks, gates (either may be nullptr), a soft cap (0: none; needs wide_p) and, with wide_p, two-term softmax
 // weights; `window` is a span (first_visible): a window, or chunks if it is negative.
 extern "C" int illm_attention_decode_ring_ex(const void* q, int q_stride, const void* kc, const void* vc,
@@ -621,7 +638,17 @@ extern "C" int illm_attention_decode_ring_ex(const void* q, int q_stride, const 
                                              int window, float scale, int n_splits, int* err, int wide_p, const float* sinks,
                                              const float* gate, int gate_stride, int gate_wide, float softcap, void* stream) {
     if (softcap > 0.f && !wide_p) return ILLM_ERR_BAD_ARG;
-    RdExtras ex{sinks, gate, gate_stride, gate_wide, softcap, softcap > 0.f ? 2.0f * scale * 1.4426950408889634f / softcap : 0.f};
+    return illm_attention_decode_ring_shared(q, q_stride, kc, vc, n_pages, block_table, max_pages, token_pos, token_seq, part_acc, part_ml, out, T, nh, nkv, d,
+                                             page_size, window, scale, n_splits, err, wide_p, sinks, gate, gate_stride, gate_wide, softcap, 1, stream);
+}
+
+// The same with a KV head's query heads over `alias` blocks (groups of more than 16 query heads).
+extern "C" int illm_attention_decode_ring_shared(const void* q, int q_stride, const void* kc, const void* vc, long long n_pages, const int* block_table,
+                                                 int max_pages, const int* token_pos, const int* token_seq, float* part_acc, float* part_ml, void* out, int T,
+                                                 int nh, int nkv, int d, int page_size, int window, float scale, int n_splits, int* err, int wide_p,
+                                                 const float* sinks, const float* gate, int gate_stride, int gate_wide, float softcap, int alias, void* stream) {
+    if (softcap > 0.f && !wide_p) return ILLM_ERR_BAD_ARG;
+    RdExtras ex{sinks, gate, gate_stride, gate_wide, softcap, softcap > 0.f ? 2.0f * scale * 1.4426950408889634f / softcap : 0.f, alias, 0};
     return rd_run(q, q_stride, kc, vc, n_pages, block_table, max_pages, token_pos, token_seq, part_acc, part_ml, out, T,
                   nh, nkv, d, page_size, window, scale, n_splits, err, stream, nullptr, &ex, wide_p != 0);
 }
@@ -647,4 +674,52 @@ extern "C" int illm_attention_decode_ring_rope(const void* qkv, const float* par
                  write_kv, step_err};
     return rd_run(qkv, (nh + 2 * nkv) * d, kc, vc, n_pages, block_table, max_pages, token_pos, token_seq, part_acc,
                   part_ml, out, T, nh, nkv, d, page_size, window, scale, n_splits, err, stream, &rp);
+}
+
+// The shares of both maps of a (token, head) put together in the order of the blocks, o = a_1 - lambda a_2, the head's unit norm and the
+// factor.  A block per (token, head), a thread per value channel.
+template <int D>
+__global__ void __launch_bounds__(D) attention_diff_ring_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, bf16* __restrict__ out,
+                                                                      int n_splits, int nh, float lambda, float eps, float out_scale) {
+    pdl_grid_sync();
+    __shared__ float scratch[32];
+    const int h = blockIdx.x, t = blockIdx.y, c = threadIdx.x;
+    float a[2];
+#pragma unroll
+    for (int m = 0; m < 2; m++) {
+        const size_t o = (((size_t)t * nh + h) * 2 + m) * n_splits;
+        float M = -INFINITY, num = 0.f, den = 0.f;
+        for (int s = 0; s < n_splits; s++) M = fmaxf(M, part_ml[(o + s) * 2]);
+        for (int s = 0; s < n_splits; s++) {
+            const float ms = part_ml[(o + s) * 2];
+            if (ms == -INFINITY) continue;          // a share without keys: its sums were not written
+            const float w = exp2f(ms - M);
+            den = fmaf(part_ml[(o + s) * 2 + 1], w, den);
+            num = fmaf(part_acc[(o + s) * D + c], w, num);
+        }
+        a[m] = num / den;
+    }
+    const float v = fmaf(-lambda, a[1], a[0]);
+    const float ss = block_sum(v * v, scratch);
+    out[((size_t)t * nh + h) * D + c] = __float2bfloat16_rn(v * (out_scale / sqrtf(ss / (float)D + eps)));
+}
+
+// Differential attention of single tokens: q [T, q_stride] with head h's [q_1, q_2] (2 x 64 channels) at column h * 128, pages of key
+// rows [k_1, k_2] and value rows of 128; scratch part_acc float [T, nh, 2, n_splits, 128], part_ml float [T, nh, 2, n_splits, 2].
+// (On CUDA cores, attention_maps.cu, one token of 32 heads over 1,800 keys took 19 us and its merge 6.3.)
+extern "C" int illm_attention_diff_ring_supported(int nh, int nkv, int d, int dv, int page_size) {
+    return d == 64 && dv == 128 && nkv > 0 && nh % nkv == 0 && nh / nkv <= 8 && page_size > 0 && page_size % RD_BN == 0;
+}
+extern "C" int illm_attention_diff_ring(const void* q, int q_stride, const void* kc, const void* vc, long long n_pages, const int* block_table, int max_pages,
+                                        const int* token_pos, const int* token_seq, float* part_acc, float* part_ml, void* out, int T, int nh, int nkv, int d, int dv,
+                                        int page_size, int window, float scale, int n_splits, float lambda, float eps, float out_scale, int* err, void* stream) {
+    if (T <= 0) return 0;
+    if (!illm_attention_diff_ring_supported(nh, nkv, d, dv, page_size) || !out) return ILLM_ERR_BAD_ARG;
+    RdExtras ex{nullptr, nullptr, 0, 0, 0.f, 0.f, 1, 1};
+    const int rc = rd_run(q, q_stride, kc, vc, n_pages, block_table, max_pages, token_pos, token_seq, part_acc, part_ml, nullptr, T, 2 * nh, nkv, 128, page_size,
+                          window, scale, n_splits, err, stream, nullptr, &ex, true);
+    if (rc) return rc;
+    illm_launch(attention_diff_ring_merge_kernel<128>, dim3(nh, T), dim3(128), 0, (cudaStream_t)stream, (const float*)part_acc, (const float*)part_ml, (bf16*)out,
+                n_splits, nh, lambda, eps, out_scale);
+    return illm_launch_status();
 }

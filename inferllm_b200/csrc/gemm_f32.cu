@@ -312,7 +312,7 @@ extern "C" int illm_gemm_f32_nt(const float* A, const float* W, float* C, int M,
     // A larger thread tile reads less shared memory per FMA, a smaller block leaves fewer SMs idle in the last round and fewer
     // rows beyond M: the tile with the least work on the busiest SM, per output 1 : 1.2 : 1.6 (512 rows of 7B size: Q/K/V and
     // gate/up 49 TF/s with 8 x 16 outputs a thread against 44 with 8 x 8).  Where an SM gets one block of the large tile, 256
-    // threads of 8 x 8 outputs hide more than 128 of 8 x 16 (output and down products 39 TF/s; 64 x 128 tiles 28).
+    // threads of 8 x 8 outputs hide more than 128 of 8 x 16 (output and down products 34 TF/s; 64 x 128 tiles 28).
     cudaStream_t s = (cudaStream_t)stream;
     const int sms = illm_sm_count();
     auto rounds = [&](long long bm, long long bn) { return (double)(((M + bm - 1) / bm * ((N + bn - 1) / bn) + sms - 1) / sms); };

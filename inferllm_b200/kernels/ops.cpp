@@ -685,6 +685,16 @@ Mat attention_decode_gqa(Device& dev, const Mat& qkv, const KVView& kv, const St
     return decode_chunked(dev, illm_attention_decode_gqa, "attention_decode_gqa", kGqaDecodeChunk, qkv, kv, ctx, g, scale, max_len);
 }
 
+// Blocks side by side that a KV head's query heads need in the ring kernel's 16 rows each (1: they fit one), 0 where the group does not
+// divide so.
+static int ring_alias(int nh, int nkv) {
+    if (nkv <= 0 || nh % nkv) return 0;
+    const int group = nh / nkv;
+    for (int a = 1; a <= 8; a++)
+        if (group % a == 0 && group / a <= 16) return a;
+    return 0;
+}
+
 Mat attention_decode_ring(Device& dev, const MatOrPartials& in, const KVView& kv, const StepView& ctx, Geometry g, float scale,
                           long long max_len, int splits, const FusedRope* rope, const AttentionExtras* extras) {
     if (rope && extras) throw KernelError("attention_decode_ring: sinks and gates do not go with the fused position encoding");
@@ -704,19 +714,21 @@ Mat attention_decode_ring(Device& dev, const MatOrPartials& in, const KVView& kv
     Mat out = new_mat_exact(dev, T, (long long)g.n_heads * g.head_dim, DType::BF16);
     for (long long t0 = 0; t0 < T; t0 += 65535) {
         const long long t1 = std::min(T, t0 + 65535);
-        const int n = splits > 0 ? splits : attention_decode_ring_splits(t1 - t0, g.n_kv_heads, max_len, g.head_dim, dev.n_sms(), dev.stream_bytes_per_us());
+        const int groups = g.n_kv_heads * (extras ? ring_alias(g.n_heads, g.n_kv_heads) : 1);
+        const int n = splits > 0 ? splits : attention_decode_ring_splits(t1 - t0, groups, max_len, g.head_dim, dev.n_sms(), dev.stream_bytes_per_us());
         float *part_acc = nullptr, *part_ml = nullptr;
         if (n > 1) {
             part_acc = dev.alloc_n<float>((size_t)(t1 - t0) * g.n_heads * n * g.head_dim);
             part_ml = dev.alloc_n<float>((size_t)(t1 - t0) * g.n_heads * n * 2);
         }
         if (extras) {
-            check_kernel(illm_attention_decode_ring_ex(row_ptr(in.m, t0), (int)width, kv.k, kv.v, kv.num_pages, kv.block_table, kv.width,
-                                                       ctx.token_pos + t0, ctx.token_seq + t0, part_acc, part_ml, row_ptr(out, t0), (int)(t1 - t0),
-                                                       g.n_heads, g.n_kv_heads, g.head_dim, kv.page_size, kv.span(), scale, n, dev.tc_error_word(),
-                                                       extras->wide_weights ? 1 : 0, extras->sinks,
-                                                       extras->gate ? extras->gate + (size_t)t0 * extras->gate_stride : nullptr, extras->gate_stride,
-                                                       extras->wide_gate ? 1 : 0, extras->softcap, dev.stream()),
+            const int alias = ring_alias(g.n_heads, g.n_kv_heads);
+            check_kernel(illm_attention_decode_ring_shared(row_ptr(in.m, t0), (int)width, kv.k, kv.v, kv.num_pages, kv.block_table, kv.width,
+                                                           ctx.token_pos + t0, ctx.token_seq + t0, part_acc, part_ml, row_ptr(out, t0), (int)(t1 - t0),
+                                                           g.n_heads, g.n_kv_heads, g.head_dim, kv.page_size, kv.span(), scale, n, dev.tc_error_word(),
+                                                           extras->wide_weights || alias > 1 ? 1 : 0, extras->sinks,
+                                                           extras->gate ? extras->gate + (size_t)t0 * extras->gate_stride : nullptr, extras->gate_stride,
+                                                           extras->wide_gate ? 1 : 0, extras->softcap, alias, dev.stream()),
                          "attention_decode_ring");
             continue;
         }
@@ -817,7 +829,10 @@ Mat attention_one(Device& dev, const Mat& q, const KVView& kv, const StepView& c
 Mat attention_ex(Device& dev, const Mat& q, const KVView& kv, const StepView& ctx, Geometry g, float scale, const AttentionExtras& ex) {
     const int dv = kv.v_head_dim > 0 ? kv.v_head_dim : g.head_dim;
     if (q.dtype == DType::BF16 && dv == g.head_dim) {
-        if (ctx.is_decode && attention_decode_ring_supported(q.dtype, g.n_heads, g.n_kv_heads, g.head_dim, kv.page_size)) {
+        // (A group beyond the ring's 16 rows walked the keys on CUDA cores in float32, attention_maps.cu; its blocks' weights are two
+        // bfloat16 terms.)
+        const int alias = ring_alias(g.n_heads, g.n_kv_heads);
+        if (ctx.is_decode && alias && attention_decode_ring_supported(q.dtype, g.n_heads / alias, g.n_kv_heads, g.head_dim, kv.page_size)) {
             MatOrPartials in;
             in.m = q;
             // the blocks are dealt the keys of the longest range a token can see
@@ -861,6 +876,17 @@ Mat attention_diff(Device& dev, const Mat& q, const KVView& kv, const StepView& 
     }
     // grids and scratch of a single-token step are sized for the longest sequence the cache allows, so that the launch is
     // the same at every step
+    if (q.dtype == DType::BF16 && ctx.is_decode && q.rows <= 65535 && q.cols % 8 == 0 &&
+        illm_attention_diff_ring_supported(g.n_heads, g.n_kv_heads, g.head_dim, dv, kv.page_size)) {
+        const int n = attention_decode_ring_splits(q.rows, g.n_kv_heads, ctx.max_seq_len, dv, dev.n_sms(), dev.stream_bytes_per_us());
+        float* part_acc = dev.alloc_n<float>((size_t)q.rows * g.n_heads * 2 * n * dv);
+        float* part_ml = dev.alloc_n<float>((size_t)q.rows * g.n_heads * 2 * n * 2);
+        check_kernel(illm_attention_diff_ring(q.p, (int)q.cols, kv.k, kv.v, kv.num_pages, kv.block_table, kv.width, ctx.token_pos, ctx.token_seq, part_acc, part_ml, out.p,
+                                              (int)q.rows, g.n_heads, g.n_kv_heads, g.head_dim, dv, kv.page_size, kv.window, scale, n, p.lambda, p.eps, p.out_scale,
+                                              dev.tc_error_word(), dev.stream()),
+                     "attention_diff_ring");
+        return out;
+    }
     if (q.dtype == DType::BF16 && ctx.is_decode && illm_attention_diff_decode_supported(g.n_heads, g.n_kv_heads, g.head_dim, dv)) {
         const int group = g.n_heads / g.n_kv_heads, hb = group >= 8 ? 8 : group > 2 ? 4 : group;
         const int splits = attention_diff_splits(q.rows, g.n_kv_heads * (int)ceil_div(group, hb), ctx.max_seq_len, dev.n_sms());

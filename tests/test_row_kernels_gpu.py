@@ -213,3 +213,102 @@ def test_addends_as_slices(H, n1, n2):
     assert rc == 0
     v = xs + 0.5 * norm(s1, ls)
     close(y, norm(v, w), tol, big * (1 + ls.abs().double().numpy()) + np.abs(norm(v, w)))
+
+
+def paged(lens, nkv, widths, g, page=64):
+    """Keys and values of sequences in pages dealt out at random, rows that nothing wrote full of NaN: the rows, the pools and the table."""
+    width = max(-(-n // page) for n in lens) + 1
+    table = torch.randperm(len(lens) * width, generator=g).to(torch.int32).view(len(lens), width)
+    rows = [[torch.randn(n, nkv, w, generator=g).bfloat16() for n in lens] for w in widths]
+    pools = [torch.full((len(lens) * width, nkv, page, w), float("nan"), dtype=torch.bfloat16) for w in widths]
+    for pool, of in zip(pools, rows):
+        for b, n in enumerate(lens):
+            for t in range(n):
+                pool[table[b, t // page], :, t % page] = of[b][t]
+    return rows, pools, table
+
+
+def weights_of(q, k, scale, window, cap=0.0, sink=None):
+    """Float64 softmax weights of the last token's heads [heads, d] over keys [n, d]."""
+    s = q @ k.T * scale
+    s = np.tanh(s / cap) * cap if cap else s
+    if window:
+        s[:, :max(0, k.shape[0] - window)] = -np.inf
+    top = s.max(-1, keepdims=True) if sink is None else np.maximum(s.max(-1, keepdims=True), sink[:, None])
+    e = np.exp(s - top)
+    return e / (e.sum(-1, keepdims=True) + (0.0 if sink is None else np.exp(sink[:, None] - top)))
+
+
+@pytest.mark.parametrize("nh,nkv,window,lens", [(8, 1, 0, [1, 64, 65, 700]), (32, 4, 0, [1821]), (3, 3, 70, [200, 5]), (2, 1, 1, [70])])
+@pytest.mark.parametrize("splits", [1, 3, 16])
+def test_differential_attention_of_single_tokens(nh, nkv, window, lens, splits):
+    """Beside the kernel on CUDA cores, both against float64: as near to it as that one (both round their output to bfloat16)."""
+    d, dv, page, T = 64, 128, 64, len(lens)
+    g = torch.Generator().manual_seed(nh + window + splits)
+    (ks, vs), pools, table = paged(lens, nkv, (2 * d, dv), g)
+    q = torch.randn(T, nh * 2 * d, generator=g).bfloat16()
+    width, n_pages = table.shape[1], pools[0].shape[0]
+    dev = [t.cuda() for t in (q, *pools, table, torch.tensor(lens, dtype=torch.int32) - 1, torch.arange(T, dtype=torch.int32))]
+    scale, lam, eps, factor = d ** -0.5, 0.45, 1e-6, 0.6
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    outs = [torch.full((T, nh * dv), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    acc, ml = torch.empty(T * nh * 2 * splits * dv, device="cuda"), torch.empty(T * nh * 2 * splits * 2, device="cuda")
+    rc = entry("illm_attention_diff_ring", I_, P_, I_, P_, P_, L_, P_, I_, P_, P_, P_, P_, P_, I_, I_, I_, I_, I_, I_, I_, F_, I_, F_, F_, F_, P_, P_)(
+        p(dev[0]), nh * 2 * d, p(dev[1]), p(dev[2]), n_pages, p(dev[3]), width, p(dev[4]), p(dev[5]), p(acc), p(ml), p(outs[0]), T, nh, nkv, d, dv, page, window,
+        scale, splits, lam, eps, factor, p(err), stream())
+    assert rc == 0
+    scratch = torch.empty(T * nh * 2 * 64 * (dv + 2), device="cuda")
+    rc = entry("illm_attention_diff_decode", I_, P_, I_, P_, P_, P_, I_, P_, P_, P_, I_, I_, I_, I_, I_, I_, I_, F_, F_, F_, F_, L_, I_, P_, P_)(
+        p(dev[0]), nh * 2 * d, p(dev[1]), p(dev[2]), p(dev[3]), width, p(dev[4]), p(dev[5]), p(outs[1]), T, nh, nkv, d, dv, page, window, scale, lam, eps, factor,
+        max(lens), 4, p(scratch), stream())
+    assert rc == 0 and int(err) == 0
+    ref = np.zeros((T, nh, dv))
+    for b in range(T):
+        kv = np.arange(nh) // (nh // nkv)
+        qq, k, v = q[b].double().numpy().reshape(nh, 2, d), ks[b].double().numpy().reshape(-1, nkv, 2, d), vs[b].double().numpy()
+        for h in range(nh):
+            a = [weights_of(qq[h:h + 1, m], k[:, kv[h], m], scale, window) @ v[:, kv[h]] for m in range(2)]
+            o = (a[0] - lam * a[1])[0]
+            ref[b, h] = o / np.sqrt((o * o).mean() + eps) * factor
+    mine, theirs = (np.abs(o.cpu().double().numpy().reshape(T, nh, dv) - ref) for o in outs)
+    # the output's rounding, and 2^-16 of the values' size for the weights' two terms, the products and the powers of two
+    assert (mine <= 2.0 ** -8 * np.abs(ref) + 2.0 ** -12).all()
+    print("errors", np.linalg.norm(mine) / np.linalg.norm(ref), np.linalg.norm(theirs) / np.linalg.norm(ref))
+    assert np.linalg.norm(mine) <= 1.01 * np.linalg.norm(theirs) + 1e-6
+
+
+@pytest.mark.parametrize("nh,nkv,alias,d", [(32, 1, 2, 128), (20, 1, 2, 64), (96, 2, 3, 64), (128, 1, 8, 128), (6, 2, 3, 128), (4, 4, 1, 64)])
+@pytest.mark.parametrize("window,cap,sinks", [(0, 0.0, False), (70, 20.0, True)])
+@pytest.mark.parametrize("splits", [1, 5])
+def test_single_tokens_with_a_group_over_several_blocks(nh, nkv, alias, d, window, cap, sinks, splits):
+    """Against float64, and beside the kernel on CUDA cores."""
+    lens, page = [1, 64, 300], 64
+    T, scale = len(lens), d ** -0.5
+    g = torch.Generator().manual_seed(nh + window)
+    (ks, vs), pools, table = paged(lens, nkv, (d, d), g)
+    q, sink = torch.randn(T, nh * d, generator=g).bfloat16(), torch.randn(nh, generator=g)
+    dev = [t.cuda() for t in (q, *pools, table, torch.tensor(lens, dtype=torch.int32) - 1, torch.arange(T, dtype=torch.int32), sink)]
+    width, n_pages = table.shape[1], pools[0].shape[0]
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    outs = [torch.full((T, nh * d), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    acc, ml = torch.empty(T * nh * splits * d, device="cuda"), torch.empty(T * nh * splits * 2, device="cuda")
+    sp = p(dev[6]) if sinks else None
+    rc = entry("illm_attention_decode_ring_shared", I_, P_, I_, P_, P_, L_, P_, I_, P_, P_, P_, P_, P_, I_, I_, I_, I_, I_, I_, F_, I_, P_, I_, P_, P_, I_, I_, F_, I_, P_)(
+        p(dev[0]), nh * d, p(dev[1]), p(dev[2]), n_pages, p(dev[3]), width, p(dev[4]), p(dev[5]), p(acc), p(ml), p(outs[0]), T, nh, nkv, d, page, window, scale, splits,
+        p(err), 1, sp, None, 0, 0, cap, alias, stream())
+    assert rc == 0
+    scratch = torch.empty(T * nh * 64 * (d + 2), device="cuda")
+    rc = entry("illm_attention_one_decode", I_, P_, I_, P_, P_, P_, I_, P_, P_, P_, I_, I_, I_, I_, I_, I_, I_, F_, F_, P_, P_, I_, I_, L_, I_, P_, P_)(
+        p(dev[0]), nh * d, p(dev[1]), p(dev[2]), p(dev[3]), width, p(dev[4]), p(dev[5]), p(outs[1]), T, nh, nkv, d, d, page, window, scale, cap, sp, None, 0, 0,
+        max(lens), 2, p(scratch), stream())
+    assert rc == 0 and int(err) == 0
+    ref = np.zeros((T, nh, d))
+    for b in range(T):
+        qq, k, v = q[b].double().numpy().reshape(nh, d), ks[b].double().numpy(), vs[b].double().numpy()
+        for hk in range(nkv):
+            of = slice(hk * nh // nkv, (hk + 1) * nh // nkv)
+            ref[b, of] = weights_of(qq[of], k[:, hk], scale, window, cap, sink.double().numpy()[of] if sinks else None) @ v[:, hk]
+    mine, theirs = (np.abs(o.cpu().double().numpy().reshape(T, nh, d) - ref) for o in outs)
+    assert (mine <= 2.0 ** -8 * np.abs(ref) + 2.0 ** -13).all()
+    print("errors", np.linalg.norm(mine) / np.linalg.norm(ref), np.linalg.norm(theirs) / np.linalg.norm(ref))
+    assert np.linalg.norm(mine) <= 1.01 * np.linalg.norm(theirs) + 1e-6
