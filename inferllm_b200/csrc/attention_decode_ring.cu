@@ -184,6 +184,7 @@ __device__ __forceinline__ float rd_finish(float num, float den, float m, const 
 template <int D, bool FUSE, bool WIDE>
 __global__ void __launch_bounds__(RD_THREADS + 32)
 attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
+                             const __grid_constant__ CUtensorMap map_k16, const __grid_constant__ CUtensorMap map_v16,
                              const bf16* __restrict__ q, int q_stride, const int* __restrict__ block_table,
                              int max_pages, const int* __restrict__ token_pos, const int* __restrict__ token_seq,
                              float* __restrict__ part_acc, float* __restrict__ part_ml, bf16* __restrict__ out,
@@ -204,6 +205,9 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
     const unsigned row_ready = tc_smem_u32(&bars[2 * STAGES]);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int split = blockIdx.x, hk = blockIdx.y, t = blockIdx.z;
+    int p = 0, seq = 0;
+    if (FUSE) p = token_pos[t], seq = token_seq[t];           // on their way while the barriers are made
     if (tid == 0) {
         for (int s = 0; s < STAGES; s++) {
             mbar_init(full0 + 8 * s, 1);
@@ -220,10 +224,10 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
     // on their way while that kernel drains.  Everything that reads the projection or writes global
     // memory waits.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (!FUSE) asm volatile("griddepcontrol.wait;" ::: "memory");
-
-    const int split = blockIdx.x, hk = blockIdx.y, t = blockIdx.z;
-    const int p = token_pos[t];
+    if (!FUSE) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        p = token_pos[t], seq = token_seq[t];
+    }
     const int lo = first_visible(p, span);
     const int tile_lo = lo / RD_BN, tile_hi = p / RD_BN;
     const int n_tiles = tile_hi - tile_lo + 1;
@@ -269,7 +273,7 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
 #pragma unroll
                 for (int k = 0; k < 4; k++) h2[k] = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
                 *reinterpret_cast<uint4*>(new_row_s + (is_k ? 0 : D) + c * 8) = v;
-                const int page = block_table[(size_t)token_seq[t] * max_pages + p / page_size];
+                const int page = block_table[(size_t)seq * max_pages + p / page_size];
                 if (page < 0) {
                     atomicExch(rp.err, 2);
                 } else {
@@ -285,7 +289,7 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
     if (warp == RD_CONSUMERS) {
         // ---- producer
         if (lane == 0) {
-            const int* bt = block_table + (size_t)token_seq[t] * max_pages;
+            const int* bt = block_table + (size_t)seq * max_pages;
             bool alive = true;
             for (int i = 0; i < n_my && alive; i++) {
                 const int s = i % STAGES;
@@ -297,6 +301,21 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
                 const int page = bt[key0 / page_size];
                 const int row = (page * nkv + (!FUSE && ex.alias > 1 ? hk / ex.alias : hk)) * page_size + key0 % page_size;
                 const unsigned kdst = base + (unsigned)s * 2 * TILE_BYTES, vdst = kdst + TILE_BYTES;
+                // The last tile's keys in boxes of 16, one group per consumer warp that has a visible key: whole tiles read a tenth more
+                // at contexts of 64 to 430 keys.  (64 tokens of 32 heads there: 62 us a layer, 52 with this, the merge of the warps
+                // for the heads alone and the positions loaded ahead; 5.5 TB/s.  Rings of two stages, three blocks an SM: 61, and up
+                // to 8 % slower at 600 to 4,000 keys.)
+                const int groups = (p - key0) / 16 + 1;
+                if (groups < RD_BN / 16) {
+                    mbar_expect_tx(full0 + 8 * s, (unsigned)groups * (2 * TILE_BYTES / (RD_BN / 16)));
+#pragma unroll
+                    for (int hx = 0; hx < D / 64; hx++)
+                        for (int u = 0; u < groups; u++) {
+                            tma_load_2d(kdst + hx * (RD_BN * 128) + u * (16 * 128), &map_k16, hx * 64, row + u * 16, full0 + 8 * s);
+                            tma_load_2d(vdst + hx * (RD_BN * 128) + u * (16 * 128), &map_v16, hx * 64, row + u * 16, full0 + 8 * s);
+                        }
+                    continue;
+                }
                 mbar_expect_tx(full0 + 8 * s, 2 * TILE_BYTES);
 #pragma unroll
                 for (int hx = 0; hx < D / 64; hx++) {
@@ -464,12 +483,10 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
 #pragma unroll
     for (int e = 0; e < 2; e++) {
         const int r = g + e * 8;
+        if (r >= G) continue;
         float* dst = mrg + ((size_t)warp * 16 + r) * ROW;
 #pragma unroll
-        for (int i = 0; i < NT_D; i++) {
-            dst[i * 8 + t4 * 2] = o[i][e * 2];
-            dst[i * 8 + t4 * 2 + 1] = o[i][e * 2 + 1];
-        }
+        for (int i = 0; i < NT_D; i++) *reinterpret_cast<float2*>(dst + i * 8 + t4 * 2) = make_float2(o[i][e * 2], o[i][e * 2 + 1]);
         if (t4 == 0) {
             dst[D] = m_run[e];
             dst[D + 1] = l_run[e];
@@ -503,6 +520,39 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
     }
 }
 
+// The weight of a head's share s (lane s of every warp, at most 32 shares; 0 for a share without keys, whose sums were not written)
+// and, returned, the largest maximum.  All shares' words are one load, where a thread that goes through them waits for each round.
+__device__ __forceinline__ float rd_share_weights(const float* __restrict__ part_ml, size_t o, int n_splits, float& w, float& l) {
+    const int lane = threadIdx.x & 31;
+    float2 ml = make_float2(-INFINITY, 0.f);
+    if (lane < n_splits) ml = *reinterpret_cast<const float2*>(part_ml + (o + lane) * 2);
+    float M = ml.x;
+#pragma unroll
+    for (int k = 16; k; k >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, k));
+    w = ml.x == -INFINITY ? 0.f : fast_exp2(ml.x - M);
+    l = ml.y;
+    return M;
+}
+// sum of w acc and of w l over the shares, ascending, shares of weight 0 left out; eight rows' loads in flight
+template <int D>
+__device__ __forceinline__ void rd_add_shares(const float* __restrict__ acc, int n_splits, float w, float l, float& num, float& den) {
+    num = den = 0.f;
+    for (int s0 = 0; s0 < n_splits; s0 += 8) {
+        float v[8], ws[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            ws[k] = __shfl_sync(0xffffffffu, w, (s0 + k) & 31);
+            v[k] = s0 + k < n_splits && ws[k] != 0.f ? acc[(size_t)(s0 + k) * D] : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            den += __shfl_sync(0xffffffffu, l, (s0 + k) & 31) * (s0 + k < n_splits ? ws[k] : 0.f);
+            num += v[k] * ws[k];
+        }
+    }
+}
+
+// (One sequence of 32 heads: 2.4 -> 1.9 us; with the two maps of differential heads 5.8 -> 2.9.)
 // out[t, h, :] = sum over splits (ascending) of acc * 2^(m - M) / sum of l * 2^(m - M); splits
 // without keys carry m = -inf and are skipped.
 template <int D>
@@ -512,16 +562,9 @@ __global__ void attention_decode_ring_merge_kernel(const float* __restrict__ par
     pdl_grid_sync();
     const int h = blockIdx.x, t = blockIdx.y, c = threadIdx.x;
     const size_t o = ((size_t)t * nh + h) * n_splits;
-    float M = -INFINITY;
-    for (int s = 0; s < n_splits; s++) M = fmaxf(M, part_ml[(o + s) * 2]);
-    float num = 0.f, den = 0.f;
-    for (int s = 0; s < n_splits; s++) {
-        const float m = part_ml[(o + s) * 2];
-        if (m == -INFINITY) continue;
-        const float w = fast_exp2(m - M);
-        den += part_ml[(o + s) * 2 + 1] * w;
-        num += part_acc[(o + s) * D + c] * w;
-    }
+    float w, l, num, den;
+    const float M = rd_share_weights(part_ml, o, n_splits, w, l);
+    rd_add_shares<D>(part_acc + o * D + c, n_splits, w, l, num, den);
     out[((size_t)t * nh + h) * D + c] = __float2bfloat16_rn(rd_finish(num, den, M, ex, t, h, D, c));
 }
 
@@ -543,13 +586,13 @@ static RdEncodeTiledFn rd_encode_fn() {
     return fn;
 }
 
-// one cache entry seen as a bfloat16 matrix [rows = pages * kv heads * page_size, d]; boxes of [64, 64]
-static int rd_make_map(CUtensorMap* map, const void* ptr, long long rows, int d) {
+// one cache entry seen as a bfloat16 matrix [rows = pages * kv heads * page_size, d]; boxes of [box_rows, 64]
+static int rd_make_map(CUtensorMap* map, const void* ptr, long long rows, int d, int box_rows) {
     RdEncodeTiledFn fn = rd_encode_fn();
     if (!fn) return ILLM_ERR_BAD_ARG;
     cuuint64_t dims[2] = {(cuuint64_t)d, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)d * 2};
-    cuuint32_t box[2] = {64, RD_BN};
+    cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -562,11 +605,11 @@ static int rd_launch(const void* q, int q_stride, const void* kc, const void* vc
                      const int* block_table, int max_pages, const int* token_pos, const int* token_seq,
                      float* part_acc, float* part_ml, void* out, int T, int nh, int nkv, int page_size, int window,
                      float scale, int n_splits, int* err, cudaStream_t s, const RdRope* rope, const RdExtras* extras, bool wide) {
-    CUtensorMap mk, mv;
+    CUtensorMap mk, mv, mk16, mv16;
     int rc;
     const long long rows = n_pages * nkv * page_size;
-    if ((rc = rd_make_map(&mk, kc, rows, D)) != 0) return rc;
-    if ((rc = rd_make_map(&mv, vc, rows, D)) != 0) return rc;
+    if ((rc = rd_make_map(&mk, kc, rows, D, RD_BN)) != 0 || (rc = rd_make_map(&mv, vc, rows, D, RD_BN)) != 0) return rc;
+    if ((rc = rd_make_map(&mk16, kc, rows, D, 16)) != 0 || (rc = rd_make_map(&mv16, vc, rows, D, 16)) != 0) return rc;
     constexpr int STAGES = 384 / D;
     const size_t smem = (size_t)STAGES * 2 * RD_BN * D * 2 + (size_t)16 * D * 2 + 1024;
     RdRope rp = {};
@@ -578,7 +621,7 @@ static int rd_launch(const void* q, int q_stride, const void* kc, const void* vc
     auto launch = [&](auto kern) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
-        illm_launch(kern, dim3(n_splits, groups, T), dim3(rope ? RD_THREADS + 32 : RD_THREADS), smem, s, mk, mv, (const bf16*)q, q_stride,
+        illm_launch(kern, dim3(n_splits, groups, T), dim3(rope ? RD_THREADS + 32 : RD_THREADS), smem, s, mk, mv, mk16, mv16, (const bf16*)q, q_stride,
                     block_table, max_pages, token_pos, token_seq, part_acc, part_ml, (bf16*)out, n_splits, nh, nkv,
                     nh / groups, page_size, window, scale * 1.4426950408889634f, err, rp, ex);
         return illm_launch_status();
@@ -677,36 +720,27 @@ extern "C" int illm_attention_decode_ring_rope(const void* qkv, const float* par
 }
 
 // The shares of both maps of a (token, head) put together in the order of the blocks, o = a_1 - lambda a_2, the head's unit norm and the
-// factor.  A block per (token, head), a thread per value channel.
+// factor.  A block per (token, head), a thread per map and value channel.
 template <int D>
-__global__ void __launch_bounds__(D) attention_diff_ring_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, bf16* __restrict__ out,
-                                                                      int n_splits, int nh, float lambda, float eps, float out_scale) {
+__global__ void __launch_bounds__(2 * D) attention_diff_ring_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, bf16* __restrict__ out,
+                                                                          int n_splits, int nh, float lambda, float eps, float out_scale) {
     pdl_grid_sync();
-    __shared__ float scratch[32];
-    const int h = blockIdx.x, t = blockIdx.y, c = threadIdx.x;
-    float a[2];
-#pragma unroll
-    for (int m = 0; m < 2; m++) {
-        const size_t o = (((size_t)t * nh + h) * 2 + m) * n_splits;
-        float M = -INFINITY, num = 0.f, den = 0.f;
-        for (int s = 0; s < n_splits; s++) M = fmaxf(M, part_ml[(o + s) * 2]);
-        for (int s = 0; s < n_splits; s++) {
-            const float ms = part_ml[(o + s) * 2];
-            if (ms == -INFINITY) continue;          // a share without keys: its sums were not written
-            const float w = exp2f(ms - M);
-            den = fmaf(part_ml[(o + s) * 2 + 1], w, den);
-            num = fmaf(part_acc[(o + s) * D + c], w, num);
-        }
-        a[m] = num / den;
-    }
-    const float v = fmaf(-lambda, a[1], a[0]);
+    __shared__ float scratch[32], second[D];
+    const int h = blockIdx.x, t = blockIdx.y, m = threadIdx.x / D, c = threadIdx.x % D;
+    const size_t o = (((size_t)t * nh + h) * 2 + m) * n_splits;
+    float w, l, num, den;
+    rd_share_weights(part_ml, o, n_splits, w, l);
+    rd_add_shares<D>(part_acc + o * D + c, n_splits, w, l, num, den);
+    if (m == 1) second[c] = num / den;
+    __syncthreads();
+    const float v = m == 0 ? fmaf(-lambda, second[c], num / den) : 0.f;
     const float ss = block_sum(v * v, scratch);
-    out[((size_t)t * nh + h) * D + c] = __float2bfloat16_rn(v * (out_scale / sqrtf(ss / (float)D + eps)));
+    if (m == 0) out[((size_t)t * nh + h) * D + c] = __float2bfloat16_rn(v * (out_scale / sqrtf(ss / (float)D + eps)));
 }
 
 // Differential attention of single tokens: q [T, q_stride] with head h's [q_1, q_2] (2 x 64 channels) at column h * 128, pages of key
 // rows [k_1, k_2] and value rows of 128; scratch part_acc float [T, nh, 2, n_splits, 128], part_ml float [T, nh, 2, n_splits, 2].
-// (On CUDA cores, attention_maps.cu, one token of 32 heads over 1,800 keys took 19 us and its merge 6.3.)
+// (On CUDA cores, attention_maps.cu, one token of 32 heads over 1,800 keys took 19 us and its merge 6.3; here 6.9 and 2.9.)
 extern "C" int illm_attention_diff_ring_supported(int nh, int nkv, int d, int dv, int page_size) {
     return d == 64 && dv == 128 && nkv > 0 && nh % nkv == 0 && nh / nkv <= 8 && page_size > 0 && page_size % RD_BN == 0;
 }
@@ -719,7 +753,7 @@ extern "C" int illm_attention_diff_ring(const void* q, int q_stride, const void*
     const int rc = rd_run(q, q_stride, kc, vc, n_pages, block_table, max_pages, token_pos, token_seq, part_acc, part_ml, nullptr, T, 2 * nh, nkv, 128, page_size,
                           window, scale, n_splits, err, stream, nullptr, &ex, true);
     if (rc) return rc;
-    illm_launch(attention_diff_ring_merge_kernel<128>, dim3(nh, T), dim3(128), 0, (cudaStream_t)stream, (const float*)part_acc, (const float*)part_ml, (bf16*)out,
+    illm_launch(attention_diff_ring_merge_kernel<128>, dim3(nh, T), dim3(256), 0, (cudaStream_t)stream, (const float*)part_acc, (const float*)part_ml, (bf16*)out,
                 n_splits, nh, lambda, eps, out_scale);
     return illm_launch_status();
 }

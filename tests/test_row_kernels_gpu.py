@@ -312,3 +312,30 @@ def test_single_tokens_with_a_group_over_several_blocks(nh, nkv, alias, d, windo
     assert (mine <= 2.0 ** -8 * np.abs(ref) + 2.0 ** -13).all()
     print("errors", np.linalg.norm(mine) / np.linalg.norm(ref), np.linalg.norm(theirs) / np.linalg.norm(ref))
     assert np.linalg.norm(mine) <= 1.01 * np.linalg.norm(theirs) + 1e-6
+
+
+@pytest.mark.parametrize("nh,nkv,d", [(4, 4, 128), (6, 2, 64), (32, 2, 128)])
+@pytest.mark.parametrize("splits", [1, 2, 32])
+@pytest.mark.parametrize("window", [0, 40])
+def test_ring_attention_loads_no_more_than_the_last_tiles_keys(nh, nkv, d, splits, window):
+    """Contexts that end in each of a tile's four groups of 16 keys, against float64; every row that nothing wrote is NaN."""
+    g = torch.Generator().manual_seed(d + splits)
+    lens, page = [1, 15, 16, 17, 31, 33, 47, 48, 49, 63, 64, 65, 80, 97, 128, 129, 200, 2047], 64
+    T, scale = len(lens), d ** -0.5
+    (ks, vs), pools, table = paged(lens, nkv, (d, d), g)
+    q = torch.randn(T, nh * d, generator=g).bfloat16()
+    dev = [t.cuda() for t in (q, *pools, table, torch.tensor(lens, dtype=torch.int32) - 1, torch.arange(T, dtype=torch.int32))]
+    err, out = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.empty(T, nh * d, dtype=torch.bfloat16, device="cuda")
+    acc, ml = torch.full((T * nh * splits * d,), float("nan"), device="cuda"), torch.empty(T * nh * splits * 2, device="cuda")
+    ring = entry("illm_attention_decode_ring", I_, P_, I_, P_, P_, L_, P_, I_, P_, P_, P_, P_, P_, I_, I_, I_, I_, I_, I_, F_, I_, P_, P_)
+    assert ring(p(dev[0]), nh * d, p(dev[1]), p(dev[2]), pools[0].shape[0], p(dev[3]), table.shape[1], p(dev[4]), p(dev[5]), p(acc), p(ml), p(out), T, nh, nkv, d, page,
+                window, scale, splits, p(err), stream()) == 0
+    got = out.cpu().double().numpy().reshape(T, nh, d)
+    assert int(err) == 0
+    for b in range(T):
+        qq = q[b].double().numpy().reshape(nh, d)
+        for h in range(nh):
+            k, v = ks[b][:, h // (nh // nkv)].double().numpy(), vs[b][:, h // (nh // nkv)].double().numpy()
+            w = weights_of(qq[h:h + 1], k, scale, window)
+            # every weight and the output rounded to bfloat16
+            assert (np.abs(got[b, h] - (w @ v)[0]) <= 2.0 ** -8 * ((w @ np.abs(v))[0] + np.abs((w @ v)[0])) + 2.0 ** -20).all()
