@@ -9,7 +9,7 @@
 // [64 keys x 64 channels] boxes of K and V straight from the page that holds them (128-byte
 // swizzle; a tile never crosses a page because pages are multiples of 64 positions) into a ring of
 // 3 (head size 128) or 6 (head size 64) stages, arming a "full" mbarrier per stage with the byte
-// count.  Four consumer warps wait for it; warp w takes keys 16w..16w+15 of every tile:
+// count (the last tile comes in boxes of 16 keys, as many as hold a visible key).  Four consumer warps wait for it; warp w takes keys 16w..16w+15 of every tile:
 // S = Q K^T with m16n8k16 MMAs (rows = the G query heads, zero rows above), scaling, masking and
 // the running softmax in float32, P V again on MMAs, then an arrive on the stage's "empty"
 // barrier.  Nothing but the ring is synchronised inside the loop.  At the end the four warps are
@@ -25,6 +25,8 @@
 // the token's new K row (rotated) and V row, writes them to the cache page and hands them through
 // shared memory to the consumer warp that owns their place in that tile.  The TMA thread starts
 // at once: it needs neither.
+// Two further forms (RdExtras): the query heads of a group beyond 16 over several blocks that walk the same keys, and the two maps
+// of a differential head as two rows, each with the other map's channels zero.
 // Formulas: src/kern/naive/naive.cpp:576-604 (scores with key head h / G), :531-553 (mask),
 // :209-240 (softmax), :634-662 (values); the reference's GPU code loops over the heads with one
 // library call each (src/kern/gpu/kernel_gpu.cu:688-756).
