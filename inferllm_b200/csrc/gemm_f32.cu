@@ -146,11 +146,21 @@ gemm_f32_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
     }
 }
 
+// Blocks go where there is room first: launched while the kernel before still holds most SMs, a grid of fewer blocks than SMs comes
+// to lie two and three to an SM beside idle ones (88 tiles of 64 x 64, K = 2,048: 190 us, spread out 80).  A grid that gives an SM at
+// most three blocks therefore asks for so much shared memory that no more of them fit.
 template <int BM, int BN, int TM, int TN>
 static int launch_gemm_f32_tile(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
     const dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN);      // the row tiles of a panel of W next to each other
     if (grid.y > 65535) return ILLM_ERR_BAD_ARG;
-    illm_launch(gemm_f32_nt_kernel<BM, BN, TM, TN>, grid, dim3((BM / TM) * (BN / TN)), 0, s, A, W, C, M, N, K, lda, ldw, ldc);
+    auto kern = gemm_f32_nt_kernel<BM, BN, TM, TN>;
+    constexpr int SM_BYTES = 228 * 1024, OWN = 2 * GF_BK * (BM + BN + 8) * (int)sizeof(float), MOST = SM_BYTES / 2 - OWN;
+    const int sms = illm_sm_count();
+    const long long per = ((long long)grid.x * grid.y + sms - 1) / sms, share = SM_BYTES / (per + 1) - OWN;
+    const int pad = per <= 3 && share > 0 ? (int)share : 0;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST);
+    if (e != cudaSuccess) return (int)e;
+    illm_launch(kern, grid, dim3((BM / TM) * (BN / TN)), pad, s, A, W, C, M, N, K, lda, ldw, ldc);
     return illm_launch_status();
 }
 
@@ -310,15 +320,14 @@ extern "C" int illm_gemm_f32_nt(const float* A, const float* W, float* C, int M,
         return launch_gemm_f32_small<8>(A, W, C, M, N, K, lda, ldw, ldc, err, s);
     }
     // A larger thread tile reads less shared memory per FMA, a smaller block leaves fewer SMs idle in the last round and fewer
-    // rows beyond M: the tile with the least work on the busiest SM, per output 1 : 1.2 : 1.6 (512 rows of 7B size: Q/K/V and
-    // gate/up 49 TF/s with 8 x 16 outputs a thread against 44 with 8 x 8).  Where an SM gets one block of the large tile, 256
-    // threads of 8 x 8 outputs hide more than 128 of 8 x 16 (output and down products 34 TF/s; 64 x 128 tiles 28).
+    // rows beyond M: the tile with the least work on the busiest SM, per output 1 : 1.2 : 1.6.  (512 rows of 7B size: Q/K/V and
+    // gate/up 47 TF/s, output and down products 41; over 294 shapes of 9 to 2,048 rows 0.55 of the time of one 64 x 64 tile of 4 x 4
+    // outputs a thread, 0.83 where it gains least.)
     cudaStream_t s = (cudaStream_t)stream;
     const int sms = illm_sm_count();
     auto rounds = [&](long long bm, long long bn) { return (double)(((M + bm - 1) / bm * ((N + bn - 1) / bn) + sms - 1) / sms); };
-    const double r0 = rounds(128, 128), c0 = r0 * 128 * 128, c1 = rounds(64, 64) * 64 * 64 * 1.2, c2 = rounds(32, 64) * 32 * 64 * 1.6;
-    if (c0 <= c1 && c0 <= c2)
-        return r0 < 2 ? launch_gemm_f32_tile<128, 128, 8, 8>(A, W, C, M, N, K, lda, ldw, ldc, s) : launch_gemm_f32_tile<128, 128, 8, 16>(A, W, C, M, N, K, lda, ldw, ldc, s);
+    const double c0 = rounds(128, 128) * 128 * 128, c1 = rounds(64, 64) * 64 * 64 * 1.2, c2 = rounds(32, 64) * 32 * 64 * 1.6;
+    if (c0 <= c1 && c0 <= c2) return launch_gemm_f32_tile<128, 128, 8, 16>(A, W, C, M, N, K, lda, ldw, ldc, s);
     if (c1 <= c2) return launch_gemm_f32_tile<64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
     return launch_gemm_f32_tile<32, 64, 4, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
 }

@@ -174,6 +174,27 @@ def test_gemm_f32_tiles(M, N, K):
         assert torch.equal(ops.gemm_f32(dev(x[r:r + 1]), dev(w)).cpu()[0], out[r])
 
 
+def test_gemm_f32_spreads_its_tiles():
+    """A product whose tiles fit the SMs once takes about as long with twice the tiles (64 and 128 of 32 x 64), behind other
+    kernels too: two tiles on one SM beside an idle one would double it."""
+    M, K, times = 64, 2048, []
+    x = torch.randn(M, K, device="cuda")
+    for N in (2048, 4096):
+        w, best = torch.randn(N, K, device="cuda"), float("inf")
+        for _ in range(5):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            ops.gemm_f32(x, w)
+            torch.cuda._sleep(1 << 22)          # the calls are in the queue before the first begins
+            begin.record()
+            for _ in range(20):
+                ops.gemm_f32(x, w)
+            end.record()
+            end.synchronize()
+            best = min(best, begin.elapsed_time(end))
+        times.append(best)
+    assert times[1] <= 1.6 * times[0], times
+
+
 @pytest.mark.parametrize("M,N,K", [(5, 96, 64), (2048, 300, 128), (1, 1000, 4096)])
 def test_linear_bf16(M, N, K):
     g = torch.Generator().manual_seed(K)
