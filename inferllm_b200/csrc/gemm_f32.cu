@@ -74,7 +74,8 @@ gemm_f32_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
     pdl_grid_sync();
     __shared__ __align__(16) float As[2][GF_BK][BM + 4];
     __shared__ __align__(16) float Ws[2][GF_BK][BN + 4];
-    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    const int m_tiles = (M + BM - 1) / BM;          // the row tiles of a panel of W next to each other
+    const int m0 = (int)(blockIdx.x % m_tiles) * BM, n0 = (int)(blockIdx.x / m_tiles) * BN;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // first row and column of the thread's first piece; the second piece lies 16 rows / 32 columns further on
     const int tm = (warp / WARPS_N) * 4 * TM + (lane >> 3) * 4, tn = (warp % WARPS_N) * 8 * TN + (lane & 7) * 4;
@@ -151,16 +152,16 @@ gemm_f32_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, flo
 // most three blocks therefore asks for so much shared memory that no more of them fit.
 template <int BM, int BN, int TM, int TN>
 static int launch_gemm_f32_tile(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
-    const dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN);      // the row tiles of a panel of W next to each other
-    if (grid.y > 65535) return ILLM_ERR_BAD_ARG;
+    const long long tiles = ((long long)M + BM - 1) / BM * (((long long)N + BN - 1) / BN);
+    if (tiles > 0x7fffffffLL) return ILLM_ERR_BAD_ARG;
     auto kern = gemm_f32_nt_kernel<BM, BN, TM, TN>;
     constexpr int SM_BYTES = 228 * 1024, OWN = 2 * GF_BK * (BM + BN + 8) * (int)sizeof(float), MOST = SM_BYTES / 2 - OWN;
     const int sms = illm_sm_count();
-    const long long per = ((long long)grid.x * grid.y + sms - 1) / sms, share = SM_BYTES / (per + 1) - OWN;
+    const long long per = (tiles + sms - 1) / sms, share = SM_BYTES / (per + 1) - OWN;
     const int pad = per <= 3 && share > 0 ? (int)share : 0;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST);
     if (e != cudaSuccess) return (int)e;
-    illm_launch(kern, grid, dim3((BM / TM) * (BN / TN)), pad, s, A, W, C, M, N, K, lda, ldw, ldc);
+    illm_launch(kern, dim3((unsigned)tiles), dim3((BM / TM) * (BN / TN)), pad, s, A, W, C, M, N, K, lda, ldw, ldc);
     return illm_launch_status();
 }
 

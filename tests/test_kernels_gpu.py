@@ -174,6 +174,15 @@ def test_gemm_f32_tiles(M, N, K):
         assert torch.equal(ops.gemm_f32(dev(x[r:r + 1]), dev(w)).cpu()[0], out[r])
 
 
+@pytest.mark.parametrize("M,N", [(9, 4194304 + 64 + 5), (4194304 + 64 + 5, 9)])
+def test_gemm_f32_of_more_than_65535_tiles(M, N):
+    """Either size beyond 65,535 tiles of 64: whole numbers, whose sums are exact."""
+    g = torch.Generator().manual_seed(M)
+    x, w = (torch.randint(-8, 9, (n, 4), generator=g).float() for n in (M, N))
+    out = ops.gemm_f32(dev(x), dev(w)).cpu()
+    assert torch.equal(out, x @ w.T)
+
+
 def test_gemm_f32_spreads_its_tiles():
     """A product whose tiles fit the SMs once takes about as long with twice the tiles (64 and 128 of 32 x 64), behind other
     kernels too: two tiles on one SM beside an idle one would double it."""
