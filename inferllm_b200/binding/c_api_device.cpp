@@ -350,6 +350,11 @@ ILLM_API int illm_policy_ring_splits(long long T, int n_kv_heads, long long max_
 ILLM_API int illm_policy_attention_diff_splits(long long T, int head_groups, long long max_seq_len, int n_sms) {
     return ops::attention_diff_splits(T, head_groups, max_seq_len, n_sms);
 }
+// the tiles of a step's tokens into out[0] (dense) and out[1]; returns the form in which attention_generic takes them
+ILLM_API int illm_policy_attention_generic(const int* q_lens, int B, int nh, int n_sms, int* out) {
+    ops::count_token_tiles(q_lens, B, out[0], out[1]);
+    return ops::attention_generic_form(out[0], out[1], nh, n_sms);
+}
 // which: 0 decode_ring, 1 decode (split keys), 2 decode_gqa, 3 prefill (mma.sync), 4 prefill_tc
 ILLM_API int illm_policy_attention_supported(int which, int dtype, int nh, int nkv, int d, int page_size) {
     const DType t = (DType)dtype;

@@ -17,6 +17,7 @@
 //                                  and prompts behind a sliding window;
 //   attention_generic_tile_kernel  eight tokens of a prompt and a head per block: a key or value row that a warp has
 //                                  read serves all of them.
+// In a step of both kinds of tokens each kernel takes its own tiles of eight neighbouring tokens (ag_dense).
 //   score = (q . k) * scale;  keys lo..p with lo = first_visible(p, span): all, a window or a chunk
 //
 // Four options for mixers that are more than the plain softmax attention: values of another head
@@ -83,7 +84,18 @@ struct AgArgs {
     const float *sinks, *gate;
     int gate_stride, gate_wide;
     float softcap;
+    int mixed;          // the tile kernel takes the dense tiles of AG_TILE tokens alone, the other kernel the rest
 };
+
+#define AG_TILE 8
+// Whether the tile of tokens t0 .. t0 + n - 1 is worth the tile kernel: it walks the keys once per sequence in the tile, for the
+// price of about three tokens by themselves.  (512 prompt tokens beside 40 single tokens at 2,000 keys, 32 heads of 128 in
+// float32: every token by itself 1,380 us, all by tiles 2,300, each kind its own way 850.)  ops::attention_generic_form counts with the same rule.
+__device__ __forceinline__ bool ag_dense(const int* token_seq, int t0, int n) {
+    int seqs = 1;
+    for (int i = 1; i < n; i++) seqs += token_seq[t0 + i] != token_seq[t0 + i - 1];
+    return 3 * seqs <= n;
+}
 
 // NV: value channels per lane (dv <= 32 NV).  G blocks of a cluster share a (token, head): each runs sixteen / G of its
 // strands and leaves their sums in block 0's shared memory, which merges them.  A single token of a few heads is
@@ -98,6 +110,7 @@ __global__ void __launch_bounds__(AG_WARPS / G * 32) attention_generic_kernel(co
 
     const int d = a.d, dv = a.dv, page_size = a.page_size;
     const int t = blockIdx.x / G, h = blockIdx.y, part = blockIdx.x % G;
+    if (G == 1 && a.mixed && ag_dense(a.token_seq, t / AG_TILE * AG_TILE, min(AG_TILE, a.T - t / AG_TILE * AG_TILE))) return;
     const int lane = threadIdx.x & 31, warp = part * (AG_WARPS / G) + (threadIdx.x >> 5);
     const int hk = h / (a.nh / a.nkv);
     const int p = a.token_pos[t];
@@ -204,7 +217,6 @@ __global__ void __launch_bounds__(AG_WARPS / G * 32) attention_generic_kernel(co
 // float32 multiply-adds (d + dv per key and token) and the shared-memory reads of q between them; a prompt of 512
 // tokens and 32 heads of 128 in float32 took 1,140 us per layer with a block per (token, head), which read each key
 // and value row from L2 once per token.
-#define AG_TILE 8
 #define AG_TILE_WARPS 8
 template <typename TA, int NV>
 __global__ void __launch_bounds__(AG_TILE_WARPS * 32, 2) attention_generic_tile_kernel(const AgArgs a) {
@@ -223,6 +235,7 @@ __global__ void __launch_bounds__(AG_TILE_WARPS * 32, 2) attention_generic_tile_
         pos_s[threadIdx.x] = (int)threadIdx.x < n ? a.token_pos[t0 + threadIdx.x] : 0;
         seq_s[threadIdx.x] = (int)threadIdx.x < n ? a.token_seq[t0 + threadIdx.x] : -1;
     }
+    if (a.mixed && !ag_dense(a.token_seq, t0, n)) return;
     __syncthreads();
     for (int f = 0, e; f < n; f = e) {                // tokens f .. e - 1 share their keys
         const int lo = first_visible(pos_s[f], a.span), seq = seq_s[f];
@@ -344,26 +357,28 @@ static int ag_launch(const AgArgs& a, cudaStream_t s) {
 }
 
 template <typename TA, int NV>
-static int ag_launch_for(const AgArgs& a, bool prompts, cudaStream_t s) {
+static int ag_launch_for(AgArgs a, int prompts, cudaStream_t s) {
     // Tokens of prompts share key blocks unless every token's window begins somewhere else.
+    a.mixed = 0;
     if (NV == 4 && prompts && a.span <= 0 && a.d <= 128 && a.d % 8 == 0) {
+        a.mixed = prompts == 2;
         const size_t smem = (size_t)AG_TILE * ((size_t)a.d + (size_t)AG_WARPS * a.dv) * sizeof(float);
         auto kern = attention_generic_tile_kernel<TA, 4>;
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         illm_launch(kern, dim3((a.T + AG_TILE - 1) / AG_TILE, a.nh), dim3(AG_TILE_WARPS * 32), smem, s, a);
-        return illm_launch_status();
+        return a.mixed ? ag_launch<TA, NV, 1>(a, s) : illm_launch_status();
     }
     // as many blocks per (token, head) as leave every SM at most about two
-    const long long pairs = (long long)a.T * a.nh;
-    if (pairs <= 37) return ag_launch<TA, NV, 8>(a, s);
-    if (pairs <= 74) return ag_launch<TA, NV, 4>(a, s);
-    if (pairs <= 148) return ag_launch<TA, NV, 2>(a, s);
+    const long long pairs = (long long)a.T * a.nh, sms = illm_sm_count();
+    if (pairs <= sms / 4) return ag_launch<TA, NV, 8>(a, s);
+    if (pairs <= sms / 2) return ag_launch<TA, NV, 4>(a, s);
+    if (pairs <= sms) return ag_launch<TA, NV, 2>(a, s);
     return ag_launch<TA, NV, 1>(a, s);
 }
 
-// span: see first_visible; gate_wide: a gate per value channel; softcap 0: none; prompts: the step holds more than one token
-// of a sequence (which kernel runs follows from it; the results do not)
+// span: see first_visible; gate_wide: a gate per value channel; softcap 0: none; prompts: 0 every token by itself, 1 tokens by
+// eights, 2 by eights where eight neighbours are worth it (which kernel runs follows from it; the results do not)
 extern "C" int illm_attention_generic_ex(const void* q, int q_stride, const void* kc, const void* vc,
                                          const int* block_table, int max_pages, const int* token_pos,
                                          const int* token_seq, void* out, int act_dtype, int T, int nh,
@@ -374,10 +389,10 @@ extern "C" int illm_attention_generic_ex(const void* q, int q_stride, const void
     if (dv <= 0) dv = d;
     if (d <= 0 || d > AG_MAX_D || dv > AG_MAX_D || nkv <= 0 || nh % nkv || nh > 65535) return ILLM_ERR_BAD_ARG;
     const AgArgs a{q, kc, vc, q_stride, block_table, max_pages, token_pos, token_seq, out, T, nh, nkv, d, page_size, span, scale, dv, sinks, gate,
-                   gate_stride, gate_wide, softcap};
+                   gate_stride, gate_wide, softcap, 0};
     cudaStream_t s = (cudaStream_t)stream;
-    if (act_dtype == ILLM_BF16) return dv <= 128 ? ag_launch_for<bf16, 4>(a, prompts != 0, s) : ag_launch_for<bf16, 8>(a, prompts != 0, s);
-    if (act_dtype == ILLM_F32) return dv <= 128 ? ag_launch_for<float, 4>(a, prompts != 0, s) : ag_launch_for<float, 8>(a, prompts != 0, s);
+    if (act_dtype == ILLM_BF16) return dv <= 128 ? ag_launch_for<bf16, 4>(a, prompts, s) : ag_launch_for<bf16, 8>(a, prompts, s);
+    if (act_dtype == ILLM_F32) return dv <= 128 ? ag_launch_for<float, 4>(a, prompts, s) : ag_launch_for<float, 8>(a, prompts, s);
     return ILLM_ERR_BAD_ARG;
 }
 

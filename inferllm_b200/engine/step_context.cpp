@@ -88,6 +88,7 @@ StepContext StepContextBuilder::build(const SequenceCache& cache, const StepPlan
     ctx.B = B;
     ctx.K = K;
     ctx.max_q = max_q;
+    ops::count_token_tiles(plan.q_lens.data(), B, ctx.dense_tiles, ctx.sparse_tiles);
     ctx.max_len = max_len;
     ctx.max_seq_len = cache.max_seq_len;
     ctx.is_decode = max_q == 1;

@@ -67,6 +67,32 @@ int gemm_tc_splits(long long M, long long N, long long K, int n_sms) {
     return (int)ceil_div(k_iters, per);          // every slice owns at least one 64-wide piece of K
 }
 
+void count_token_tiles(const int* q_lens, int B, int& dense, int& sparse) {
+    dense = sparse = 0;
+    int tokens = 0, seqs = 0;           // of the tile that is being filled
+    auto close = [&] {
+        (3 * seqs <= tokens ? dense : sparse)++;
+        tokens = seqs = 0;
+    };
+    for (int b = 0; b < B; b++)
+        for (int left = q_lens[b]; left > 0;) {
+            if (tokens == 0 && left >= 8) {
+                dense += left / 8;
+                left %= 8;
+                continue;
+            }
+            const int n = std::min(left, 8 - tokens);
+            tokens += n, seqs++, left -= n;
+            if (tokens == 8) close();
+        }
+    if (tokens) close();
+}
+
+int attention_generic_form(int dense_tiles, int sparse_tiles, int n_heads, int n_sms) {
+    if ((long long)dense_tiles * n_heads < n_sms) return 0;
+    return sparse_tiles ? 2 : 1;
+}
+
 int attention_decode_ring_splits(long long T, int n_kv_heads, long long max_len, int head_dim, int n_sms, double stream_bytes_per_us) {
     const long long pairs = std::max<long long>(1, T * n_kv_heads), tiles = std::max<long long>(1, ceil_div(max_len, 64));
     const long long slots = 2LL * n_sms;
@@ -451,7 +477,7 @@ Mat attention_generic(Device& dev, const Mat& qkv, const KVView& kv, const StepV
                                            code_of(qkv.dtype, "attention_generic"), (int)qkv.rows, g.n_heads, g.n_kv_heads, g.head_dim, kv.page_size,
                                            kv.span(), scale, dv, extras ? extras->sinks : nullptr, extras ? extras->gate : nullptr,
                                            extras ? extras->gate_stride : 0, extras && extras->wide_gate ? 1 : 0, extras ? extras->softcap : 0.f,
-                                           ctx.is_decode ? 0 : 1, dev.stream()),
+                                           attention_generic_form(ctx.dense_tiles, ctx.sparse_tiles, g.n_heads, dev.n_sms()), dev.stream()),
                  "attention_generic");
     return out;
 }

@@ -338,10 +338,10 @@ def rope_kv_write(qkv, cos_sin, rot_dim, token_pos, token_seq, block_table, k_ca
 
 
 def attention_generic(qkv, k_cache, v_cache, block_table, token_pos, token_seq, n_heads,
-                      n_kv_heads, head_dim, page_size, window, scale, prompts=False):
+                      n_kv_heads, head_dim, page_size, window, scale, prompts=0):
     """Attention of each token (query heads in the first n_heads*head_dim columns of `qkv`)
     over its sequence's cache pages; returns [T, n_heads*head_dim].  `window` may be negative: chunks of that many
-    positions.  `prompts`: the step holds more than one token of a sequence (another kernel, the same result)."""
+    positions.  `prompts`: 1 takes the tokens by eights, 2 those that are worth it (other kernels, the same result)."""
     if head_dim % 8 or head_dim > MAX_HEAD_DIM_GENERIC:
         raise KernelError(f"attention: head size {head_dim} is not supported (multiples of 8 up to "
                           f"{MAX_HEAD_DIM_GENERIC})")
@@ -356,7 +356,7 @@ def attention_generic(qkv, k_cache, v_cache, block_table, token_pos, token_seq, 
         _ptr(qkv), qkv.shape[1], _ptr(k_cache), _ptr(v_cache), _ptr(block_table),
         block_table.shape[1], _ptr(token_pos), _ptr(token_seq), _ptr(out), act_code(qkv.dtype), T,
         n_heads, n_kv_heads, head_dim, page_size, int(window or 0), float(scale), head_dim, None, None, 0,
-        0, 0.0, 1 if prompts else 0, _stream()),
+        0, 0.0, int(prompts), _stream()),
         "attention_generic")
     return out
 
@@ -442,6 +442,13 @@ def attention_diff_splits(T, head_groups, max_seq_len, n_sms=None) -> int:
     """Blocks per (token, group of query heads) of the single-token kernel of differential attention: the engine's
     policy (`ops::attention_diff_splits`), for the SM count of the current device unless given."""
     return int(_b.lib().illm_policy_attention_diff_splits(int(T), int(head_groups), int(max_seq_len), int(n_sms or n_sms_of_device())))
+
+
+def attention_generic_form(q_lens, n_heads, n_sms=None):
+    """How the engine's policy has `attention_generic` take a step whose sequences bring `q_lens` tokens (0 one by one, 1 by eights, 2 by
+    eights where that is worth it), and the step's dense and sparse tiles of eight tokens."""
+    lens, tiles = (ctypes.c_int * len(q_lens))(*q_lens), (ctypes.c_int * 2)()
+    return int(_b.lib().illm_policy_attention_generic(lens, len(q_lens), int(n_heads), int(n_sms or n_sms_of_device()), tiles)), tiles[0], tiles[1]
 
 
 def attention_decode_ring(qkv, k_cache, v_cache, block_table, token_pos, token_seq, n_heads, n_kv_heads,

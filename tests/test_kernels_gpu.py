@@ -724,7 +724,7 @@ def test_attention_generic_bits_do_not_depend_on_the_kernel(dtype, nh, nkv, d, p
     every = list(range(T))
     out = run(every, False)
     assert torch.isfinite(out.float()).all()
-    assert torch.equal(run(every, True), out)
+    assert torch.equal(run(every, True), out) and torch.equal(run(every, 2), out)
     for n in (1, 9, 36):               # 36 tokens of 40 heads: a block each; fewer: clusters of 2, 4, 8
         some = every[5:5 + n]
         assert torch.equal(run(some, False), out[some]) and torch.equal(run(some, True), out[some])

@@ -1,5 +1,7 @@
 """Host-side choices that need no GPU: how many blocks the decode attention gives a (token, KV head)
 pair, and how many K slices a decode-sized product is cut into."""
+import numpy as np
+
 from inferllm_b200.kernels import ops
 
 
@@ -36,6 +38,23 @@ def test_split_k_of_decode_sized_products():
     assert ops.gemm_tc_splits(65, 4096, 4096) == 1   # larger steps are not split
     assert ops.gemm_tc_splits(8, 22016, 4096) == 1   # 172 tiles fill the GPU by themselves
     assert ops.gemm_tc_splits(8, 4096, 4096) == 8
+
+
+def test_how_generic_attention_takes_a_steps_tokens():
+    """Tokens by eights where the tiles of one or two sequences fill the SMs, single tokens beside them one by one; the counts against a
+    walk over the tokens."""
+    form = lambda lens, heads=32: ops.attention_generic_form(lens, heads, 148)  # noqa: E731
+    rng = np.random.default_rng(0)
+    for _ in range(300):
+        lens = rng.choice([0, 1, 2, 3, 7, 8, 9, 17, 40], rng.integers(1, 12)).tolist()
+        seqs = np.repeat(np.arange(len(lens)), lens)
+        tiles = [seqs[i:i + 8] for i in range(0, len(seqs), 8)]
+        dense = sum(3 * len(set(t.tolist())) <= len(t) for t in tiles)
+        assert form(lens)[1:] == (dense, len(tiles) - dense), lens
+    assert form([512]) == (1, 64, 0) and form([300, 200, 100])[0] == 1 and form([20] * 8)[0] == 1
+    assert form([512] + [1] * 40) == (2, 64, 5)         # the single tokens' tiles are not walked by eights
+    assert form([1] * 64)[0] == 0 and form([17] + [1] * 63)[0] == 0 and form([3] * 4)[0] == 0
+    assert form([64], heads=4)[0] == 0 and form([17], heads=4)[0] == 0      # few blocks: a block per token
 
 
 def test_differential_decode_splits():
