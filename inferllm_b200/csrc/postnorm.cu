@@ -56,7 +56,8 @@ scale_add_rmsnorm_kernel(float* __restrict__ resid, const TD* __restrict__ delta
 // before drains, and the row's pieces of the stream, the addend and up to eight of its slices are on their way together: a
 // single token's block is bound by the latency of its loads (one row of 2,048 with eight slices took 7 us channel by
 // channel with the sum going out to the stream and back).
-template <typename TD, typename TY, int IT>
+// SLICES: the addend comes as slices.
+template <typename TD, typename TY, int IT, bool SLICES>
 __global__ void __launch_bounds__(1024)
 scale_add_rmsnorm_vec_kernel(float* __restrict__ resid, const TD* __restrict__ delta, const float* __restrict__ w, TY* __restrict__ y, int H,
                              float alpha, float eps, const float* __restrict__ partials, int splits, long long split_stride) {
@@ -78,8 +79,8 @@ scale_add_rmsnorm_vec_kernel(float* __restrict__ resid, const TD* __restrict__ d
         if (c >= H) continue;
         const float4 x = row_load4(resid + base + c);
         float4 add = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (delta) add = row_load4(delta + base + c);
-        else if (partials) add = row_sum_slices(partials + base + c, splits, split_stride);
+        if (SLICES) add = row_sum_slices(partials + base + c, splits, split_stride);
+        else if (delta) add = row_load4(delta + base + c);
         v[i] = make_float4(fmaf(alpha, x.x, add.x), fmaf(alpha, x.y, add.y), fmaf(alpha, x.z, add.z), fmaf(alpha, x.w, add.w));
         ss = fmaf(v[i].x, v[i].x, ss), ss = fmaf(v[i].y, v[i].y, ss), ss = fmaf(v[i].z, v[i].z, ss), ss = fmaf(v[i].w, v[i].w, ss);
     }
@@ -104,8 +105,9 @@ extern "C" int illm_scale_add_rmsnorm(float* resid, const void* delta, int delta
     // which kernel runs and its threads follow from the width and the layout alone, so a row's sums have the same order in every launch
     if (H % 4 == 0 && row_pieces(H) && split_stride % 4 == 0 && !row_odd(resid) && !row_odd(delta) && !row_odd(w) && !row_odd(y) && !row_odd(partials)) {
         const int pieces = row_pieces(H), vthreads = row_threads(H);
+        const bool slices = !delta && partials && splits > 0;
 #define ILLM_PNV(TD, TY, IT)                                                                                                          \
-    illm_launch(scale_add_rmsnorm_vec_kernel<TD, TY, IT>, dim3(n_rows), dim3(vthreads), 0, s, resid, (const TD*)delta, w, (TY*)y, H, alpha, eps, \
+    illm_launch(slices ? scale_add_rmsnorm_vec_kernel<TD, TY, IT, true> : scale_add_rmsnorm_vec_kernel<TD, TY, IT, false>, dim3(n_rows), dim3(vthreads), 0, s, resid, (const TD*)delta, w, (TY*)y, H, alpha, eps, \
                 partials, splits, split_stride)
 #define ILLM_PNV_FOR(TD, TY)                            \
     do {                                                \

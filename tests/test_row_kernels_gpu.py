@@ -70,6 +70,51 @@ def test_norm_sandwich(H, center, with_y, with_rows):
     close(out, ref, 4 * math.sqrt(H) + 32, np.abs(ref) + 4 * w.abs().double().numpy())
 
 
+@pytest.mark.parametrize("H", [64, 4096, 5120, 8192, 12288, 20480, 4097])
+@pytest.mark.parametrize("center", [0, 1])
+def test_norm_sandwich_rows_do_not_depend_on_the_step(H, center):
+    """A row of many (more than the SMs, which take another form of the kernel) has the bits that it has alone."""
+    g = torch.Generator().manual_seed(H + center)
+    n, post = 400, 1.0 if center else 0.5
+    x, y, wb, w = (torch.randn(*s, generator=g).cuda() for s in ((n, H), (n, H), (H,), (H,)))
+    f = entry("illm_norm_sandwich", I_, P_, P_, P_, P_, P_, I_, P_, I_, I_, F_, I_, I_, F_, P_)
+
+    def run(at, rows):
+        xd, yd, out = x[at:at + rows].clone(), y[at:at + rows].clone(), torch.empty(rows, H, device="cuda")
+        assert f(p(xd), p(yd), p(wb), p(w), p(out), 0, None, rows, H, 1e-5, 1, center, post, stream()) == 0
+        return xd, out
+
+    many = run(0, n)
+    for at in (0, 7, n - 1):
+        for a, b in zip(run(at, 1), many):
+            assert torch.equal(a[0], b[at])
+
+
+@pytest.mark.parametrize("name", ["illm_norm_sandwich", "illm_add2_rmsnorm", "illm_scaled_add_rmsnorm"])
+def test_norms_of_wide_rows_take_their_bytes_time(name):
+    """2,048 rows of 20,480 channels beside as many of 8,192, both at the rate of memory: 2.5 times the bytes, at most twice that in time."""
+    f = entry(name, I_, P_, P_, P_, P_, P_, I_, P_, I_, I_, F_, I_, I_, F_, P_) if "sandwich" in name else entry(name, I_, P_, P_, P_, P_, P_, I_, I_, I_, F_, P_)
+    n, times = 2048, []
+    for H in (8192, 20480):
+        x, a, b, w = (torch.randn(*s, device="cuda") for s in ((n, H), (n, H), (n, H), (H,)))
+        y = torch.empty(n, H, dtype=torch.bfloat16, device="cuda")
+        args = {"illm_norm_sandwich": (p(x), p(a), p(w), p(w), p(y), 1, None, n, H, 1e-5, 1, 0, 0.5), "illm_add2_rmsnorm": (p(x), p(a), p(b), p(w), p(y), 1, n, H, 1e-5),
+                "illm_scaled_add_rmsnorm": (p(x), p(a), p(w), p(w), p(y), 1, n, H, 1e-5)}[name]
+        best = float("inf")
+        for _ in range(5):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            assert f(*args, stream()) == 0
+            torch.cuda._sleep(1 << 21)
+            begin.record()
+            for _ in range(5):
+                f(*args, stream())
+            end.record()
+            end.synchronize()
+            best = min(best, begin.elapsed_time(end))
+        times.append(best)
+    assert times[1] <= 5 * times[0], times
+
+
 @pytest.mark.parametrize("width,group", [(2048, 2048), (1032, 516), (8192, 8192), (1024, 128), (12, 4), (8196, 8196), (30, 15)])
 @pytest.mark.parametrize("act", [1, 2])
 def test_group_norm_gate(width, group, act):
