@@ -56,8 +56,10 @@ __device__ __forceinline__ float rotated(const float* buf, int e, int rot, int p
     }
     const float c = cs[2 * j], s = cs[2 * j + 1];
     const float a = buf[e], b = buf[partner];
-    return first ? a * c - b * s : a * c + b * s;
+    return fmaf(a, c, first ? -__fmul_rn(b, s) : __fmul_rn(b, s));       // explicit: the same bits in every kernel of this file
 }
+
+__device__ __forceinline__ float mixed(float own, float first, float lambda) { return fmaf(1.0f - lambda, own, __fmul_rn(lambda, first)); }
 
 template <typename TI, typename TA>
 __global__ void __launch_bounds__(256) qk_prep_kernel(QkPrepArgs a) {
@@ -137,7 +139,7 @@ __global__ void __launch_bounds__(256) qk_prep_kernel(QkPrepArgs a) {
         float v = to_f32(x[a.v_off + c]);
         if (a.bv) v += a.bv[c];
         if (a.v_keep) a.v_keep[(size_t)t * nv + c] = v;
-        if (a.v_first) v = (1.0f - lambda) * v + lambda * a.v_first[(size_t)t * a.v_first_ld + c];
+        if (a.v_first) v = mixed(v, a.v_first[(size_t)t * a.v_first_ld + c], lambda);
         ((TA*)a.vc)[(((size_t)page * a.nkv + hk) * a.page_size + slot) * a.dv + e] = from_f32<TA>(v);
     }
 }
@@ -149,8 +151,11 @@ __global__ void __launch_bounds__(256) qk_prep_kernel(QkPrepArgs a) {
 // took 13 to 17 us for one token of 32 + 2 x 8 heads of 128.  A head's norm is added within the d / 4 lanes that hold the head (d / 4 a power
 // of two up to 32).  Only the rotate-half layout, whose channels pair up across threads, goes through shared memory.
 // The block size follows from the sizes alone, so that a row's sums have one order in every step.
-template <typename TI, typename TA, int IT>
-__global__ void __launch_bounds__(1024) qk_prep_vec_kernel(const QkPrepArgs a) {
+// EARLY false: the same sums in the same order with the weights, biases and values to mix in read where they are used, so that two
+// blocks lie on an SM, for steps of more tokens than SMs (2,000 tokens of 32 + 2 x 8 heads of 128, norms over all heads, rotate-half: 68 us,
+// so 47).  Four pieces a thread leave no registers for early reads at any number of tokens.
+template <typename TI, typename TA, int IT, bool EARLY>
+__global__ void __launch_bounds__(1024, EARLY || IT > 2 ? 1 : 2) qk_prep_vec_kernel(const QkPrepArgs a) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     extern __shared__ __align__(16) float buf[];      // the rotate-half layout: [nh d] q, then [nkv d] k
     __shared__ float scratch[32];
@@ -159,17 +164,21 @@ __global__ void __launch_bounds__(1024) qk_prep_vec_kernel(const QkPrepArgs a) {
     const bool whole = a.wq && !a.head_norm, halves = a.rot && !a.pairs;
     // weights, biases and the indices of the step are no result of the kernel before
     const int pos = a.token_pos[t];
-    float4 w[IT], bias[IT];
-#pragma unroll
-    for (int i = 0; i < IT; i++) {
-        const int at = threadIdx.x + i * threads;
+    auto weight = [&](int at) {
         const bool is_q = at < nq4, is_k = !is_q && at < nq4 + nk4;
-        const int c = is_q ? at : is_k ? at - nq4 : at - nq4 - nk4;
         const float* wp = is_q ? a.wq : is_k ? a.wk : nullptr;
+        const int c = is_q ? at : at - nq4;
+        return wp ? row_load4(wp + 4 * (a.head_norm ? c % d4 : c)) : make_float4(1.f, 1.f, 1.f, 1.f);
+    };
+    auto bias_of = [&](int at) {
+        const bool is_q = at < nq4, is_k = !is_q && at < nq4 + nk4;
         const float* bp = is_q ? a.bq : is_k ? a.bk : a.bv;
-        const bool in = at < nq4 + nk4 + nv4;
-        w[i] = in && wp ? *reinterpret_cast<const float4*>(wp + 4 * (a.head_norm ? c % d4 : c)) : make_float4(1.f, 1.f, 1.f, 1.f);
-        bias[i] = in && bp ? *reinterpret_cast<const float4*>(bp + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        return bp && at < nq4 + nk4 + nv4 ? row_load4(bp + 4 * (is_q ? at : is_k ? at - nq4 : at - nq4 - nk4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    float4 w[IT], bias[IT];
+    if (EARLY) {
+#pragma unroll
+        for (int i = 0; i < IT; i++) w[i] = weight(threadIdx.x + i * threads), bias[i] = bias_of(threadIdx.x + i * threads);
     }
     const int page = nk4 && a.kc ? a.block_table[(size_t)a.token_seq[t] * a.max_pages + pos / a.page_size] : -1;
     int p = pos;
@@ -189,12 +198,13 @@ __global__ void __launch_bounds__(1024) qk_prep_vec_kernel(const QkPrepArgs a) {
         const bool is_q = at < nq4, is_k = !is_q && at < nq4 + nk4, is_v = !is_q && !is_k && at < nq4 + nk4 + nv4;
         const int c = is_q ? at : is_k ? at - nq4 : at - nq4 - nk4, off = is_q ? a.q_off : is_k ? a.k_off : a.v_off;
         v[i] = is_q || is_k || is_v ? row_load4(x + off + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
-        first[i] = is_v && a.v_first ? *reinterpret_cast<const float4*>(a.v_first + (size_t)t * a.v_first_ld + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (EARLY) first[i] = is_v && a.v_first ? row_load4(a.v_first + (size_t)t * a.v_first_ld + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     float ssq = 0.f, ssk = 0.f;
 #pragma unroll
     for (int i = 0; i < IT; i++) {
         const int at = threadIdx.x + i * threads;
+        if (!EARLY) bias[i] = bias_of(at);
         v[i].x += bias[i].x, v[i].y += bias[i].y, v[i].z += bias[i].z, v[i].w += bias[i].w;
         if (at < nq4 && a.qt_every > 0) v[i].x *= q_temp, v[i].y *= q_temp, v[i].z *= q_temp, v[i].w *= q_temp;
         float s = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, v[i].w * v[i].w)));
@@ -202,6 +212,7 @@ __global__ void __launch_bounds__(1024) qk_prep_vec_kernel(const QkPrepArgs a) {
             for (int o = 1; o < d4; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
             if (at < nq4 + nk4) {
                 const float inv = 1.0f / sqrtf(s / (float)a.d + a.eps);
+                if (!EARLY) w[i] = weight(at);
                 v[i].x = (v[i].x * inv) * w[i].x, v[i].y = (v[i].y * inv) * w[i].y, v[i].z = (v[i].z * inv) * w[i].z, v[i].w = (v[i].w * inv) * w[i].w;
             }
         }
@@ -217,6 +228,7 @@ __global__ void __launch_bounds__(1024) qk_prep_vec_kernel(const QkPrepArgs a) {
             const int at = threadIdx.x + i * threads;
             if (at >= nq4 && (at >= nq4 + nk4 || !a.wk)) continue;
             const float inv = at < nq4 ? inv_q : inv_k;
+            if (!EARLY) w[i] = weight(at);
             v[i].x = (v[i].x * inv) * w[i].x, v[i].y = (v[i].y * inv) * w[i].y, v[i].z = (v[i].z * inv) * w[i].z, v[i].w = (v[i].w * inv) * w[i].w;
         }
     }
@@ -229,6 +241,8 @@ __global__ void __launch_bounds__(1024) qk_prep_vec_kernel(const QkPrepArgs a) {
         __syncthreads();
     }
     if (page < 0 && nk4 && a.kc && threadIdx.x == 0) atomicExch(a.err, 2);
+    auto turn = [](float x, float c, float y, float s) { return fmaf(x, c, __fmul_rn(y, s)); };
+    auto mix = [&](float x, float y) { return mixed(x, y, lambda); };
     const int slot = pos % a.page_size;
 #pragma unroll
     for (int i = 0; i < IT; i++) {
@@ -239,7 +253,7 @@ __global__ void __launch_bounds__(1024) qk_prep_vec_kernel(const QkPrepArgs a) {
             if (e < a.rot) {
                 if (a.pairs) {
                     const float4 f = *reinterpret_cast<const float4*>(cs + e);      // cos, sin of the two pairs
-                    v[i] = make_float4(v[i].x * f.x - v[i].y * f.y, v[i].y * f.x + v[i].x * f.y, v[i].z * f.z - v[i].w * f.w, v[i].w * f.z + v[i].z * f.w);
+                    v[i] = make_float4(turn(v[i].x, f.x, -v[i].y, f.y), turn(v[i].y, f.x, v[i].x, f.y), turn(v[i].z, f.z, -v[i].w, f.w), turn(v[i].w, f.z, v[i].z, f.w));
                 } else {
                     const float* head = buf + 4 * (at - (c - hd * d4));
                     v[i].x = rotated(head, e, a.rot, 0, cs);
@@ -253,9 +267,9 @@ __global__ void __launch_bounds__(1024) qk_prep_vec_kernel(const QkPrepArgs a) {
         } else if (page >= 0) {
             const int c = at - nq4 - nk4, hd = c / (a.dv >> 2), e = (c - hd * (a.dv >> 2)) * 4;
             if (a.v_keep) *reinterpret_cast<float4*>(a.v_keep + (size_t)t * 4 * nv4 + 4 * c) = v[i];
+            if (!EARLY && a.v_first) first[i] = row_load4(a.v_first + (size_t)t * a.v_first_ld + 4 * c);
             if (a.v_first)
-                v[i] = make_float4((1.0f - lambda) * v[i].x + lambda * first[i].x, (1.0f - lambda) * v[i].y + lambda * first[i].y,
-                                   (1.0f - lambda) * v[i].z + lambda * first[i].z, (1.0f - lambda) * v[i].w + lambda * first[i].w);
+                v[i] = make_float4(mix(v[i].x, first[i].x), mix(v[i].y, first[i].y), mix(v[i].z, first[i].z), mix(v[i].w, first[i].w));
             row_store4((TA*)a.vc + (((size_t)page * a.nkv + hd) * a.page_size + slot) * a.dv + e, v[i]);
         }
     }
@@ -285,8 +299,9 @@ static int qk_prep_vec_launch(const QkPrepArgs& a, int T, cudaStream_t s) {
     if (smem > 200 * 1024) return -1;
 #define ILLM_QKV(IT)                                                                                                                          \
     do {                                                                                                                                      \
-        if (smem > 48 * 1024) cudaFuncSetAttribute(qk_prep_vec_kernel<TI, TA, IT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
-        illm_launch(qk_prep_vec_kernel<TI, TA, IT>, dim3(T), dim3(threads), smem, s, a);                                                       \
+        auto kern = T <= illm_sm_count() ? qk_prep_vec_kernel<TI, TA, IT, IT <= 2> : qk_prep_vec_kernel<TI, TA, IT, false>;                    \
+        if (smem > 47 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                              \
+        illm_launch(kern, dim3(T), dim3(threads), smem, s, a);                                                                                 \
     } while (0)
     if (iters == 1) ILLM_QKV(1);
     else if (iters == 2) ILLM_QKV(2);
@@ -362,7 +377,7 @@ extern "C" int illm_qk_prep_heads(const void* x, int x_dtype, int ld, int q_off,
     }
 #define ILLM_QKP(TI, TA)                                                                                                    \
     do {                                                                                                                    \
-        if (smem > 48 * 1024) cudaFuncSetAttribute(qk_prep_kernel<TI, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        if (smem > 47 * 1024) cudaFuncSetAttribute(qk_prep_kernel<TI, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
         illm_launch(qk_prep_kernel<TI, TA>, dim3(T), dim3(256), smem, s, a);                                                \
     } while (0)
     if (x_dtype == ILLM_F32 && act_dtype == ILLM_BF16) ILLM_QKP(float, bf16);
