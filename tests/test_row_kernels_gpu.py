@@ -24,6 +24,24 @@ def close(got, ref, roundings, mag=None):
     assert (np.abs(got.cpu().double().numpy() - ref) <= tol * mag + 1e-30).all()
 
 
+@pytest.mark.parametrize("H", [4, 8, 30, 1028, 4096])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("off_table,off_out", [(0, 0), (1, 0), (0, 1), (3, 2)])
+def test_scaled_embedding_at_any_address(H, dtype, off_table, off_out):
+    """Tables and outputs on 16-byte boundaries and off them, widths that are whole pieces or not: exact (one product per value)."""
+    g = torch.Generator().manual_seed(H)
+    V, T = 9, 5
+    table, ids = torch.randn(V, H, generator=g).to(dtype), torch.tensor([8, 0, 3, 3, 7], dtype=torch.int32)
+    held, out = torch.zeros(V * H + 8, dtype=dtype, device="cuda"), torch.full((T * H + 8,), float("nan"), device="cuda")
+    held[off_table:off_table + V * H] = table.reshape(-1).cuda()
+    err, idd = torch.zeros(1, dtype=torch.int32, device="cuda"), ids.cuda()
+    rc = entry("illm_embedding_scaled", I_, P_, P_, P_, I_, P_, I_, I_, I_, F_, P_, P_, P_)(
+        p(idd), p(idd), held[off_table:].data_ptr(), 1 if dtype == torch.bfloat16 else 0, out[off_out:].data_ptr(), T, H, V, 1.5, None, p(err), stream())
+    assert rc == 0 and int(err) == 0
+    assert torch.equal(out[off_out:off_out + T * H].cpu().view(T, H), table.float()[ids.long()] * 1.5)
+    assert torch.isnan(out[:off_out]).all() and torch.isnan(out[off_out + T * H:]).all()
+
+
 @pytest.mark.parametrize("H", WIDTHS)
 @pytest.mark.parametrize("splits", [0, 3, 9])
 def test_scale_add_rmsnorm(H, splits):
