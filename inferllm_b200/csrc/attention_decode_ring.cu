@@ -56,6 +56,9 @@ __device__ __forceinline__ void rd_mma(float* c, const unsigned* a, unsigned b0,
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// the two bfloat16 of a register as float32
+__device__ __forceinline__ float rd_low(unsigned v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float rd_high(unsigned v) { return __uint_as_float(v & 0xffff0000u); }
 __device__ __forceinline__ unsigned rd_pack(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<unsigned*>(&v);
@@ -150,8 +153,10 @@ __device__ __forceinline__ void rd_encoded_chunk(const RdRope& rp, const bf16* _
 // What mixers beyond the plain attention add: `sinks` (float32 [nh]: one more term exp(sink) of the
 // softmax denominator, without a value), `gate` (float32, gate[t * gate_stride + h]: the head's output
 // is multiplied by its sigmoid; with gate_wide gate[t * gate_stride + h * D + c], one per channel), `softcap` (> 0: the scaled
-// scores s become softcap * tanh(s / softcap); softcap_x is 2 scale log2(e) / softcap).  WIDE: the softmax weights enter the product with V as two bfloat16
-// terms (P1 = P rounded, P2 = P - P1 rounded), sixteen bits of their mantissa instead of eight.
+// scores s become softcap * tanh(s / softcap); softcap_x is 2 scale log2(e) / softcap).  TERMS: the softmax weights enter the product with V as so many
+// bfloat16 terms (P1 = P rounded, P2 = P - P1 rounded, P3 = P - P1 - P2): 8, 16 or all 24 bits of their mantissa.  With three the
+// heads are 9e-8 to 3.4e-7 of their norm from float64 before their last rounding, on CUDA cores in float32 1.3e-7 to 5.9e-7 (with two
+// 6.5e-7 to 2.2e-6); 64 tokens of 32 heads at 2,000 keys 105.5 -> 109.6 us for it, one token of 32 heads as before.
 struct RdExtras {
     const float* sinks;
     const float* gate;
@@ -183,7 +188,7 @@ __device__ __forceinline__ float rd_finish(float num, float den, float m, const 
     return r;
 }
 
-template <int D, bool FUSE, bool WIDE>
+template <int D, bool FUSE, int TERMS>
 __global__ void __launch_bounds__(RD_THREADS + 32)
 attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                              const __grid_constant__ CUtensorMap map_k16, const __grid_constant__ CUtensorMap map_v16,
@@ -406,7 +411,7 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
                 for (int e = 0; e < 4; e++) {
                     const int key = key0 + nt * 8 + t4 * 2 + (e & 1);
                     float v = (sa[nt][e] + sb[nt][e]) * scale_log2e;
-                    if (WIDE && ex.softcap > 0.f) v = 1.4426950408889634f * soft_cap_fast(sa[nt][e] + sb[nt][e], ex.softcap, ex.softcap_x);
+                    if (TERMS > 1 && ex.softcap > 0.f) v = 1.4426950408889634f * soft_cap_fast(sa[nt][e] + sb[nt][e], ex.softcap, ex.softcap_x);
                     if (key > p || key < lo) v = -INFINITY;
                     sc[nt][e] = v;
                     mx[e >> 1] = fmaxf(mx[e >> 1], v);
@@ -422,7 +427,7 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
                 m_run[e] = m_new;
                 l_run[e] *= alpha[e];
             }
-            unsigned pf[4], pl[4];
+            unsigned pf[4], pl[4], pt[4];
 #pragma unroll
             for (int nt = 0; nt < 2; nt++) {
                 const float p0 = fast_exp2(sc[nt][0] - mref[0]), p1 = fast_exp2(sc[nt][1] - mref[0]);
@@ -431,9 +436,14 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
                 l_run[1] += p2 + p3;
                 pf[nt * 2] = rd_pack(p0, p1);
                 pf[nt * 2 + 1] = rd_pack(p2, p3);
-                if (WIDE) {     // what the rounding took away
-                    pl[nt * 2] = rd_pack(p0 - __uint_as_float(pf[nt * 2] << 16), p1 - __uint_as_float(pf[nt * 2] & 0xffff0000u));
-                    pl[nt * 2 + 1] = rd_pack(p2 - __uint_as_float(pf[nt * 2 + 1] << 16), p3 - __uint_as_float(pf[nt * 2 + 1] & 0xffff0000u));
+                if (TERMS > 1) {     // what the rounding took away (exact differences), and what the rounding of that took
+                    const float r0 = p0 - rd_low(pf[nt * 2]), r1 = p1 - rd_high(pf[nt * 2]), r2 = p2 - rd_low(pf[nt * 2 + 1]), r3 = p3 - rd_high(pf[nt * 2 + 1]);
+                    pl[nt * 2] = rd_pack(r0, r1);
+                    pl[nt * 2 + 1] = rd_pack(r2, r3);
+                    if (TERMS > 2) {
+                        pt[nt * 2] = rd_pack(r0 - rd_low(pl[nt * 2]), r1 - rd_high(pl[nt * 2]));
+                        pt[nt * 2 + 1] = rd_pack(r2 - rd_low(pl[nt * 2 + 1]), r3 - rd_high(pl[nt * 2 + 1]));
+                    }
                 }
             }
             if (key0 + 15 > p || key0 < lo) {
@@ -453,6 +463,23 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
             for (int np = 0; np < NT_D / 2; np++) {
                 unsigned b0, b1, b2, b3;
                 rd_ldm_t(b0, b1, b2, b3, vbase + rd_tile_off(vrow, np * 2 + (mtx >> 1)));
+                if (TERMS > 2) {
+                    // the 16 keys' sum from zero, the smallest terms first, and onto the running sum in float32: the tensor cores cut
+                    // off what does not fit an accumulator, which with the running sum in it is lost in one direction key by key
+                    float v0[4] = {0.f, 0.f, 0.f, 0.f}, v1[4] = {0.f, 0.f, 0.f, 0.f};
+                    rd_mma(v0, pt, b0, b1);
+                    rd_mma(v1, pt, b2, b3);
+                    rd_mma(v0, pl, b0, b1);
+                    rd_mma(v1, pl, b2, b3);
+                    rd_mma(v0, pf, b0, b1);
+                    rd_mma(v1, pf, b2, b3);
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        o[np * 2][e] = fmaf(o[np * 2][e], alpha[e >> 1], v0[e]);
+                        o[np * 2 + 1][e] = fmaf(o[np * 2 + 1][e], alpha[e >> 1], v1[e]);
+                    }
+                    continue;
+                }
                 o[np * 2][0] *= alpha[0];
                 o[np * 2][1] *= alpha[0];
                 o[np * 2][2] *= alpha[1];
@@ -463,7 +490,7 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
                 o[np * 2 + 1][3] *= alpha[1];
                 rd_mma(o[np * 2], pf, b0, b1);
                 rd_mma(o[np * 2 + 1], pf, b2, b3);
-                if (WIDE) {
+                if (TERMS > 1) {
                     rd_mma(o[np * 2], pl, b0, b1);
                     rd_mma(o[np * 2 + 1], pl, b2, b3);
                 }
@@ -606,7 +633,7 @@ template <int D>
 static int rd_launch(const void* q, int q_stride, const void* kc, const void* vc, long long n_pages,
                      const int* block_table, int max_pages, const int* token_pos, const int* token_seq,
                      float* part_acc, float* part_ml, void* out, int T, int nh, int nkv, int page_size, int window,
-                     float scale, int n_splits, int* err, cudaStream_t s, const RdRope* rope, const RdExtras* extras, bool wide) {
+                     float scale, int n_splits, int* err, cudaStream_t s, const RdRope* rope, const RdExtras* extras, int terms) {
     CUtensorMap mk, mv, mk16, mv16;
     int rc;
     const long long rows = n_pages * nkv * page_size;
@@ -618,7 +645,7 @@ static int rd_launch(const void* q, int q_stride, const void* kc, const void* vc
     if (rope) rp = *rope;
     RdExtras ex = {};
     if (extras) ex = *extras;
-    if (rope && (wide || extras)) return ILLM_ERR_BAD_ARG;      // the fused form is the plain attention's
+    if (rope && (terms > 1 || extras)) return ILLM_ERR_BAD_ARG;      // the fused form is the plain attention's
     const int groups = nkv * (ex.alias > 1 ? ex.alias : 1);
     auto launch = [&](auto kern) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -628,8 +655,10 @@ static int rd_launch(const void* q, int q_stride, const void* kc, const void* vc
                     nh / groups, page_size, window, scale * 1.4426950408889634f, err, rp, ex);
         return illm_launch_status();
     };
-    rc = rope ? launch(attention_decode_ring_kernel<D, true, false>)
-              : wide ? launch(attention_decode_ring_kernel<D, false, true>) : launch(attention_decode_ring_kernel<D, false, false>);
+    rc = rope         ? launch(attention_decode_ring_kernel<D, true, 1>)
+         : terms == 1 ? launch(attention_decode_ring_kernel<D, false, 1>)
+         : terms == 2 ? launch(attention_decode_ring_kernel<D, false, 2>)
+                      : launch(attention_decode_ring_kernel<D, false, 3>);
     if (rc != 0 || n_splits == 1 || !out) return rc;        // no out: the shares are the caller's to put together
     illm_launch(attention_decode_ring_merge_kernel<D>, dim3(nh, T), dim3(D), 0, s, (const float*)part_acc,
                 (const float*)part_ml, (bf16*)out, n_splits, nh, ex);
@@ -639,7 +668,7 @@ static int rd_launch(const void* q, int q_stride, const void* kc, const void* vc
 static int rd_run(const void* q, int q_stride, const void* kc, const void* vc, long long n_pages,
                   const int* block_table, int max_pages, const int* token_pos, const int* token_seq, float* part_acc,
                   float* part_ml, void* out, int T, int nh, int nkv, int d, int page_size, int window, float scale,
-                  int n_splits, int* err, void* stream, const RdRope* rope, const RdExtras* extras = nullptr, bool wide = false) {
+                  int n_splits, int* err, void* stream, const RdRope* rope, const RdExtras* extras = nullptr, int terms = 1) {
     if (T <= 0) return 0;
     const int alias = extras && extras->alias > 1 ? extras->alias : 1;
     if (nkv <= 0 || nh % (nkv * alias) || nh / (nkv * alias) > 16 || T > 65535 || nkv * alias > 65535 || (q_stride & 7) || page_size % RD_BN ||
@@ -650,10 +679,10 @@ static int rd_run(const void* q, int q_stride, const void* kc, const void* vc, l
     cudaStream_t s = (cudaStream_t)stream;
     if (d == 128)
         return rd_launch<128>(q, q_stride, kc, vc, n_pages, block_table, max_pages, token_pos, token_seq, part_acc,
-                              part_ml, out, T, nh, nkv, page_size, window, scale, n_splits, err, s, rope, extras, wide);
+                              part_ml, out, T, nh, nkv, page_size, window, scale, n_splits, err, s, rope, extras, terms);
     if (d == 64)
         return rd_launch<64>(q, q_stride, kc, vc, n_pages, block_table, max_pages, token_pos, token_seq, part_acc,
-                             part_ml, out, T, nh, nkv, page_size, window, scale, n_splits, err, s, rope, extras, wide);
+                             part_ml, out, T, nh, nkv, page_size, window, scale, n_splits, err, s, rope, extras, terms);
     return ILLM_ERR_BAD_ARG;
 }
 
@@ -687,7 +716,8 @@ extern "C" int illm_attention_decode_ring_ex(const void* q, int q_stride, const 
                                              page_size, window, scale, n_splits, err, wide_p, sinks, gate, gate_stride, gate_wide, softcap, 1, stream);
 }
 
-// The same with a KV head's query heads over `alias` blocks (groups of more than 16 query heads).
+// The same with a KV head's query heads over `alias` blocks (groups of more than 16 query heads).  With wide_p their weights enter in
+// three terms: such groups ran in float32 on CUDA cores before (attention_maps.cu), and keep its precision.
 extern "C" int illm_attention_decode_ring_shared(const void* q, int q_stride, const void* kc, const void* vc, long long n_pages, const int* block_table,
                                                  int max_pages, const int* token_pos, const int* token_seq, float* part_acc, float* part_ml, void* out, int T,
                                                  int nh, int nkv, int d, int page_size, int window, float scale, int n_splits, int* err, int wide_p,
@@ -695,7 +725,7 @@ extern "C" int illm_attention_decode_ring_shared(const void* q, int q_stride, co
     if (softcap > 0.f && !wide_p) return ILLM_ERR_BAD_ARG;
     RdExtras ex{sinks, gate, gate_stride, gate_wide, softcap, softcap > 0.f ? 2.0f * scale * 1.4426950408889634f / softcap : 0.f, alias, 0};
     return rd_run(q, q_stride, kc, vc, n_pages, block_table, max_pages, token_pos, token_seq, part_acc, part_ml, out, T,
-                  nh, nkv, d, page_size, window, scale, n_splits, err, stream, nullptr, &ex, wide_p != 0);
+                  nh, nkv, d, page_size, window, scale, n_splits, err, stream, nullptr, &ex, !wide_p ? 1 : alias > 1 ? 3 : 2);
 }
 
 // The same with the position encoding and the cache write inside: `qkv` is the unrotated packed
@@ -753,7 +783,7 @@ extern "C" int illm_attention_diff_ring(const void* q, int q_stride, const void*
     if (!illm_attention_diff_ring_supported(nh, nkv, d, dv, page_size) || !out) return ILLM_ERR_BAD_ARG;
     RdExtras ex{nullptr, nullptr, 0, 0, 0.f, 0.f, 1, 1};
     const int rc = rd_run(q, q_stride, kc, vc, n_pages, block_table, max_pages, token_pos, token_seq, part_acc, part_ml, nullptr, T, 2 * nh, nkv, 128, page_size,
-                          window, scale, n_splits, err, stream, nullptr, &ex, true);
+                          window, scale, n_splits, err, stream, nullptr, &ex, 3);
     if (rc) return rc;
     illm_launch(attention_diff_ring_merge_kernel<128>, dim3(nh, T), dim3(256), 0, (cudaStream_t)stream, (const float*)part_acc, (const float*)part_ml, (bf16*)out,
                 n_splits, nh, lambda, eps, out_scale);

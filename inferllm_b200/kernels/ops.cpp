@@ -855,8 +855,8 @@ Mat attention_one(Device& dev, const Mat& q, const KVView& kv, const StepView& c
 Mat attention_ex(Device& dev, const Mat& q, const KVView& kv, const StepView& ctx, Geometry g, float scale, const AttentionExtras& ex) {
     const int dv = kv.v_head_dim > 0 ? kv.v_head_dim : g.head_dim;
     if (q.dtype == DType::BF16 && dv == g.head_dim) {
-        // (A group beyond the ring's 16 rows walked the keys on CUDA cores in float32, attention_maps.cu; its blocks' weights are two
-        // bfloat16 terms.)
+        // (A group beyond the ring's 16 rows walked the keys on CUDA cores in float32, attention_maps.cu; its blocks' weights are three
+        // bfloat16 terms, all of a float32's bits.)
         const int alias = ring_alias(g.n_heads, g.n_kv_heads);
         if (ctx.is_decode && alias && attention_decode_ring_supported(q.dtype, g.n_heads / alias, g.n_kv_heads, g.head_dim, kv.page_size)) {
             MatOrPartials in;

@@ -396,6 +396,60 @@ def test_differential_attention_of_single_tokens(nh, nkv, window, lens, splits):
     assert np.linalg.norm(mine) <= 1.01 * np.linalg.norm(theirs) + 1e-6
 
 
+def shares(acc, ml, base2):
+    """(acc, maximum, sum) of a head's shares put together in float64; base2: the maxima are in units of log2."""
+    m, l = ml[..., 0].double(), ml[..., 1].double()
+    w = torch.exp2(m - m.amax(-1, keepdim=True)) if base2 else torch.exp(m - m.amax(-1, keepdim=True))
+    live = (w > 0)[..., None]
+    return ((torch.where(live, acc.double(), 0.0) * w[..., None]).sum(-2) / (l * w).sum(-1)[..., None]).cpu().numpy()
+
+
+@pytest.mark.parametrize("maps", [1, 2])
+@pytest.mark.parametrize("sharp", [0.3, 1.0, 4.0])
+def test_ring_attention_keeps_float32_weights(maps, sharp):
+    """Single tokens of differential heads (two maps) and of a group of 32 heads: what the shares hold before the output is rounded is no
+    farther from float64 than the float32 kernel's on CUDA cores.  sharp: the scores' spread."""
+    nh, nkv, d, dv, page, splits = 32, 4 if maps == 2 else 1, 64 if maps == 2 else 128, 128, 64, 4
+    lens = [17, 400, 2100]
+    T, scale = len(lens), sharp * d ** -0.5
+    g = torch.Generator().manual_seed(maps)
+    (ks, vs), pools, table = paged(lens, nkv, (maps * d, dv), g)
+    q = torch.randn(T, nh * maps * d, generator=g).bfloat16()
+    width, n_pages = table.shape[1], pools[0].shape[0]
+    dev = [t.cuda() for t in (q, *pools, table, torch.tensor(lens, dtype=torch.int32) - 1, torch.arange(T, dtype=torch.int32))]
+    err, out = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.empty(T, nh * dv, dtype=torch.bfloat16, device="cuda")
+    acc, ml = torch.empty(T, nh, maps, splits, dv, device="cuda"), torch.empty(T, nh, maps, splits, 2, device="cuda")
+    old = torch.empty(T, nh, splits, maps, dv + 2, device="cuda")
+    if maps == 2:
+        rc = entry("illm_attention_diff_ring", I_, P_, I_, P_, P_, L_, P_, I_, P_, P_, P_, P_, P_, I_, I_, I_, I_, I_, I_, I_, F_, I_, F_, F_, F_, P_, P_)(
+            p(dev[0]), nh * 2 * d, p(dev[1]), p(dev[2]), n_pages, p(dev[3]), width, p(dev[4]), p(dev[5]), p(acc), p(ml), p(out), T, nh, nkv, d, dv, page, 0, scale,
+            splits, 0.4, 1e-6, 1.0, p(err), stream())
+        rc |= entry("illm_attention_diff_decode", I_, P_, I_, P_, P_, P_, I_, P_, P_, P_, I_, I_, I_, I_, I_, I_, I_, F_, F_, F_, F_, L_, I_, P_, P_)(
+            p(dev[0]), nh * 2 * d, p(dev[1]), p(dev[2]), p(dev[3]), width, p(dev[4]), p(dev[5]), p(out), T, nh, nkv, d, dv, page, 0, scale, 0.4, 1e-6, 1.0, max(lens),
+            splits, p(old), stream())
+    else:
+        rc = entry("illm_attention_decode_ring_shared", I_, P_, I_, P_, P_, L_, P_, I_, P_, P_, P_, P_, P_, I_, I_, I_, I_, I_, I_, F_, I_, P_, I_, P_, P_, I_, I_, F_, I_,
+                   P_)(p(dev[0]), nh * d, p(dev[1]), p(dev[2]), n_pages, p(dev[3]), width, p(dev[4]), p(dev[5]), p(acc), p(ml), p(out), T, nh, nkv, d, page, 0, scale,
+                       splits, p(err), 1, None, None, 0, 0, 0.0, 2, stream())
+        rc |= entry("illm_attention_one_decode", I_, P_, I_, P_, P_, P_, I_, P_, P_, P_, I_, I_, I_, I_, I_, I_, I_, F_, F_, P_, P_, I_, I_, L_, I_, P_, P_)(
+            p(dev[0]), nh * d, p(dev[1]), p(dev[2]), p(dev[3]), width, p(dev[4]), p(dev[5]), p(out), T, nh, nkv, d, d, page, 0, scale, 0.0, None, None, 0, 0, max(lens),
+            splits, p(old), stream())
+    assert rc == 0 and int(err) == 0
+    ring, cores = shares(acc, ml, True), shares(old[..., 2:].transpose(2, 3), old[..., :2].transpose(2, 3), False)
+    num = [0.0, 0.0]
+    for b in range(T):
+        qq, k, v = q[b].double().numpy().reshape(nh, maps, d), ks[b].double().numpy().reshape(-1, nkv, maps, d), vs[b].double().numpy()
+        for h in range(nh):
+            hk = h // (nh // nkv)
+            for m in range(maps):
+                ref = (weights_of(qq[h:h + 1, m], k[:, hk, m], scale, 0) @ v[:, hk])[0]
+                for i, got in enumerate((ring, cores)):
+                    num[i] += (np.linalg.norm(got[b, h, m] - ref) / np.linalg.norm(ref)) ** 2
+    ours, theirs = (math.sqrt(x / (T * nh * maps)) for x in num)
+    print("errors before the output's rounding:", maps, sharp, ours, theirs)
+    assert ours <= theirs
+
+
 @pytest.mark.parametrize("nh,nkv,alias,d", [(32, 1, 2, 128), (20, 1, 2, 64), (96, 2, 3, 64), (128, 1, 8, 128), (6, 2, 3, 128), (4, 4, 1, 64)])
 @pytest.mark.parametrize("window,cap,sinks", [(0, 0.0, False), (70, 20.0, True)])
 @pytest.mark.parametrize("splits", [1, 5])
