@@ -25,8 +25,8 @@
 // the token's new K row (rotated) and V row, writes them to the cache page and hands them through
 // shared memory to the consumer warp that owns their place in that tile.  The TMA thread starts
 // at once: it needs neither.
-// Two further forms (RdExtras): the query heads of a group beyond 16 over several blocks that walk the same keys, and the two maps
-// of a differential head as two rows, each with the other map's channels zero.
+// Two further forms: the query heads of a group beyond 16 over several blocks that walk the same keys (RdExtras::alias), and the two
+// maps of a differential head as two rows (DIFF).
 // Formulas: src/kern/naive/naive.cpp:576-604 (scores with key head h / G), :531-553 (mask),
 // :209-240 (softmax), :634-662 (values); the reference's GPU code loops over the heads with one
 // library call each (src/kern/gpu/kernel_gpu.cu:688-756).
@@ -157,6 +157,8 @@ __device__ __forceinline__ void rd_encoded_chunk(const RdRope& rp, const bf16* _
 // bfloat16 terms (P1 = P rounded, P2 = P - P1 rounded, P3 = P - P1 - P2): 8, 16 or all 24 bits of their mantissa.  With three the
 // heads are 9e-8 to 3.4e-7 of their norm from float64 before their last rounding, on CUDA cores in float32 1.3e-7 to 5.9e-7 (with two
 // 6.5e-7 to 2.2e-6); 64 tokens of 32 heads at 2,000 keys 105.5 -> 109.6 us for it, one token of 32 heads as before.
+// DIFF: differential attention.  A query row holds [q_1, q_2], a key row [k_1, k_2]; row 2 h + m of a block's products is map m of
+// query head h, so that one walk over the keys serves both maps.  nh counts maps.
 struct RdExtras {
     const float* sinks;
     const float* gate;
@@ -166,9 +168,6 @@ struct RdExtras {
     // alias > 1: every KV head of the cache is walked by so many blocks side by side, each for its own share of the head's query
     // heads (a group beyond the 16 rows of a block's products; the rows come from L2 from the second on).  0 counts as 1.
     int alias;
-    // diff: differential attention.  A query row holds [q_1, q_2], a key row [k_1, k_2]; row 2 h + m of a block's products is map m
-    // of query head h, the other half of its channels zero, so that one walk over the keys serves both maps.  nh counts maps.
-    int diff;
 };
 
 // num / den of a head with the sink's term added (m and the sink in units of log2) and the gate applied
@@ -188,7 +187,7 @@ __device__ __forceinline__ float rd_finish(float num, float den, float m, const 
     return r;
 }
 
-template <int D, bool FUSE, int TERMS>
+template <int D, bool FUSE, int TERMS, bool DIFF>
 __global__ void __launch_bounds__(RD_THREADS + 32)
 attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                              const __grid_constant__ CUtensorMap map_k16, const __grid_constant__ CUtensorMap map_v16,
@@ -344,7 +343,7 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
             store8(Qs + rd_qswz<D>(r, c), f);
         } else {
             uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (!FUSE && ex.diff) {
+            if (DIFF) {
                 if (r < G && (c >= CH / 2) == ((r & 1) != 0)) v = *reinterpret_cast<const uint4*>(q + (size_t)t * q_stride + (size_t)(hk * (G / 2) + (r >> 1)) * D + c * 8);
             } else if (r < G) {
                 v = *reinterpret_cast<const uint4*>(q + (size_t)t * q_stride + (size_t)(hk * G + r) * D + c * 8);
@@ -387,7 +386,8 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
         }
         if (key0 <= p && key0 + 15 >= lo) {
             const unsigned kbase = base + (unsigned)s * 2 * TILE_BYTES, vbase = kbase + TILE_BYTES;
-            // two accumulator sets shorten the chain of dependent MMAs
+            // two accumulator sets shorten the chain of dependent MMAs; with DIFF one for each map's channels, of which a row takes its
+            // own (its zeros for the other map's channels are not to meet an infinite key there)
             float sa[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
             float sb[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
             const int krow = warp * 16 + (mtx >> 1) * 8 + (lane & 7);
@@ -395,7 +395,7 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
             for (int ks = 0; ks < KS; ks++) {
                 unsigned b0, b1, b2, b3;
                 rd_ldm(b0, b1, b2, b3, kbase + rd_tile_off(krow, ks * 2 + (mtx & 1)));
-                if (ks & 1) {
+                if (DIFF ? ks >= KS / 2 : (ks & 1) != 0) {
                     rd_mma(sb[0], qf[ks], b0, b1);
                     rd_mma(sb[1], qf[ks], b2, b3);
                 } else {
@@ -410,7 +410,7 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
                     const int key = key0 + nt * 8 + t4 * 2 + (e & 1);
-                    float v = (sa[nt][e] + sb[nt][e]) * scale_log2e;
+                    float v = (!DIFF ? sa[nt][e] + sb[nt][e] : g & 1 ? sb[nt][e] : sa[nt][e]) * scale_log2e;
                     if (TERMS > 1 && ex.softcap > 0.f) v = 1.4426950408889634f * soft_cap_fast(sa[nt][e] + sb[nt][e], ex.softcap, ex.softcap_x);
                     if (key > p || key < lo) v = -INFINITY;
                     sc[nt][e] = v;
@@ -422,8 +422,9 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
                 mx[e] = fmaxf(mx[e], __shfl_xor_sync(0xffffffffu, mx[e], 1));
                 mx[e] = fmaxf(mx[e], __shfl_xor_sync(0xffffffffu, mx[e], 2));
                 const float m_new = fmaxf(m_run[e], mx[e]);      // finite: the warp has a valid key
-                mref[e] = m_new;
-                alpha[e] = fast_exp2(m_run[e] - m_new);          // 0 the first time (m_run = -inf)
+                // (or infinite keys, whose scores of minus infinity have weight 0 as on CUDA cores)
+                mref[e] = TERMS > 2 && m_new == -INFINITY ? 0.f : m_new;
+                alpha[e] = fast_exp2(m_run[e] - mref[e]);        // 0 the first time (m_run = -inf)
                 m_run[e] = m_new;
                 l_run[e] *= alpha[e];
             }
@@ -633,7 +634,7 @@ template <int D>
 static int rd_launch(const void* q, int q_stride, const void* kc, const void* vc, long long n_pages,
                      const int* block_table, int max_pages, const int* token_pos, const int* token_seq,
                      float* part_acc, float* part_ml, void* out, int T, int nh, int nkv, int page_size, int window,
-                     float scale, int n_splits, int* err, cudaStream_t s, const RdRope* rope, const RdExtras* extras, int terms) {
+                     float scale, int n_splits, int* err, cudaStream_t s, const RdRope* rope, const RdExtras* extras, int terms, bool diff) {
     CUtensorMap mk, mv, mk16, mv16;
     int rc;
     const long long rows = n_pages * nkv * page_size;
@@ -655,10 +656,15 @@ static int rd_launch(const void* q, int q_stride, const void* kc, const void* vc
                     nh / groups, page_size, window, scale * 1.4426950408889634f, err, rp, ex);
         return illm_launch_status();
     };
-    rc = rope         ? launch(attention_decode_ring_kernel<D, true, 1>)
-         : terms == 1 ? launch(attention_decode_ring_kernel<D, false, 1>)
-         : terms == 2 ? launch(attention_decode_ring_kernel<D, false, 2>)
-                      : launch(attention_decode_ring_kernel<D, false, 3>);
+    if (diff) {
+        if constexpr (D == 128) rc = launch(attention_decode_ring_kernel<D, false, 3, true>);
+        else return ILLM_ERR_BAD_ARG;
+    } else {
+        rc = rope         ? launch(attention_decode_ring_kernel<D, true, 1, false>)
+             : terms == 1 ? launch(attention_decode_ring_kernel<D, false, 1, false>)
+             : terms == 2 ? launch(attention_decode_ring_kernel<D, false, 2, false>)
+                          : launch(attention_decode_ring_kernel<D, false, 3, false>);
+    }
     if (rc != 0 || n_splits == 1 || !out) return rc;        // no out: the shares are the caller's to put together
     illm_launch(attention_decode_ring_merge_kernel<D>, dim3(nh, T), dim3(D), 0, s, (const float*)part_acc,
                 (const float*)part_ml, (bf16*)out, n_splits, nh, ex);
@@ -668,7 +674,7 @@ static int rd_launch(const void* q, int q_stride, const void* kc, const void* vc
 static int rd_run(const void* q, int q_stride, const void* kc, const void* vc, long long n_pages,
                   const int* block_table, int max_pages, const int* token_pos, const int* token_seq, float* part_acc,
                   float* part_ml, void* out, int T, int nh, int nkv, int d, int page_size, int window, float scale,
-                  int n_splits, int* err, void* stream, const RdRope* rope, const RdExtras* extras = nullptr, int terms = 1) {
+                  int n_splits, int* err, void* stream, const RdRope* rope, const RdExtras* extras = nullptr, int terms = 1, bool diff = false) {
     if (T <= 0) return 0;
     const int alias = extras && extras->alias > 1 ? extras->alias : 1;
     if (nkv <= 0 || nh % (nkv * alias) || nh / (nkv * alias) > 16 || T > 65535 || nkv * alias > 65535 || (q_stride & 7) || page_size % RD_BN ||
@@ -679,10 +685,10 @@ static int rd_run(const void* q, int q_stride, const void* kc, const void* vc, l
     cudaStream_t s = (cudaStream_t)stream;
     if (d == 128)
         return rd_launch<128>(q, q_stride, kc, vc, n_pages, block_table, max_pages, token_pos, token_seq, part_acc,
-                              part_ml, out, T, nh, nkv, page_size, window, scale, n_splits, err, s, rope, extras, terms);
+                              part_ml, out, T, nh, nkv, page_size, window, scale, n_splits, err, s, rope, extras, terms, diff);
     if (d == 64)
         return rd_launch<64>(q, q_stride, kc, vc, n_pages, block_table, max_pages, token_pos, token_seq, part_acc,
-                             part_ml, out, T, nh, nkv, page_size, window, scale, n_splits, err, s, rope, extras, terms);
+                             part_ml, out, T, nh, nkv, page_size, window, scale, n_splits, err, s, rope, extras, terms, diff);
     return ILLM_ERR_BAD_ARG;
 }
 
@@ -723,7 +729,7 @@ extern "C" int illm_attention_decode_ring_shared(const void* q, int q_stride, co
                                                  int nh, int nkv, int d, int page_size, int window, float scale, int n_splits, int* err, int wide_p,
                                                  const float* sinks, const float* gate, int gate_stride, int gate_wide, float softcap, int alias, void* stream) {
     if (softcap > 0.f && !wide_p) return ILLM_ERR_BAD_ARG;
-    RdExtras ex{sinks, gate, gate_stride, gate_wide, softcap, softcap > 0.f ? 2.0f * scale * 1.4426950408889634f / softcap : 0.f, alias, 0};
+    RdExtras ex{sinks, gate, gate_stride, gate_wide, softcap, softcap > 0.f ? 2.0f * scale * 1.4426950408889634f / softcap : 0.f, alias};
     return rd_run(q, q_stride, kc, vc, n_pages, block_table, max_pages, token_pos, token_seq, part_acc, part_ml, out, T,
                   nh, nkv, d, page_size, window, scale, n_splits, err, stream, nullptr, &ex, !wide_p ? 1 : alias > 1 ? 3 : 2);
 }
@@ -781,9 +787,9 @@ extern "C" int illm_attention_diff_ring(const void* q, int q_stride, const void*
                                         int page_size, int window, float scale, int n_splits, float lambda, float eps, float out_scale, int* err, void* stream) {
     if (T <= 0) return 0;
     if (!illm_attention_diff_ring_supported(nh, nkv, d, dv, page_size) || !out) return ILLM_ERR_BAD_ARG;
-    RdExtras ex{nullptr, nullptr, 0, 0, 0.f, 0.f, 1, 1};
+    RdExtras ex{nullptr, nullptr, 0, 0, 0.f, 0.f, 1};
     const int rc = rd_run(q, q_stride, kc, vc, n_pages, block_table, max_pages, token_pos, token_seq, part_acc, part_ml, nullptr, T, 2 * nh, nkv, 128, page_size,
-                          window, scale, n_splits, err, stream, nullptr, &ex, 3);
+                          window, scale, n_splits, err, stream, nullptr, &ex, 3, true);
     if (rc) return rc;
     illm_launch(attention_diff_ring_merge_kernel<128>, dim3(nh, T), dim3(256), 0, (cudaStream_t)stream, (const float*)part_acc, (const float*)part_ml, (bf16*)out,
                 n_splits, nh, lambda, eps, out_scale);

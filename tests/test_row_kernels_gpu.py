@@ -450,6 +450,50 @@ def test_ring_attention_keeps_float32_weights(maps, sharp):
     assert ours <= theirs
 
 
+@pytest.mark.parametrize("maps", [1, 2])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_ring_attention_of_infinite_keys(maps, splits):
+    """A key with an infinite channel whose scores are minus infinity has weight 0 in its own map and the other map does not see it, among
+    other keys and as the only one of the last 16 (differential heads; a group of 32 heads)."""
+    nh, nkv, d, dv, page = 32, 4 if maps == 2 else 1, 64 if maps == 2 else 128, 128, 64
+    lens, far = [40, 65, 300, 300], [3, 64, 17, 299]
+    T, scale = len(lens), d ** -0.5
+    g = torch.Generator().manual_seed(maps)
+    q = torch.randn(T, nh, maps, d, generator=g).bfloat16()
+    q[:, :, maps - 1, 5] = -q[:, :, maps - 1, 5].abs() - 0.1
+    width = max(-(-n // page) for n in lens)
+    table = torch.arange(T * width, dtype=torch.int32).view(T, width)
+    ks, vs = [[torch.randn(n, nkv, w, generator=g).bfloat16() for n in lens] for w in (maps * d, dv)]
+    kc, vc = (torch.full((T * width, nkv, page, w), float("nan"), dtype=torch.bfloat16) for w in (maps * d, dv))
+    for b, n in enumerate(lens):
+        ks[b][far[b], :, (maps - 1) * d + 5] = float("inf")
+        for t in range(n):
+            kc[table[b, t // page], :, t % page], vc[table[b, t // page], :, t % page] = ks[b][t], vs[b][t]
+    dev = [t.cuda() for t in (q.reshape(T, -1), kc, vc, table, torch.tensor(lens, dtype=torch.int32) - 1, torch.arange(T, dtype=torch.int32))]
+    err, out = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.empty(T, nh * dv, dtype=torch.bfloat16, device="cuda")
+    acc, ml = torch.empty(T * nh * maps * splits * dv, device="cuda"), torch.empty(T * nh * maps * splits * 2, device="cuda")
+    lam, eps = 0.4, 1e-6
+    if maps == 2:
+        rc = entry("illm_attention_diff_ring", I_, P_, I_, P_, P_, L_, P_, I_, P_, P_, P_, P_, P_, I_, I_, I_, I_, I_, I_, I_, F_, I_, F_, F_, F_, P_, P_)(
+            p(dev[0]), nh * 2 * d, p(dev[1]), p(dev[2]), T * width, p(dev[3]), width, p(dev[4]), p(dev[5]), p(acc), p(ml), p(out), T, nh, nkv, d, dv, page, 0, scale,
+            splits, lam, eps, 1.0, p(err), stream())
+    else:
+        rc = entry("illm_attention_decode_ring_shared", I_, P_, I_, P_, P_, L_, P_, I_, P_, P_, P_, P_, P_, I_, I_, I_, I_, I_, I_, F_, I_, P_, I_, P_, P_, I_, I_, F_, I_,
+                   P_)(p(dev[0]), nh * d, p(dev[1]), p(dev[2]), T * width, p(dev[3]), width, p(dev[4]), p(dev[5]), p(acc), p(ml), p(out), T, nh, nkv, d, page, 0, scale,
+                       splits, p(err), 1, None, None, 0, 0, 0.0, 2, stream())
+    assert rc == 0 and int(err) == 0
+    got = out.cpu().double().numpy().reshape(T, nh, dv)
+    for b in range(T):
+        for h in range(nh):
+            k, v = ks[b][:, h // (nh // nkv)].double().numpy().reshape(-1, maps, d), vs[b][:, h // (nh // nkv)].double().numpy()
+            a = [(weights_of(q[b, h, m:m + 1].double().numpy(), k[:, m], scale, 0) @ v)[0] for m in range(maps)]
+            ref = a[0]
+            if maps == 2:
+                o = a[0] - lam * a[1]
+                ref = o / np.sqrt((o * o).mean() + eps)
+            assert (np.abs(got[b, h] - ref) <= 2.0 ** -8 * np.abs(ref) + 2.0 ** -12).all(), (b, h)
+
+
 @pytest.mark.parametrize("nh,nkv,alias,d", [(32, 1, 2, 128), (20, 1, 2, 64), (96, 2, 3, 64), (128, 1, 8, 128), (6, 2, 3, 128), (4, 4, 1, 64)])
 @pytest.mark.parametrize("window,cap,sinks", [(0, 0.0, False), (70, 20.0, True)])
 @pytest.mark.parametrize("splits", [1, 5])
