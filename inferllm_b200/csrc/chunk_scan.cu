@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(CS_THREADS, KIND == CHUNK_DELTA_HEAD ? 2 : 3) 
                     float m[CS_T], o = rec[2 * CS_T + j] * z;
                     eight(4 * CS_T + CS_T * CS_T + j * CS_T, m);
 #pragma unroll
-                    for (int i = 0; i < CS_T; i++) o = fmaf(m[i], v[i], o);      // zero behind j
+                    for (int i = 0; i < CS_T; i++) o = i <= j ? fmaf(m[i], v[i], o) : o;     // (a later token's infinite value stays out)
                     if (c0 + j < nt && j0 + col0 + cc < dv)
                         p.out[(size_t)(first + t0 + c0 + j) * p.nh * dv + (size_t)h * dv + j0 + col0 + cc] = o;
                 }

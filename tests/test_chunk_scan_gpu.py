@@ -64,6 +64,30 @@ def test_linear_attention(d, dv, nh, off, segments):
         assert (np.abs(state[s] - S) <= bound * M).all()
 
 
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("segments,at", [(1, 19), (1, 23), (1, 8), (2, 90)])
+def test_linear_attention_keeps_a_value_from_earlier_tokens(segments, at, bad):
+    """A value that is no finite number at token `at` leaves the bits of all tokens before it as they are."""
+    d, dv, nh, n = 64, 64, 2, 131
+    g = torch.Generator().manual_seed(at)
+    x, C = torch.randn(n, nh * (2 * d + dv), generator=g), nh * (2 * d + dv)
+    ints = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")  # noqa: E731
+    outs = []
+    for planted in (False, True):
+        xd, out, Sd = x.cuda(), torch.full((n, nh * dv), 7.0, device="cuda"), torch.zeros(1, nh, dv, d, device="cuda")
+        if planted:
+            xd[at, 2 * nh * d:] = bad
+        size = entry("illm_decay_chunk_scratch", L_, I_, I_, I_, I_, I_, I_)(n, 1, nh, d, dv, segments)
+        rec, err, decay = torch.empty(size, device="cuda"), ints([0]), torch.tensor([0.9, 0.99], device="cuda")
+        zero, cu, pos = ints([0]), ints([0, n]), ints(list(range(n)))
+        rc = entry("illm_decay_chunk_scan", I_, P_, I_, I_, I_, I_, I_, I_, I_, I_, I_, I_, P_, I_, I_, F_, P_, P_, P_, P_, P_, P_, I_, I_, I_, P_, P_, P_)(
+            p(xd), n, C, 0, nh * d, 2 * nh * d, nh, d, dv, 0, 0, None, 0, 0, 1.0, p(decay), p(Sd), p(zero), p(cu), p(pos), p(out), 1, n, segments, p(err), p(rec),
+            torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        outs.append(out.cpu())
+    assert torch.equal(outs[0][:at], outs[1][:at]) and not torch.isfinite(outs[1][at]).any()
+
+
 @pytest.mark.parametrize("head_decay", [0, 1])
 @pytest.mark.parametrize("d,dv,nh,nkv", [(128, 128, 4, 2), (128, 64, 1, 1), (20, 130, 2, 2), (9, 7, 3, 1), (100, 65, 2, 1)])
 @pytest.mark.parametrize("strong", [False, True])
