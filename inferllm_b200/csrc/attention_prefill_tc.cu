@@ -218,7 +218,7 @@ static FtCap ft_make_cap(float softcap, float scale) {
 // then works on capped scores in units of log2 and its scale is 1.
 // DK: score channels, D but for the differential form (DIFF): there head h has two score maps of DK channels over the same
 // values, its query row holds [q_1, q_2] and a key row [k_1, k_2]; a block takes one (head, map), reads the map's columns of
-// both, and leaves the map's output in float32, rows of nh x 2 x D, for attention_diff_combine_kernel.
+// both, and leaves the map's output in float32, rows of gridDim.x x D (the maps from map0 on), for attention_diff_combine_kernel.
 template <int D, int DK, bool WIDE_P, bool CAP, bool DIFF>
 __global__ void __launch_bounds__(FT_THREADS, 2)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -226,7 +226,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             int max_pages, const int* __restrict__ cu_q, const int* __restrict__ seq_lens,
                             void* __restrict__ out, int nh, int nkv, int page_size, int span,
                             float scale_log2e, int* __restrict__ err, const float* __restrict__ sinks,
-                            const float* __restrict__ gate, int gate_stride, int gate_wide, const FtCap cap) {
+                            const float* __restrict__ gate, int gate_stride, int gate_wide, const FtCap cap, int map0) {
     constexpr int FT_MMA_WARP = 4, FT_TMA_WARP = 5;
     constexpr int NA = DK / 64, NV = D / 64;              // 64-channel atoms of the keys and of the values
     constexpr unsigned Q_TILE = FT_BM * DK * 2;           // the query tile: [NA][128 rows][128 B]
@@ -290,7 +290,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     // end and the x-th from the start, which gives all blocks equal work, was slower at every prompt
     // length: 52.5 against 50.2 us at 2,048 tokens of 32 heads, 138 against 101 us at 3,072.)  With chunks the work of a
     // tile grows with its place inside its chunk, and the tiles of all chunks are taken in the order of that place.
-    const int b = blockIdx.z, h = DIFF ? blockIdx.x >> 1 : blockIdx.x, map = DIFF ? blockIdx.x & 1 : 0;
+    const int b = blockIdx.z, hm = blockIdx.x + (DIFF ? map0 : 0), h = DIFF ? hm >> 1 : hm, map = DIFF ? hm & 1 : 0;
     const int q0 = cu_q[b], qlen = cu_q[b + 1] - q0;
     const int n_tiles = (qlen + FT_BM - 1) / FT_BM;
     int tile = n_tiles - 1 - (int)blockIdx.y;                 // < 0: this sequence is shorter than the longest
@@ -320,7 +320,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         // block i-2 has; the loop asks in the order in which those come true.
         if (lane == 0 && has_rows) {
             bar_expect_tx(q_full, Q_TILE);
-            for (int a = 0; a < NA; a++) tma_2d(q_s + a * Q_ATOM, &map_q, (int)blockIdx.x * DK + 64 * a, q0 + row0, q_full);
+            for (int a = 0; a < NA; a++) tma_2d(q_s + a * Q_ATOM, &map_q, hm * DK + 64 * a, q0 + row0, q_full);
             auto kv_row = [&](int i) {
                 const int key0 = (jb0 + i) * FT_BN;
                 return (bt[key0 / page_size] * nkv + hk) * page_size + (key0 % page_size);
@@ -557,7 +557,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             }
             if (gate && !gate_wide && r < rows) inv *= 1.0f / (1.0f + expf(-gate[(size_t)(q0 + row0 + r) * gate_stride + h]));
             bf16* dst = (bf16*)out + ((size_t)(q0 + row0 + r) * nh + h) * D;
-            float* dst_map = (float*)out + ((size_t)(q0 + row0 + r) * 2 * nh + blockIdx.x) * D;      // DIFF
+            float* dst_map = (float*)out + ((size_t)(q0 + row0 + r) * gridDim.x + blockIdx.x) * D;      // DIFF
             // a gate per channel: a warp brings its 32 rows, whole rows at a time, into the shared memory that the tiles of
             // Q and K no longer need (every product has been done), from where a thread reads its own row
             constexpr int G_ROW = D * 4 + 16;
@@ -654,7 +654,7 @@ template <int D, bool WIDE_P, bool CAP, int DK = D, bool DIFF = false>
 static int ft_launch(const void* q, int q_stride, int T, const void* kc, const void* vc, long long n_pages,
                      const int* block_table, int max_pages, const int* cu_q, const int* seq_lens, void* out, int B,
                      int max_q, int nh, int nkv, int page_size, int span, float scale, int* err, const float* sinks,
-                     const float* gate, int gate_stride, int gate_wide, float softcap, cudaStream_t s) {
+                     const float* gate, int gate_stride, int gate_wide, float softcap, cudaStream_t s, int head0 = 0, int heads = 0) {
     CUtensorMap mq, mk, mv;
     int rc;
     if ((rc = ft_make_map(&mq, q, T, (long long)nh * (DIFF ? 2 : 1) * DK, q_stride, FT_BM)) != 0) return rc;
@@ -666,10 +666,10 @@ static int ft_launch(const void* q, int q_stride, int T, const void* kc, const v
     auto kern = attention_prefill_tc_kernel<D, DK, WIDE_P, CAP, DIFF>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    dim3 grid(DIFF ? 2 * nh : nh, (max_q + FT_BM - 1) / FT_BM, B);
+    dim3 grid(DIFF ? 2 * heads : nh, (max_q + FT_BM - 1) / FT_BM, B);
     illm_launch(kern, grid, dim3(FT_THREADS), smem, s, mq, mk, mv, block_table, max_pages, cu_q, seq_lens,
                 out, nh, nkv, page_size, span, CAP ? 1.0f : scale * 1.4426950408889634f, err, sinks, gate, gate_stride, gate_wide,
-                CAP ? ft_make_cap(softcap, scale) : FtCap{});
+                CAP ? ft_make_cap(softcap, scale) : FtCap{}, 2 * head0);
     return illm_launch_status();
 }
 
@@ -710,14 +710,14 @@ extern "C" int illm_attention_prefill_tc(const void* q, int q_stride, int T, con
 }
 
 // o = a_1 - lambda a_2 of every (token, head), the head's unit norm over its D values and the factor: a warp per head, a lane per
-// four channels.  maps: float32 [T, nh, 2, D].
+// four channels.  maps: float32 [T, heads, 2, D], the step's heads head0 .. head0 + heads - 1 of nh.
 template <int D>
-__global__ void __launch_bounds__(256) attention_diff_combine_kernel(const float* __restrict__ maps, bf16* __restrict__ out, long long heads, float lambda,
-                                                                     float eps, float out_scale) {
+__global__ void __launch_bounds__(256) attention_diff_combine_kernel(const float* __restrict__ maps, bf16* __restrict__ out, long long T, int head0, int heads,
+                                                                     int nh, float lambda, float eps, float out_scale) {
     pdl_grid_sync();
     const long long i = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int c = (threadIdx.x & 31) * 4;
-    if (i >= heads) return;
+    if (i >= T * heads) return;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 a = c < D ? *reinterpret_cast<const float4*>(maps + i * 2 * D + c) : zero, b = c < D ? *reinterpret_cast<const float4*>(maps + (i * 2 + 1) * D + c) : zero;
     const float4 o = make_float4(fmaf(-lambda, b.x, a.x), fmaf(-lambda, b.y, a.y), fmaf(-lambda, b.z, a.z), fmaf(-lambda, b.w, a.w));
@@ -725,29 +725,47 @@ __global__ void __launch_bounds__(256) attention_diff_combine_kernel(const float
     const float f = out_scale / sqrtf(ss / (float)D + eps);
     if (c >= D) return;
     const __nv_bfloat162 lo = __floats2bfloat162_rn(o.x * f, o.y * f), hi = __floats2bfloat162_rn(o.z * f, o.w * f);
-    *reinterpret_cast<uint2*>(out + i * D + c) = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
+    const long long t = i / heads, h = head0 + i - t * heads;
+    *reinterpret_cast<uint2*>(out + (t * nh + h) * D + c) = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
 }
 
 // Differential attention of prompts (two score maps of 64 channels over values of 128): q [T, q_stride] with head h's
-// [q_1, q_2] at column h * 128, pages of key rows [k_1, k_2] and value rows; maps: scratch, float32 [T, nh, 2, dv]; window: see
+// [q_1, q_2] at column h * 128, pages of key rows [k_1, k_2] and value rows; maps: scratch, float32 [T, heads, 2, dv]; window: see
 // first_visible.  A map is one pass of the kernel above over its own columns, so the two maps run side by side on
 // tensor memory; the warp-level MMA kernel of attention_maps.cu, which holds both maps' outputs in registers, took 622 us for
 // 1,777 tokens of 32 heads.
+// The scratch holds `heads` heads, which are taken together; illm_attention_diff_tc_heads: as many as 128 MiB hold (at 32 heads up
+// to 4,096 tokens all of them), at least one.  A pass over fewer heads still has 2 x heads x T / 128 blocks, several per SM from there on, and what
+// it leaves is read back while L2 holds most of it.
 extern "C" int illm_attention_diff_tc_supported(int nh, int nkv, int d, int dv, int page_size) {
     return d == 64 && dv == 128 && page_size > 0 && page_size % 64 == 0 && nkv > 0 && nh % nkv == 0 && nh <= 32767;
+}
+extern "C" int illm_attention_diff_tc_heads(long long T, int nh, int dv) {
+    const long long n = (128LL << 20) / (T * 2 * dv * 4);
+    return (int)(n < 1 ? 1 : n > nh ? nh : n);
+}
+extern "C" int illm_attention_diff_tc_sliced(const void* q, int q_stride, int T, const void* kc, const void* vc, long long n_pages, const int* block_table,
+                                             int max_pages, const int* cu_q, const int* seq_lens, float* maps, void* out, int B, int max_q, int nh, int nkv,
+                                             int d, int dv, int page_size, int window, float scale, float lambda, float eps, float out_scale, int heads, int* err,
+                                             void* stream) {
+    if (B <= 0 || max_q <= 0 || T <= 0) return 0;
+    if (!illm_attention_diff_tc_supported(nh, nkv, d, dv, page_size) || heads < 1 || max_q > 65535 * FT_BM || B > 65535 || (q_stride & 7) || !maps ||
+        ((uintptr_t)q & 15) || ((uintptr_t)kc & 15) || ((uintptr_t)vc & 15) || ((uintptr_t)maps & 15) || ((uintptr_t)out & 15))
+        return ILLM_ERR_BAD_ARG;
+    cudaStream_t s = (cudaStream_t)stream;
+    for (int h0 = 0; h0 < nh; h0 += heads) {
+        const int n = nh - h0 < heads ? nh - h0 : heads;
+        const int rc = ft_launch<128, true, false, 64, true>(q, q_stride, T, kc, vc, n_pages, block_table, max_pages, cu_q, seq_lens, maps, B, max_q, nh, nkv,
+                                                             page_size, window, scale, err, nullptr, nullptr, 0, 0, 0.f, s, h0, n);
+        if (rc) return rc;
+        illm_launch(attention_diff_combine_kernel<128>, dim3((unsigned)(((long long)T * n + 7) / 8)), dim3(256), 0, s, maps, (bf16*)out, (long long)T, h0, n, nh, lambda,
+                    eps, out_scale);
+    }
+    return illm_launch_status();
 }
 extern "C" int illm_attention_diff_tc(const void* q, int q_stride, int T, const void* kc, const void* vc, long long n_pages, const int* block_table,
                                       int max_pages, const int* cu_q, const int* seq_lens, float* maps, void* out, int B, int max_q, int nh, int nkv, int d,
                                       int dv, int page_size, int window, float scale, float lambda, float eps, float out_scale, int* err, void* stream) {
-    if (B <= 0 || max_q <= 0 || T <= 0) return 0;
-    if (!illm_attention_diff_tc_supported(nh, nkv, d, dv, page_size) || max_q > 65535 * FT_BM || B > 65535 || (q_stride & 7) || !maps || ((uintptr_t)q & 15) ||
-        ((uintptr_t)kc & 15) || ((uintptr_t)vc & 15) || ((uintptr_t)maps & 15) || ((uintptr_t)out & 15))
-        return ILLM_ERR_BAD_ARG;
-    cudaStream_t s = (cudaStream_t)stream;
-    const int rc = ft_launch<128, true, false, 64, true>(q, q_stride, T, kc, vc, n_pages, block_table, max_pages, cu_q, seq_lens, maps, B, max_q, nh, nkv,
-                                                         page_size, window, scale, err, nullptr, nullptr, 0, 0, 0.f, s);
-    if (rc) return rc;
-    const long long heads = (long long)T * nh;
-    illm_launch(attention_diff_combine_kernel<128>, dim3((unsigned)((heads + 7) / 8)), dim3(256), 0, s, maps, (bf16*)out, heads, lambda, eps, out_scale);
-    return illm_launch_status();
+    return illm_attention_diff_tc_sliced(q, q_stride, T, kc, vc, n_pages, block_table, max_pages, cu_q, seq_lens, maps, out, B, max_q, nh, nkv, d, dv, page_size,
+                                         window, scale, lambda, eps, out_scale, nh > 0 ? nh : 1, err, stream);
 }

@@ -166,6 +166,8 @@ long long illm_attention_diff_scratch(int T, int nh, int dv, int splits);
 int illm_attention_diff_tc_supported(int nh, int nkv, int d, int dv, int page_size);
 int illm_attention_diff_tc(const void* q, int q_stride, int T, const void* kc, const void* vc, long long n_pages, const int* block_table, int max_pages, const int* cu_q, const int* seq_lens, float* maps, void* out, int B, int max_q, int nh, int nkv, int d, int dv, int page_size, int window, float scale, float lambda, float eps, float out_scale, int* err, void* stream);
 int illm_attention_diff_mma_supported(int d, int dv);
+int illm_attention_diff_tc_heads(long long T, int nh, int dv);
+int illm_attention_diff_tc_sliced(const void* q, int q_stride, int T, const void* kc, const void* vc, long long n_pages, const int* block_table, int max_pages, const int* cu_q, const int* seq_lens, float* maps, void* out, int B, int max_q, int nh, int nkv, int d, int dv, int page_size, int window, float scale, float lambda, float eps, float out_scale, int heads, int* err, void* stream);
 int illm_attention_diff_decode_supported(int nh, int nkv, int d, int dv);
 int illm_attention_diff_decode(const void* q, int q_stride, const void* kc, const void* vc, const int* block_table, int max_pages, const int* token_pos, const int* token_seq, void* out, int T, int nh, int nkv, int d, int dv, int page_size, int window, float scale, float lambda, float eps, float out_scale, long long max_len, int splits, float* scratch, void* stream);
 int illm_attention_diff_mma(const void* q, int q_stride, const void* kc, const void* vc, const int* block_table, int max_pages, const int* cu_q, const int* seq_lens, void* out, int B, int max_q, int nh, int nkv, int d, int dv, int page_size, int window, float scale, float lambda, float eps, float out_scale, void* stream);

@@ -887,10 +887,11 @@ Mat attention_diff(Device& dev, const Mat& q, const KVView& kv, const StepView& 
         throw KernelError("attention_diff: the cache entry must hold key rows of two maps (2 x " + std::to_string(g.head_dim) + " channels) in the queries' dtype");
     Mat out = new_mat(dev, q.rows, (long long)g.n_heads * dv, q.dtype);
     if (q.dtype == DType::BF16 && !ctx.is_decode && q.cols % 8 == 0 && illm_attention_diff_tc_supported(g.n_heads, g.n_kv_heads, g.head_dim, dv, kv.page_size)) {
-        float* maps = dev.alloc_n<float>((size_t)q.rows * g.n_heads * 2 * dv);
-        check_kernel(illm_attention_diff_tc(q.p, (int)q.cols, (int)q.rows, kv.k, kv.v, kv.num_pages, kv.block_table, kv.width, ctx.cu_q, ctx.seq_lens, maps, out.p,
+        const int heads = illm_attention_diff_tc_heads(q.rows, g.n_heads, dv);
+        float* maps = dev.alloc_n<float>((size_t)q.rows * heads * 2 * dv);
+        check_kernel(illm_attention_diff_tc_sliced(q.p, (int)q.cols, (int)q.rows, kv.k, kv.v, kv.num_pages, kv.block_table, kv.width, ctx.cu_q, ctx.seq_lens, maps, out.p,
                                             ctx.B, ctx.max_q, g.n_heads, g.n_kv_heads, g.head_dim, dv, kv.page_size, kv.window, scale, p.lambda, p.eps, p.out_scale,
-                                            dev.tc_error_word(), dev.stream()),
+                                            heads, dev.tc_error_word(), dev.stream()),
                      "attention_diff_tc");
         return out;
     }

@@ -296,6 +296,34 @@ def test_differential_attention_on_tensor_memory(nh, nkv, window, lens):
         assert np.linalg.norm(mine) <= 1.5 * np.linalg.norm(theirs) + 1e-6
 
 
+@pytest.mark.parametrize("heads", [1, 2, 5])
+def test_differential_attention_in_passes_over_heads(heads):
+    """Any number of heads per pass gives the bits of one pass over all, and a pass's scratch is bounded."""
+    nh, nkv, d, dv, page, lens = 6, 2, 64, 128, 64, [5, 200, 64]
+    g = torch.Generator().manual_seed(heads)
+    _, pools, table = paged(lens, nkv, (2 * d, dv), g)
+    T, B, width, n_pages = sum(lens), len(lens), table.shape[1], pools[0].shape[0]
+    q = torch.randn(T, nh * 2 * d, generator=g).bfloat16()
+    cu = torch.tensor([0] + list(np.cumsum(lens)), dtype=torch.int32)
+    dev = [t.cuda() for t in (q, *pools, table, cu, torch.tensor(lens, dtype=torch.int32))]
+    err, outs = torch.zeros(1, dtype=torch.int32, device="cuda"), []
+    for n in (nh, heads):
+        guard = 64
+        maps = torch.full((T * n * 2 * dv + guard,), -7.0, device="cuda")
+        out = torch.full((T, nh * dv), float("nan"), dtype=torch.bfloat16, device="cuda")
+        rc = entry("illm_attention_diff_tc_sliced", I_, P_, I_, I_, P_, P_, L_, P_, I_, P_, P_, P_, P_, I_, I_, I_, I_, I_, I_, I_, I_, F_, F_, F_, F_, I_, P_, P_)(
+            p(dev[0]), nh * 2 * d, T, p(dev[1]), p(dev[2]), n_pages, p(dev[3]), width, p(dev[4]), p(dev[5]), p(maps), p(out), B, max(lens), nh, nkv, d, dv, page, 0,
+            d ** -0.5, 0.45, 1e-6, 0.6, n, p(err), stream())
+        assert rc == 0 and (maps[-guard:] == -7.0).all()
+        outs.append(out.cpu())
+    assert int(err) == 0 and torch.isfinite(outs[0].float()).all() and torch.equal(outs[0], outs[1])
+    per_pass = entry("illm_attention_diff_tc_heads", I_, L_, I_, I_)
+    for T in (1, 1777, 4096, 16384, 65536, 1 << 20):
+        n = per_pass(T, 32, dv)
+        assert 1 <= n <= 32 and (n == 1 or n * T * 2 * dv * 4 <= 128 << 20)
+    assert per_pass(4096, 32, dv) == 32
+
+
 @pytest.mark.parametrize("H", [4, 516, 4096, 4100, 16384])
 @pytest.mark.parametrize("n1,n2", [(1, 1), (3, 1), (9, 2), (17, 0)])
 def test_addends_as_slices(H, n1, n2):
