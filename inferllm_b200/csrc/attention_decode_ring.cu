@@ -555,7 +555,7 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k, const __
 __device__ __forceinline__ float rd_share_weights(const float* __restrict__ part_ml, size_t o, int n_splits, float& w, float& l) {
     const int lane = threadIdx.x & 31;
     float2 ml = make_float2(-INFINITY, 0.f);
-    if (lane < n_splits) ml = *reinterpret_cast<const float2*>(part_ml + (o + lane) * 2);
+    if (lane < n_splits) ml = make_float2(part_ml[(o + lane) * 2], part_ml[(o + lane) * 2 + 1]);      // (any address)
     float M = ml.x;
 #pragma unroll
     for (int k = 16; k; k >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, k));

@@ -424,6 +424,25 @@ def test_differential_attention_of_single_tokens(nh, nkv, window, lens, splits):
     assert np.linalg.norm(mine) <= 1.01 * np.linalg.norm(theirs) + 1e-6
 
 
+def test_merge_of_shares_at_any_address():
+    """The shares' words need no more than a float's alignment: the same bits from scratch that starts one float further on."""
+    nh, d, dv, splits, lens = 4, 64, 128, 3, [300, 65]
+    g = torch.Generator().manual_seed(3)
+    _, pools, table = paged(lens, 1, (2 * d, dv), g)
+    T, outs = len(lens), []
+    dev = [t.cuda() for t in (torch.randn(T, nh * 2 * d, generator=g).bfloat16(), *pools, table, torch.tensor(lens, dtype=torch.int32) - 1, torch.arange(T, dtype=torch.int32))]
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for off in (0, 1):
+        acc, ml = (torch.empty(T * nh * 2 * splits * w + off, device="cuda")[off:] for w in (dv, 2))
+        out = torch.full((T, nh * dv), float("nan"), dtype=torch.bfloat16, device="cuda")
+        rc = entry("illm_attention_diff_ring", I_, P_, I_, P_, P_, L_, P_, I_, P_, P_, P_, P_, P_, I_, I_, I_, I_, I_, I_, I_, F_, I_, F_, F_, F_, P_, P_)(
+            p(dev[0]), nh * 2 * d, p(dev[1]), p(dev[2]), pools[0].shape[0], p(dev[3]), table.shape[1], p(dev[4]), p(dev[5]), p(acc), p(ml), p(out), T, nh, 1, d, dv, 64,
+            0, d ** -0.5, splits, 0.45, 1e-6, 0.6, p(err), stream())
+        assert rc == 0 and int(err) == 0
+        outs.append(out.cpu())
+    assert torch.isfinite(outs[0].float()).all() and torch.equal(*outs)
+
+
 def shares(acc, ml, base2):
     """(acc, maximum, sum) of a head's shares put together in float64; base2: the maxima are in units of log2."""
     m, l = ml[..., 0].double(), ml[..., 1].double()
