@@ -320,8 +320,9 @@ int SequenceCache::alloc_slot() {
     seq_len[slot] = 0;
     if (device_)
         for (StateGroup& g : states) {
-            // the slot's rows of all the group's entries in one call where the pitch allows (a call per layer and sequence was a
-            // tenth of a prompt step of 32 sequences)
+            // the slot's rows of all the group's entries in one call where the pitch allows, instead of one per layer (32 instead of
+            // 128 calls for 32 sequences of four layers; the 2.5 ms for which the device waits before such a step are not theirs, they
+            // are the token ids' way through Python)
             const size_t row = (size_t)g.request.elements() * dtype_size(g.request.dtype), n = g.entries.size();
             char* first = (char*)g.state + (size_t)slot * row;
             if (n > 1 && g.entry_bytes <= (size_t)0x7fffffff) {

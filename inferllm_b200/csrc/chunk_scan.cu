@@ -585,7 +585,7 @@ static int cs_launch(const ChunkScanArgs& a, int B, int max_q, cudaStream_t s) {
     auto kern = chunk_scan_kernel<KIND>;
     const int P = KIND == CHUNK_LINEAR ? a.segments : 1;
     const dim3 grid((a.dv + CS_COLS - 1) / CS_COLS, a.nh, B * P);
-    // A grid that fits the SMs once asks for the shared memory of a whole SM: launched behind kernels that still hold most SMs, its
+    // A grid that fits the SMs once asks for more than half an SM's shared memory: launched behind kernels that still hold most SMs, its
     // blocks would otherwise be packed by threes onto those that are free first, and the slowest would decide.
     const size_t need = CsBuf<KIND>::BYTES, spread = (size_t)120 * 1024;
     const size_t smem = (long long)grid.x * grid.y * grid.z <= illm_sm_count() ? spread : need;

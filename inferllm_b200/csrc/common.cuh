@@ -98,7 +98,7 @@ __device__ __forceinline__ float fast_exp2(float x) {
     return y;
 }
 
-// Programmatic dependent launch.  Every kernel of the package starts with pdl_grid_sync(): it
+// Programmatic dependent launch.  The kernels of the package start with pdl_grid_sync(): it
 // lets the kernel after it in the stream begin to launch, then waits until the kernels before
 // it have finished and their writes are visible.  With the launch attribute below, a kernel's
 // blocks are therefore scheduled and set up (shared memory, barriers, and in the matrix product
@@ -106,6 +106,10 @@ __device__ __forceinline__ float fast_exp2(float x) {
 // between the many short kernels of a decode step.  A kernel still touches no activation before
 // its own wait, and a kernel's wait covers everything before it in the stream, so the order of
 // reads and writes is the stream's.  Without the attribute both instructions do nothing.
+// Some kernels issue the two instructions by themselves and read what no kernel writes before the wait: weights (the product
+// kernels, the row kernels of norms, sums and q/k/v), and the step's positions, sequences and page table (the q/k/v preparation,
+// the ring kernel with the fused rotation), which the engine brings with a copy.  A caller of the raw entry points that makes
+// one of those with a kernel puts something between the two that is no such launch, or waits for that kernel.
 __device__ __forceinline__ void pdl_grid_sync() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");

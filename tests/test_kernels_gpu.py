@@ -163,7 +163,8 @@ def test_gemm_f32_is_true_float32_and_row_invariant():
 
 @pytest.mark.parametrize("M,N,K", [(65, 15361, 36), (128, 15360, 16), (512, 12289, 20), (257, 38000, 16), (130, 4096, 24), (300, 5124, 35), (257, 8196, 17), (33, 7700, 20), (64, 7681, 48), (12, 130, 100)])
 def test_gemm_f32_tiles(M, N, K):
-    """Edges of the four tile sizes (128 x 128, 64 x 128, 64 x 64, 32 x 64), whose choice follows from M and N: against float64 (K products and
+    """Edges of the three tile sizes, whose choice follows from M and N (on 148 SMs the first three cases are taken by 128 x 128, the
+    next six by 64 x 64, the last by 32 x 64): against float64 (K products and
     sums, each rounded: K 2^-24 of the sum of magnitudes at most), and rows bit for bit what the row alone gives."""
     g = torch.Generator().manual_seed(M + N + K)
     x, w = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g)
