@@ -770,7 +770,10 @@ __global__ void __launch_bounds__(DL_THREADS) delta_chunk_scan_kernel(DeltaArgs 
 }
 
 // floats of scratch for the chunks' records of a step
-extern "C" long long illm_delta_chunk_scratch(int T, int B, int nh) { return ((long long)T / DC + B + 1) * nh * DC_REC; }
+extern "C" long long illm_delta_chunk_scratch(int T, int B, int nh) {
+    const long long mine = ((long long)T / DC + B + 1) * nh * DC_REC, shared = chunk_scan_scratch(T, B, nh);      // (whichever kernel runs)
+    return mine > shared ? mine : shared;
+}
 
 extern "C" int illm_delta_rule_supported(int d, int dv, int taps) { return d >= 1 && d <= 16 * DL_ROWS && dv >= 1 && taps >= 1 && taps <= 64; }
 
