@@ -156,3 +156,57 @@ def test_delta_rule(head_decay, d, dv, nh, nkv, strong):
             floor = 2.0 ** -24 * np.linalg.norm(ref)
             assert np.linalg.norm(mine - ref) <= 2 * np.linalg.norm(token - ref) + 4 * floor
         assert np.array_equal(chunked[1][s, nh * d * dv:], S[s, nh * d * dv:])       # the convolution's rows
+
+
+@pytest.mark.parametrize("taps,d,dv,nh,nkv", [(4, 128, 64, 2, 1), (3, 16, 20, 3, 3), (2, 4, 4, 2, 2)])
+@pytest.mark.parametrize("head_decay", [0, 1])
+def test_delta_preparation_of_many_tokens(taps, d, dv, nh, nkv, head_decay):
+    """A step of 512 tokens and more, which the preparation takes by eights of rows: sequences that meet inside an eight, some of them behind
+    a past whose convolution rows lie in the state.  The bits are those of each sequence in a step of its own (one row at a time),
+    and q, k, v, decays and write strengths those of float64."""
+    lens, past = [1, 2, 3, 5, 130, 7, 201, 9, 166, 1], [0, 2, 1, 0, 5, 0, 1, 9, 0, 3]
+    g = torch.Generator().manual_seed(taps * d + head_decay)
+    T, B, C = sum(lens), len(lens), 2 * nkv * d + nh * dv
+    assert T >= 512 and T % 8
+    ld, na, elems = (C + nh + 3) // 4 * 4, nh if head_decay else nh * d, nh * d * dv + (taps - 1) * C
+    x, a = torch.randn(T, ld, generator=g), torch.randn(T, na, generator=g)
+    conv = [torch.randn(w, taps, generator=g) for w in (nkv * d, nkv * d, nh * dv)]
+    a_log, dt, S0 = torch.randn(nh, generator=g) * 0.5, torch.randn(na, generator=g), torch.randn(B, elems, generator=g)
+    f = entry("illm_delta_rule", I_, P_, I_, I_, I_, I_, I_, I_, P_, I_, I_, I_, I_, I_, I_, I_, P_, P_, P_, P_, P_, F_, P_, L_, P_, P_, P_, P_, P_, P_, P_, P_, P_, I_,
+              I_, P_, P_)
+    weights = [t.cuda() for t in (*conv, a_log, dt)]
+    ints = lambda v: torch.tensor(list(v), dtype=torch.int32, device="cuda")  # noqa: E731
+
+    def run(seqs, rows):
+        n = [lens[b] for b in seqs]
+        xd, ad, S = x[rows].cuda(), a[rows].cuda(), S0.cuda()
+        cu, pos = ints([0, *np.cumsum(n)]), ints(past[b] + i for b in seqs for i in range(lens[b]))
+        seq, slots, total = ints(i for i, b in enumerate(seqs) for _ in range(lens[b])), ints(seqs), ints(past[b] + lens[b] for b in seqs)
+        outs = [torch.full((sum(n), w), float("nan"), device="cuda") for w in (C, na, nh, nh * dv)]
+        rc = f(p(xd), sum(n), ld, 0, nkv * d, 2 * nkv * d, C, p(ad), na, head_decay, nh, nkv, d, dv, taps, *(p(t) for t in weights), d ** -0.5, p(S), elems, p(slots),
+               p(cu), p(pos), p(seq), p(total), *(p(t) for t in outs), len(n), max(n), None, torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        return [t.cpu() for t in (*outs, S)]
+
+    whole, cu = run(range(B), slice(0, T)), [0, *np.cumsum(lens)]
+    sig = lambda z: 1.0 / (1.0 + np.exp(-z))  # noqa: E731
+    taps_all = np.concatenate([c.double().numpy() for c in conv])
+    for b in range(B):
+        rows = slice(int(cu[b]), int(cu[b + 1]))
+        one = run([b], rows)
+        for mine, alone in zip(whole[:4], one[:4]):
+            assert torch.equal(mine[rows], alone)
+        assert torch.equal(whole[4][b], one[4][b])
+        raw = np.concatenate([S0[b, nh * d * dv:].double().numpy().reshape(taps - 1, C), x[rows, :C].double().numpy()])
+        raw[:max(0, taps - 1 - past[b])] = 0.0                 # positions before the sequence's start
+        y = sum(raw[j:j + lens[b]] * taps_all[:, j] for j in range(taps))
+        y = y * sig(y)
+        for lo in range(0, 2 * nkv * d, d):
+            head = y[:, lo:lo + d]
+            y[:, lo:lo + d] = head / np.sqrt((head * head).sum(-1, keepdims=True) + 1e-6) * (d ** -0.5 if lo < nkv * d else 1.0)
+        # fast exponentials in silu, whose error the norm of a head of small values enlarges
+        assert np.abs(whole[0][rows].double().numpy() - y).max() <= 3e-5 * max(1.0, np.abs(y).max())
+        z, rate = a[rows].double().numpy() + dt.double().numpy(), np.exp(a_log.double().numpy())
+        want = np.exp(-(rate if head_decay else np.repeat(rate, d)) * np.logaddexp(0.0, z))
+        assert np.abs(whole[1][rows].double().numpy() - want).max() <= 2e-5
+        assert np.abs(whole[2][rows].double().numpy() - sig(x[rows, C:C + nh].double().numpy())).max() <= 1e-6
