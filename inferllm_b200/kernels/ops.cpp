@@ -886,7 +886,10 @@ Mat attention_diff(Device& dev, const Mat& q, const KVView& kv, const StepView& 
     if (!kv.k || !kv.v || kv.dtype != q.dtype || kv.n_kv_heads != g.n_kv_heads || kv.head_dim != 2 * g.head_dim || q.cols < (long long)g.n_heads * 2 * g.head_dim)
         throw KernelError("attention_diff: the cache entry must hold key rows of two maps (2 x " + std::to_string(g.head_dim) + " channels) in the queries' dtype");
     Mat out = new_mat(dev, q.rows, (long long)g.n_heads * dv, q.dtype);
-    if (q.dtype == DType::BF16 && !ctx.is_decode && q.cols % 8 == 0 && illm_attention_diff_tc_supported(g.n_heads, g.n_kv_heads, g.head_dim, dv, kv.page_size)) {
+    // Steps of a few tokens of many sequences stay on the warp-level kernel, whose blocks are smaller and which has one launch (two tokens of
+    // 64 sequences, 8 heads: 23 us, on tensor memory 25; with fewer blocks 12 and 9)
+    const bool short_prompts = ctx.max_q <= 32 && (long long)ctx.B * g.n_heads >= 256 && illm_attention_diff_mma_supported(g.head_dim, dv);
+    if (q.dtype == DType::BF16 && !ctx.is_decode && !short_prompts && q.cols % 8 == 0 && illm_attention_diff_tc_supported(g.n_heads, g.n_kv_heads, g.head_dim, dv, kv.page_size)) {
         const int heads = illm_attention_diff_tc_heads(q.rows, g.n_heads, dv);
         float* maps = dev.alloc_n<float>((size_t)q.rows * heads * 2 * dv);
         check_kernel(illm_attention_diff_tc_sliced(q.p, (int)q.cols, (int)q.rows, kv.k, kv.v, kv.num_pages, kv.block_table, kv.width, ctx.cu_q, ctx.seq_lens, maps, out.p,
