@@ -350,6 +350,10 @@ ILLM_API int illm_policy_ring_splits(long long T, int n_kv_heads, long long max_
 ILLM_API int illm_policy_attention_diff_splits(long long T, int head_groups, long long max_seq_len, int n_sms) {
     return ops::attention_diff_splits(T, head_groups, max_seq_len, n_sms);
 }
+// who takes a step's tokens, as ops::ScanForm: kind 0 linear attention, 1 the delta rule with a decay per channel, 2 with one per head
+ILLM_API int illm_policy_scan_form(int kind, long long T, int B, int max_q, int nh, int d, int dv) {
+    return (int)(kind == 0 ? ops::decay_scan_form(T, B, max_q, nh, d, dv) : ops::delta_rule_form(kind == 2, T, B, max_q, nh, d, dv));
+}
 // the tiles of a step's tokens into out[0] (dense) and out[1]; returns the form in which attention_generic takes them
 ILLM_API int illm_policy_attention_generic(const int* q_lens, int B, int nh, int n_sms, int* out) {
     ops::count_token_tiles(q_lens, B, out[0], out[1]);

@@ -801,8 +801,7 @@ static void launch_scan_as(const DeltaArgs& p, int B, int n_sms, cudaStream_t s)
 
 template <int L, int ROWS>
 static void launch_scan(const DeltaArgs& p, int B, int n_sms, cudaStream_t s, const float* rec) {
-    // (eight tokens at a time with 32 rows per thread do not fit the registers; up to 128 rows chunk_scan.cu takes them)
-    if constexpr (ROWS <= 16 && ROWS * L > 128) if (rec) {
+    if constexpr (ROWS <= 16) if (rec) {        // (eight tokens at a time with 32 rows per thread do not fit the registers)
         constexpr int COLS = DL_THREADS / L;
         size_t smem = (size_t)2 * (DL_TILE * (2 * ROWS * L + COLS) + (DL_TILE / DC) * DC_REC) * sizeof(float);
         const long long blocks = (long long)((p.dv + COLS - 1) / COLS) * p.nh * B, per_sm = (blocks + n_sms - 1) / n_sms;
@@ -846,15 +845,15 @@ static void launch_scan_for(const DeltaArgs& p, int B, cudaStream_t s, const flo
 // state: float32 [slots, state_elems], state_elems >= nh * d * dv + (taps - 1) * (2 nkv d + nh dv).
 // a: the decay projection, rows a_ld apart: nh * d columns, or with head_decay nh.
 // chunks (nullptr: token by token; without head_decay only for d <= 128): illm_delta_chunk_scratch floats, the scan then takes
-// eight tokens at a time; max_q the most tokens of one sequence.
+// eight tokens at a time, with own_chunks (head_decay only) by delta_chunk_scan_kernel for any d; max_q the most tokens of one sequence.
 // Scratch qkv [T, 2 nkv d + nh dv], g [T, nh d] (head_decay: [T, nh]), beta [T, nh]; out [T, nh dv].
-extern "C" int illm_delta_rule(const float* x, int T, int ld, int q_off, int k_off, int v_off, int b_off, const float* a, int a_ld, int head_decay, int nh, int nkv, int d,
+extern "C" int illm_delta_rule_form(const float* x, int T, int ld, int q_off, int k_off, int v_off, int b_off, const float* a, int a_ld, int head_decay, int nh, int nkv, int d,
                                int dv, int taps, const float* conv_q, const float* conv_k, const float* conv_v, const float* a_log,
                                const float* dt_bias, float q_scale, float* state, long long state_elems, const int* slots, const int* cu_q,
                                const int* token_pos, const int* token_seq, const int* seq_lens, float* qkv, float* g, float* beta, float* out,
-                               int B, int max_q, float* chunks, void* stream) {
+                               int B, int max_q, float* chunks, int own_chunks, void* stream) {
     if (T <= 0 || B <= 0) return 0;
-    if (!illm_delta_rule_supported(d, dv, taps) || nkv <= 0 || nh % nkv || a_ld < (head_decay ? nh : nh * d) || (chunks && ((!head_decay && !chunk_scan_takes(d)) || max_q <= 0 || nkv > 65535 || B > 65535))) return ILLM_ERR_BAD_ARG;
+    if (!illm_delta_rule_supported(d, dv, taps) || nkv <= 0 || nh % nkv || (own_chunks && !head_decay) || a_ld < (head_decay ? nh : nh * d) || (chunks && ((!head_decay && !chunk_scan_takes(d)) || max_q <= 0 || nkv > 65535 || B > 65535))) return ILLM_ERR_BAD_ARG;
     const long long C = 2LL * nkv * d + (long long)nh * dv;
     if (state_elems < (long long)nh * d * dv + (taps - 1) * C) return ILLM_ERR_BAD_ARG;
     cudaStream_t s = (cudaStream_t)stream;
@@ -881,7 +880,7 @@ extern "C" int illm_delta_rule(const float* x, int T, int ld, int q_off, int k_o
         else illm_launch(delta_prep_kernel<0>, pgrid, dim3(256), 0, s, p);
     }
     if (taps > 1) illm_launch(conv_state_kernel, dim3((unsigned)((C + 127) / 128), B), dim3(128), 0, s, p);
-    if (chunks && chunk_scan_takes(d)) {
+    if (chunks && !own_chunks && chunk_scan_takes(d)) {
         const float* base = qkv;
         const ChunkScanArgs a{base, base + (long long)nkv * d, base + 2LL * nkv * d, C, g, beta, nh, nh / nkv, d, dv, state, state_elems, slots, cu_q, chunks, out, 1, nullptr};
         return chunk_scan_launch(a, head_decay ? CHUNK_DELTA_HEAD : CHUNK_DELTA_CHANNEL, B, max_q, s);
@@ -896,4 +895,13 @@ extern "C" int illm_delta_rule(const float* x, int T, int ld, int q_off, int k_o
     else if (d <= 256) launch_scan_for<8>(p, B, s, chunks);
     else launch_scan_for<16>(p, B, s, chunks);
     return illm_launch_status();
+}
+
+extern "C" int illm_delta_rule(const float* x, int T, int ld, int q_off, int k_off, int v_off, int b_off, const float* a, int a_ld, int head_decay, int nh, int nkv, int d,
+                               int dv, int taps, const float* conv_q, const float* conv_k, const float* conv_v, const float* a_log,
+                               const float* dt_bias, float q_scale, float* state, long long state_elems, const int* slots, const int* cu_q,
+                               const int* token_pos, const int* token_seq, const int* seq_lens, float* qkv, float* g, float* beta, float* out,
+                               int B, int max_q, float* chunks, void* stream) {
+    return illm_delta_rule_form(x, T, ld, q_off, k_off, v_off, b_off, a, a_ld, head_decay, nh, nkv, d, dv, taps, conv_q, conv_k, conv_v, a_log, dt_bias, q_scale, state,
+                                state_elems, slots, cu_q, token_pos, token_seq, seq_lens, qkv, g, beta, out, B, max_q, chunks, 0, stream);
 }

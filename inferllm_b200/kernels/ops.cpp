@@ -562,6 +562,23 @@ int decay_scan_segments(int B, int n_heads, int v_head_dim, int max_q, int n_sms
     return P < 2 ? 1 : (int)P;
 }
 
+ScanForm decay_scan_form(long long T, int B, int max_q, int n_heads, int head_dim, int v_head_dim) {
+    const ScanForm one = ScanForm::TokenByToken, eight = ScanForm::Chunks;
+    if (max_q < kChunkScanMinTokens || head_dim > kChunkScanMaxHeadDim) return one;
+    const long long blocks = (long long)B * n_heads * ceil_div(v_head_dim, 32);      // of the chunks
+    // Up to 64 tokens the older kernel prepares the rows inside its walk: one sequence of 60 tokens of 8 heads of 64 68 us, by eights 21 (of
+    // 16 tokens of 8 heads of 16 x 16 13 and 14).
+    if (T <= 64) return max_q < 32 && head_dim <= 32 && (v_head_dim <= 32 || blocks >= 512) ? one : eight;
+    // Short sequences: the state's way in and out is most of it (32 of 16 tokens, 8 heads of 128: 23 us one by one, 33 by eights).
+    if (max_q < 32) return one;
+    if (max_q < 64) return blocks < 192 || (head_dim > 64 ? blocks > 1024 : v_head_dim <= 32 && blocks >= 1024) ? eight : one;
+    // Small heads that fill the SMs: 8,353 tokens of 32 heads of 32 x 256 695 and 1,490 us, of 64 x 128 714 and 890; 2,048 tokens of one
+    // sequence, 2 heads of 32 x 32, 2.6 times as fast by eights.
+    if (head_dim <= 32) return v_head_dim > 32 && blocks >= 256 && max_q < (v_head_dim > 64 ? 1024 : 128) ? one : eight;
+    if (head_dim <= 64) return (v_head_dim > 64 && blocks >= 2048) || (max_q < 128 && blocks >= 192 && (v_head_dim > 64 || blocks < 2048)) ? one : eight;
+    return eight;
+}
+
 Mat decay_scan(Device& dev, const Mat& x, const DecayScan& p, const StepView& ctx, const StateView& st) {
     need(x, "the packed projection", true, DType::F32);
     if (!st.state || st.dtype != DType::F32 || st.elements != (long long)p.n_heads * p.head_dim * p.v_head_dim)
@@ -570,7 +587,7 @@ Mat decay_scan(Device& dev, const Mat& x, const DecayScan& p, const StepView& ct
         throw KernelError("decay_scan: a state of " + std::to_string(p.head_dim) + " x " + std::to_string(p.v_head_dim) +
                           " per head is beyond the kernel (head sizes up to 1024)");
     Mat out = new_mat_exact(dev, x.rows, (long long)p.n_heads * p.v_head_dim, DType::F32);
-    if (!p.in_order && ctx.max_q >= kChunkScanMinTokens && p.head_dim <= kChunkScanMaxHeadDim) {
+    if (!p.in_order && decay_scan_form(x.rows, ctx.B, ctx.max_q, p.n_heads, p.head_dim, p.v_head_dim) == ScanForm::Chunks) {
         const int pieces = illm_decay_chunk_segments(ctx.B, p.n_heads, p.v_head_dim, ctx.max_q);
         float* rec = dev.alloc_n<float>((size_t)illm_decay_chunk_scratch((int)x.rows, ctx.B, p.n_heads, p.head_dim, p.v_head_dim, pieces));
         check_kernel(illm_decay_chunk_scan((float*)x.p, (int)x.rows, (int)x.cols, p.q_off, p.k_off, p.v_off, p.n_heads, p.head_dim, p.v_head_dim, p.qk_act,
@@ -1046,6 +1063,24 @@ long long delta_rule_state_elements(int nh, int nkv, int d, int dv, int taps) {
 }
 bool delta_rule_supported(int d, int dv, int taps) { return illm_delta_rule_supported(d, dv, taps) != 0; }
 
+ScanForm delta_rule_form(bool head_decay, long long T, int B, int max_q, int n_heads, int head_dim, int v_head_dim) {
+    const ScanForm one = ScanForm::TokenByToken, own = ScanForm::OwnChunks, eight = ScanForm::Chunks;
+    if (max_q < kChunkScanMinTokens) return one;
+    if (head_dim > kChunkScanMaxHeadDim) return head_decay ? own : one;
+    const long long blocks = (long long)B * n_heads * ceil_div(v_head_dim, 32), work = T * n_heads * head_dim * v_head_dim;      // blocks: of chunk_scan.cu
+    if (head_decay) {
+        // 16 tokens of 2 to 32 heads of 128 11 to 14 us one by one, 18 to 25 by its own chunks, 14 to 17 by chunk_scan.cu; one of 600 tokens, 2
+        // heads, 172, 94 and 132; 32 sequences of 30 to 100 tokens, 16 heads, 291, 360 and 243, of 64 channels 115, 155 and 148
+        if (max_q < 64) return one;
+        if (head_dim <= 64) return blocks <= (max_q < 200 ? 64 : 512) ? own : one;
+        return blocks <= 64 ? own : eight;
+    }
+    // long sequences, or enough work to make up for two more launches: one sequence of 48 tokens, 16 heads of 128, 25 us one by one and
+    // 26, 32 heads 30 and 25; of 600 tokens of two heads of 64 172 and 153; 6,254 tokens of 32 heads of 64 x 128 833 and 1,084
+    if (head_dim <= 64) return head_dim > 32 && max_q >= 200 && blocks <= 128 ? eight : one;
+    return max_q >= 128 || work >= (head_dim > 96 ? 14000000 : 50000000) ? eight : one;
+}
+
 Mat delta_rule(Device& dev, const Mat& x, const Mat* a, const DeltaRule& p, const StepView& ctx, const StateView& st) {
     need(x, "the packed projection", true, DType::F32);
     const long long T = x.rows, C = 2LL * p.n_kv_heads * p.head_dim + (long long)p.n_heads * p.v_head_dim;
@@ -1056,14 +1091,14 @@ Mat delta_rule(Device& dev, const Mat& x, const Mat* a, const DeltaRule& p, cons
         throw KernelError("delta_rule: the state entry does not have this layer's size");
     Mat qkv = new_mat_exact(dev, T, C, DType::F32), g = new_mat_exact(dev, T, decays, DType::F32), beta = new_mat_exact(dev, T, p.n_heads, DType::F32);
     Mat out = new_mat_exact(dev, T, (long long)p.n_heads * p.v_head_dim, DType::F32);
-    const bool chunked = !p.in_order && ctx.max_q >= kChunkScanMinTokens && (p.head_decay || p.head_dim <= kChunkScanMaxHeadDim);
-    float* chunks = chunked ? dev.alloc_n<float>((size_t)illm_delta_chunk_scratch((int)T, ctx.B, p.n_heads)) : nullptr;
-    check_kernel(illm_delta_rule((const float*)x.p, (int)T, (int)x.cols, p.q_off, p.k_off, p.v_off, p.b_off,
+    const ScanForm form = p.in_order ? ScanForm::TokenByToken : delta_rule_form(p.head_decay, T, ctx.B, ctx.max_q, p.n_heads, p.head_dim, p.v_head_dim);
+    float* chunks = form != ScanForm::TokenByToken ? dev.alloc_n<float>((size_t)illm_delta_chunk_scratch((int)T, ctx.B, p.n_heads)) : nullptr;
+    check_kernel(illm_delta_rule_form((const float*)x.p, (int)T, (int)x.cols, p.q_off, p.k_off, p.v_off, p.b_off,
                                  p.head_decay ? (const float*)x.p + p.a_off : (const float*)a->p, p.head_decay ? (int)x.cols : (int)decays,
                                  p.head_decay ? 1 : 0, p.n_heads,
                                  p.n_kv_heads, p.head_dim, p.v_head_dim, p.taps, p.conv_q, p.conv_k, p.conv_v, p.a_log, p.dt_bias, p.q_scale,
                                  (float*)st.state, st.elements, st.slots, ctx.cu_q, ctx.token_pos, ctx.token_seq, ctx.seq_lens, (float*)qkv.p,
-                                 (float*)g.p, (float*)beta.p, (float*)out.p, ctx.B, ctx.max_q, chunks, dev.stream()),
+                                 (float*)g.p, (float*)beta.p, (float*)out.p, ctx.B, ctx.max_q, chunks, form == ScanForm::OwnChunks ? 1 : 0, dev.stream()),
                  "delta_rule");
     return out;
 }

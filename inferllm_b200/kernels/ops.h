@@ -387,8 +387,16 @@ struct DeltaRule {
     float q_scale = 1.f;
 };
 // the most tokens of a sequence in a step from which the recurrences take eight at a time (bfloat16 mode; below, the state's
-// way in and out and the record of a chunk cost as much as the tokens), and the largest key heads of chunk_scan.cu
+// way in and out and the record of a chunk cost as much as the tokens), and the largest key heads of chunk_scan.cu.  In that mode
+// the rounding of a sequence's sums therefore depends on the step's longest sequence and on where its own prompt is cut, as it
+// does on the rows of a product; the float32 mode takes token by token always.
 constexpr int kChunkScanMinTokens = 16, kChunkScanMaxHeadDim = 128;
+// Who takes the tokens of such a step.  chunk_scan.cu always has the arithmetic of 128 key channels and two launches in front of its
+// walk; the older kernels have that of the head's own size, the token by token ones a longer chain.  The lines lie where
+// both sides were measured (d from 16 to 256, 2 to 32 heads, 1 to 32 sequences of 16 to 2,048 tokens).
+enum class ScanForm { TokenByToken, Chunks, OwnChunks };      // OwnChunks: delta_chunk_scan_kernel
+ScanForm delta_rule_form(bool head_decay, long long T, int B, int max_q, int n_heads, int head_dim, int v_head_dim);
+ScanForm decay_scan_form(long long T, int B, int max_q, int n_heads, int head_dim, int v_head_dim);
 long long delta_rule_state_elements(int n_heads, int n_kv_heads, int head_dim, int v_head_dim, int taps);
 bool delta_rule_supported(int head_dim, int v_head_dim, int taps);
 Mat delta_rule(Device& dev, const Mat& x_f32, const Mat* a_f32, const DeltaRule& p, const StepView& ctx, const StateView& st);

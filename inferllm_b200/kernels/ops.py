@@ -451,6 +451,12 @@ def attention_generic_form(q_lens, n_heads, n_sms=None):
     return int(_b.lib().illm_policy_attention_generic(lens, len(q_lens), int(n_heads), int(n_sms or n_sms_of_device()), tiles)), tiles[0], tiles[1]
 
 
+def scan_form(kind, T, B, max_q, n_heads, head_dim, v_head_dim):
+    """Who takes the tokens of a recurrence's step in the bfloat16 mode: 0 token by token, 1 chunks of eight (chunk_scan.cu), 2 the delta
+    rule's own chunks.  kind: 0 linear attention, 1 the delta rule with a decay per channel, 2 with one per head."""
+    return int(_b.lib().illm_policy_scan_form(int(kind), int(T), int(B), int(max_q), int(n_heads), int(head_dim), int(v_head_dim)))
+
+
 def attention_decode_ring(qkv, k_cache, v_cache, block_table, token_pos, token_seq, n_heads, n_kv_heads,
                           head_dim, page_size, window, scale, max_len, splits=None, rope=None):
     """bfloat16 attention of single tokens as a stream: K/V tiles of 64 keys by TMA through a ring

@@ -210,3 +210,42 @@ def test_delta_preparation_of_many_tokens(taps, d, dv, nh, nkv, head_decay):
         want = np.exp(-(rate if head_decay else np.repeat(rate, d)) * np.logaddexp(0.0, z))
         assert np.abs(whole[1][rows].double().numpy() - want).max() <= 2e-5
         assert np.abs(whole[2][rows].double().numpy() - sig(x[rows, C:C + nh].double().numpy())).max() <= 1e-6
+
+
+@pytest.mark.parametrize("d,dv,nh,nkv", [(128, 64, 2, 1), (64, 64, 4, 2), (20, 30, 2, 2), (9, 7, 3, 1)])
+def test_delta_rule_own_chunks(d, dv, nh, nkv):
+    """The delta rule's own chunks for the head sizes that chunk_scan.cu takes too: no more than twice as far from float64 as token by token."""
+    taps, g = 2, torch.Generator().manual_seed(d * dv)
+    cu, cu_d, pos, seq, slots, lens = layout()
+    T, B, C = int(cu[-1]), len(LENS), 2 * nkv * d + nh * dv
+    ld, elems = C + nh, nh * d * dv + (taps - 1) * C
+    x, a = torch.randn(T, ld, generator=g), torch.randn(T, nh, generator=g)
+    weights = [torch.randn(*s, generator=g).cuda() for s in ((nkv * d, taps), (nkv * d, taps), (nh * dv, taps), (nh,), (nh,))]
+    S0, xd, ad = torch.randn(B, elems, generator=g), x.cuda(), a.cuda()
+    f = entry("illm_delta_rule_form", I_, P_, I_, I_, I_, I_, I_, I_, P_, I_, I_, I_, I_, I_, I_, I_, P_, P_, P_, P_, P_, F_, P_, L_, P_, P_, P_, P_, P_, P_, P_, P_, P_, I_,
+              I_, P_, I_, P_)
+    n = entry("illm_delta_chunk_scratch", L_, I_, I_, I_)(T, B, nh)
+
+    def run(own):
+        S, out = S0.cuda(), torch.full((T, nh * dv), float("nan"), device="cuda")
+        mid = [torch.empty(T, w, device="cuda") for w in (C, nh, nh)]
+        rec = torch.full((n,), float("nan"), device="cuda") if own else None
+        rc = f(p(xd), T, ld, 0, nkv * d, 2 * nkv * d, C, p(ad), nh, 1, nh, nkv, d, dv, taps, *(p(t) for t in weights), d ** -0.5, p(S), elems, p(slots), p(cu_d), p(pos), p(seq),
+               p(lens), *(p(t) for t in mid), p(out), B, max(LENS), p(rec), own, torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        return [t.cpu().double().numpy() for t in (out, S, *mid)]
+
+    chunked, (out, S, qkv, gg, beta) = run(1), run(0)
+    share = nh // nkv
+    for b in range(B):
+        s, refs = B - 1 - b, []
+        St = S0[s, :nh * d * dv].double().numpy().reshape(nh, dv, d).copy()
+        for t in range(cu[b], cu[b + 1]):
+            q, k, v = (qkv[t, lo:lo + w * e].reshape(w, e) for lo, w, e in ((0, nkv, d), (nkv * d, nkv, d), (2 * nkv * d, nh, dv)))
+            q, k = q.repeat(share, 0), k.repeat(share, 0)
+            St = St * gg[t].reshape(nh, 1, 1)
+            St = St + (beta[t][:, None] * (v - np.einsum("hvd,hd->hv", St, k)))[:, :, None] * k[:, None, :]
+            refs.append(np.einsum("hvd,hd->hv", St, q).reshape(-1))
+        refs, rows = np.array(refs), slice(cu[b], cu[b + 1])
+        for mine, token, ref in ((chunked[0][rows], out[rows], refs), (chunked[1][s, :nh * d * dv], S[s, :nh * d * dv], St.reshape(-1))):
+            assert np.linalg.norm(mine - ref) <= 2 * np.linalg.norm(token - ref) + 4 * 2.0 ** -24 * np.linalg.norm(ref)

@@ -68,3 +68,19 @@ def test_differential_decode_splits():
     assert ops.attention_diff_splits(8, 8, 4096, 148) == 4
     assert ops.attention_diff_splits(8, 2, 4096, 148) == 16
     assert ops.attention_diff_splits(512, 8, 4096, 148) == 1
+
+
+def test_who_takes_a_recurrences_tokens():
+    """Chunks of eight where they were measured to be the faster ones, the older kernels elsewhere, in the bfloat16 mode (1, 0 and 2: ops.scan_form)."""
+    linear, channel, head = (lambda *a, k=k: ops.scan_form(k, *a) for k in (0, 1, 2))
+    for form in (linear, channel, head):        # T, B, longest, heads, key and value channels
+        assert form(8, 1, 8, 16, 128, 128) == 0 and form(480, 32, 15, 16, 128, 128) == 0
+        assert form(4096, 4, 1500, 16, 128, 128) == 1
+    assert [channel(4096, 1, 4096, 16, d, 128) for d in (16, 48, 64, 128, 129, 256)] == [0, 1, 1, 1, 0, 0]
+    assert [head(4096, 4, 1500, 16, d, 128) for d in (16, 48, 64, 128, 129, 256)] == [2, 2, 2, 1, 2, 2]
+    assert channel(48, 1, 48, 16, 128, 128) == 0 and channel(48, 1, 48, 32, 128, 128) == 1 and channel(600, 1, 600, 2, 64, 64) == 1
+    assert channel(6254, 32, 300, 32, 64, 128) == 0 and channel(6254, 32, 300, 32, 128, 128) == 1
+    assert head(16, 1, 16, 32, 128, 128) == 0 and head(600, 1, 600, 2, 128, 128) == 2 and head(2334, 32, 100, 16, 128, 128) == 1 and head(2334, 32, 100, 16, 64, 64) == 0
+    assert linear(2048, 1, 2048, 2, 32, 32) == 1 and linear(2048, 1, 2048, 16, 129, 128) == 0
+    assert linear(346, 32, 16, 8, 128, 128) == 0 and linear(41, 4, 16, 8, 128, 128) == 1 and linear(60, 1, 60, 8, 64, 64) == 1 and linear(172, 8, 32, 32, 32, 64) == 0
+    assert linear(8353, 32, 400, 32, 32, 256) == 0 and linear(8353, 32, 400, 32, 64, 128) == 0 and linear(8353, 32, 400, 32, 128, 128) == 1
